@@ -61,10 +61,10 @@ SUBSTEP_CAP = 16
 # Algorithmic bytes per particle of each substep kernel: the particle's own
 # records it must read and write once (neighbour reads are cache hits in
 # cell order and not counted). keys+count 20, reorder 116, density 44,
-# divergence kappa 28 / apply 36, forces 84 / 92, density kappa 36 / apply
-# 36, integrate 120.
+# divergence kappa 28 / apply 36, forces (with their apply, one sweep) 148,
+# density kappa 36 / apply 36, integrate 120.
 ALGO_BYTES = {"grid": 20.0, "gather": 116.0, "density_div": 44.0, "div_kappa": 28.0,
-              "div_apply": 36.0, "forces_eval": 84.0, "forces_den_apply": 92.0,
+              "div_apply": 36.0, "forces_eval": 148.0,
               "den_kappa": 36.0, "den_apply": 36.0, "integrate": 120.0}
 # DRAM bytes (read + write) per particle per launch: a constant taken from
 # one ncu capture of each kernel on this workload at its full 1,048,576
@@ -334,7 +334,7 @@ def cuda_arm(args):
     # prediction and forces_eval, run after each divergence apply, forms the
     # next ones (no div_kappa sweep): forces_eval runs md times a substep.
     per_substep = {"grid": 1.0, "gather": 1.0, "density_div": 1.0, "div_apply": md,
-                   "forces_eval": max(md, 1.0), "forces_den_apply": 1.0, "den_kappa": 1.0 + mk,
+                   "forces_eval": max(md, 1.0), "den_kappa": 1.0 + mk,
                    "den_apply": mk, "integrate": 1.0}
     share = {k: mean[k] * per_substep[k] for k in mean if k in per_substep}
     dom = max(share, key=lambda k: share[k])

@@ -125,20 +125,20 @@ cudaError_t batch_enqueue(FluidBatch *s, cudaStream_t st, uint32_t div_iters, ui
                                        s->gw, s->ring, s->cur, s->solve, kBatchRing, &bk);
     if (e != cudaSuccess) return e;
     const Geo g = s->geo();
+    const SimBufs bd = divergence_bufs(s->b), bf = after_forces(s->b);
     launch_gather(st, s->b, s->n);
-    launch_density_div(st, g, s->b, 0);
+    launch_density_div(st, g, bd, 0);
     for (uint32_t d = 0; d < div_iters; ++d) {
-        if (d > 0) launch_div_kappa(st, g, s->b, (int)d, kGateNone);
-        launch_apply(st, g, s->b, false, kGateNone);
+        if (d > 0) launch_div_kappa(st, g, bd, (int)d, kGateNone);
+        launch_apply(st, g, bd, false, kGateNone);
     }
     launch_forces_eval(st, g, s->b);
-    launch_forces_apply(st, g, s->b);
     for (uint32_t k = 0; k < den_iters; ++k) {
-        launch_den_kappa(st, g, s->b, (int)k, kGateNone);
-        launch_apply(st, g, s->b, true, kGateNone);
+        launch_den_kappa(st, g, bf, (int)k, kGateNone);
+        launch_apply(st, g, bf, true, kGateNone);
     }
     const int div_slot = div_iters > 0 ? (int)div_iters - 1 : 0;
-    launch_integrate(st, g, s->b, div_slot, den_iters > 0 ? (int)den_iters - 1 : -1, (int)div_iters,
+    launch_integrate(st, g, bf, div_slot, den_iters > 0 ? (int)den_iters - 1 : -1, (int)div_iters,
                      (int)den_iters);
     return cudaGetLastError();
 }
@@ -191,11 +191,7 @@ int32_t batch_graph_tolerance(FluidBatch *s, cudaGraphExec_t *out) {
     // forces_eval after every divergence apply, forming the prediction that
     // decides the loop (as the one-box tolerance substep)
     const bool fused = c.max_iters >= 1;
-    SimBufs bd = s->b;
-    if (fused) {
-        bd.kd = s->b.kd2;
-        bd.wpk = s->b.wpk2;
-    }
+    const SimBufs bd = divergence_bufs(s->b), bf = after_forces(s->b);
     if (e == cudaSuccess) {
         launch_gather(st, s->b, s->n);
         launch_density_div(st, geo, bd, 0);
@@ -204,12 +200,11 @@ int32_t batch_graph_tolerance(FluidBatch *s, cudaGraphExec_t *out) {
     }
     if (e == cudaSuccess && rc == FLUID_OK) {
         if (!fused) launch_forces_eval(st, geo, s->b);
-        launch_forces_apply(st, geo, s->b);
-        launch_den_kappa(st, geo, s->b, 0, kGateNone);
+        launch_den_kappa(st, geo, bf, 0, kGateNone);
         launch_tol_finish(st, geo, 1, 1, c.den_tol, c.max_iters, hden);
         rc = host_add_while(st, g, hden, &bden);
     }
-    if (e == cudaSuccess && rc == FLUID_OK) launch_integrate(st, geo, s->b, -1, -1, 0, 0);
+    if (e == cudaSuccess && rc == FLUID_OK) launch_integrate(st, geo, bf, -1, -1, 0, 0);
     if (e == cudaSuccess) e = cudaGetLastError();
     cudaGraph_t g2 = nullptr;
     cudaError_t e2 = cudaStreamEndCapture(st, &g2);
@@ -225,12 +220,12 @@ int32_t batch_graph_tolerance(FluidBatch *s, cudaGraphExec_t *out) {
     BK(cudaStreamBeginCaptureToGraph(s->side, bdiv, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     launch_apply(s->side, geo, bd, false, kGateDiv);
     if (fused) launch_forces_div(s->side, geo, s->b, 0, kGateDiv);
-    else launch_div_kappa(s->side, geo, s->b, 0, kGateDiv);
+    else launch_div_kappa(s->side, geo, bd, 0, kGateDiv);
     launch_tol_finish(s->side, geo, 0, 0, c.div_tol, c.max_iters, hdiv);
     BK(cudaStreamEndCapture(s->side, &bdiv));
     BK(cudaStreamBeginCaptureToGraph(s->side, bden, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    launch_apply(s->side, geo, s->b, true, kGateDen);
-    launch_den_kappa(s->side, geo, s->b, 0, kGateDen);
+    launch_apply(s->side, geo, bf, true, kGateDen);
+    launch_den_kappa(s->side, geo, bf, 0, kGateDen);
     launch_tol_finish(s->side, geo, 1, 0, c.den_tol, c.max_iters, hden);
     BK(cudaStreamEndCapture(s->side, &bden));
     e = cudaGraphInstantiate(&s->tol_graph, g, 0);
@@ -345,6 +340,9 @@ int32_t batch_create_into(FluidBatch *s, const FluidSimConfig *boxes, uint32_t n
     BK(s->alloc(&b.wpk, n));
     BK(s->alloc(&b.kd2, n));
     BK(s->alloc(&b.wpk2, n));
+    BK(s->alloc(&b.aux, n));
+    BK(s->alloc(&b.fvel, n));
+    BK(s->alloc(&b.ftemp, n));
     BK(s->alloc(&b.pressure, n));
     BK(s->alloc(&b.pinc, n));
     BK(s->alloc(&b.rho_near, n));
@@ -591,16 +589,17 @@ int32_t timed_substep(FluidBatch *s, int tpb, float *ms, cudaEvent_t *ev) {
         cudaEventElapsedTime(&t, ev[e], ev[e + 1]);
         ms[slot] += t;
     };
-    timed(kTuneDensity, [&] { launch_density_div(st, g, s->b, 0); });
-    timed(kTuneApply, [&] { launch_apply(st, g, s->b, false, kGateNone); });
-    timed(kTuneDivKappa, [&] { launch_div_kappa(st, g, s->b, 1, kGateNone); });
+    const SimBufs bd = divergence_bufs(s->b), bf = after_forces(s->b);
+    timed(kTuneDensity, [&] { launch_density_div(st, g, bd, 0); });
+    timed(kTuneApply, [&] { launch_apply(st, g, bd, false, kGateNone); });
+    timed(kTuneDivKappa, [&] { launch_div_kappa(st, g, bd, 1, kGateNone); });
     timed(kTuneForcesEval, [&] { launch_forces_eval(st, g, s->b); });
-    timed(kTuneForcesApply, [&] { launch_forces_apply(st, g, s->b); });
+    ms[kTuneForcesApply] = ms[kTuneForcesEval];  // one sweep forms both
     for (int k = 0; k < 2; ++k) {
-        timed(kTuneDenKappa, [&] { launch_den_kappa(st, g, s->b, k, kGateNone); });
-        timed(kTuneApply, [&] { launch_apply(st, g, s->b, true, kGateNone); });
+        timed(kTuneDenKappa, [&] { launch_den_kappa(st, g, bf, k, kGateNone); });
+        timed(kTuneApply, [&] { launch_apply(st, g, bf, true, kGateNone); });
     }
-    timed(kTuneIntegrate, [&] { launch_integrate(st, g, s->b, 0, 1, 1, 2); });
+    timed(kTuneIntegrate, [&] { launch_integrate(st, g, bf, 0, 1, 1, 2); });
     BK(cudaGetLastError());
     return FLUID_OK;
 }

@@ -114,6 +114,7 @@ struct FluidSim {
     cudaGraphExec_t density_graph = nullptr;
     cudaGraphExec_t tol_graph = nullptr;
     cudaStream_t side = nullptr;  // captures the loop bodies
+    bool work_after_forces = false;  // the last substep went past the forces: its velocity is in fvel
     std::vector<void *> allocs;
     float stats_host[14]{};
     uint32_t last_frame_substeps = 0;
@@ -311,29 +312,28 @@ cudaError_t enqueue_substep(FluidSim *s, cudaStream_t st, uint32_t div_iters, ui
     const Geo g = s->geo();
     launch_gather(st, s->b, s->n);
     mark("gather");
-    launch_density_div(st, g, s->b, 0);
+    const SimBufs bd = divergence_bufs(s->b), bf = after_forces(s->b);
+    launch_density_div(st, g, density_only ? s->b : bd, 0);
     mark("density_div");
     if (density_only) return cudaGetLastError();
     for (uint32_t d = 0; d < div_iters; ++d) {
         if (d > 0) {
-            launch_div_kappa(st, g, s->b, (int)d, kGateNone);
+            launch_div_kappa(st, g, bd, (int)d, kGateNone);
             mark("div_kappa");
         }
-        launch_apply(st, g, s->b, false, kGateNone);
+        launch_apply(st, g, bd, false, kGateNone);
         mark("div_apply");
     }
     launch_forces_eval(st, g, s->b);
     mark("forces_eval");
-    launch_forces_apply(st, g, s->b);
-    mark("forces_den_apply");
     for (uint32_t k = 0; k < den_iters; ++k) {
-        launch_den_kappa(st, g, s->b, (int)k, kGateNone);
+        launch_den_kappa(st, g, bf, (int)k, kGateNone);
         mark("den_kappa");
-        launch_apply(st, g, s->b, true, kGateNone);
+        launch_apply(st, g, bf, true, kGateNone);
         mark("den_apply");
     }
     const int div_slot = div_iters > 0 ? (int)div_iters - 1 : 0;
-    launch_integrate(st, g, s->b, div_slot, den_iters > 0 ? (int)den_iters - 1 : -1, (int)div_iters,
+    launch_integrate(st, g, bf, div_slot, den_iters > 0 ? (int)den_iters - 1 : -1, (int)div_iters,
                      (int)den_iters);
     mark("integrate");
     return cudaGetLastError();
@@ -407,11 +407,7 @@ int32_t capture_tolerance(FluidSim *s, cudaGraphExec_t *out) {
     // and also forms the divergence prediction that decides whether the
     // loop goes on (its kappa in kd2 / wpk2, which the loop's applies read).
     const bool fused = c.max_iters >= 1;
-    SimBufs bd = s->b;
-    if (fused) {
-        bd.kd = s->b.kd2;
-        bd.wpk = s->b.wpk2;
-    }
+    const SimBufs bd = divergence_bufs(s->b), bf = after_forces(s->b);
     if (e == cudaSuccess) {
         launch_gather(st, s->b, s->n);
         launch_density_div(st, geo, bd, 0);
@@ -420,12 +416,11 @@ int32_t capture_tolerance(FluidSim *s, cudaGraphExec_t *out) {
     }
     if (e == cudaSuccess && rc == FLUID_OK) {
         if (!fused) launch_forces_eval(st, geo, s->b);
-        launch_forces_apply(st, geo, s->b);
-        launch_den_kappa(st, geo, s->b, 0, kGateNone);
+        launch_den_kappa(st, geo, bf, 0, kGateNone);
         launch_tol_finish(st, geo, 1, 1, c.den_tol, c.max_iters, hden);
         rc = add_while(st, g, hden, &bden);
     }
-    if (e == cudaSuccess && rc == FLUID_OK) launch_integrate(st, geo, s->b, -1, -1, 0, 0);
+    if (e == cudaSuccess && rc == FLUID_OK) launch_integrate(st, geo, bf, -1, -1, 0, 0);
     if (e == cudaSuccess) e = cudaGetLastError();
     cudaGraph_t g2 = nullptr;
     cudaError_t e2 = cudaStreamEndCapture(st, &g2);
@@ -439,12 +434,12 @@ int32_t capture_tolerance(FluidSim *s, cudaGraphExec_t *out) {
     CK(cudaStreamBeginCaptureToGraph(s->side, bdiv, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     launch_apply(s->side, geo, bd, false, kGateDiv);
     if (fused) launch_forces_div(s->side, geo, s->b, 0, kGateDiv);
-    else launch_div_kappa(s->side, geo, s->b, 0, kGateDiv);
+    else launch_div_kappa(s->side, geo, bd, 0, kGateDiv);
     launch_tol_finish(s->side, geo, 0, 0, c.div_tol, c.max_iters, hdiv);
     CK(cudaStreamEndCapture(s->side, &bdiv));
     CK(cudaStreamBeginCaptureToGraph(s->side, bden, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    launch_apply(s->side, geo, s->b, true, kGateDen);
-    launch_den_kappa(s->side, geo, s->b, 0, kGateDen);
+    launch_apply(s->side, geo, bf, true, kGateDen);
+    launch_den_kappa(s->side, geo, bf, 0, kGateDen);
     launch_tol_finish(s->side, geo, 1, 0, c.den_tol, c.max_iters, hden);
     CK(cudaStreamEndCapture(s->side, &bden));
     e = cudaGraphInstantiate(out, g, 0);
@@ -502,6 +497,7 @@ int32_t run_frame(FluidSim *s, const FluidStep &st, uint32_t n, uint32_t refine,
     rc = substep_graph(s, refine, &g);
     if (rc != FLUID_OK) return rc;
     for (uint32_t k = 0; k < n; ++k) CK(cudaGraphLaunch(g, s->stream));
+    if (n) s->work_after_forces = true;
     launch_stats(s->stream, s->geo(), s->b, s->stats_chunks());
     if (s->ntr) {
         FluidStep tr;
@@ -670,6 +666,9 @@ static int32_t create_into(FluidSim *s, const FluidSimConfig *cfg) {
     CK(s->alloc(&b.wpk, n));
     CK(s->alloc(&b.kd2, n));
     CK(s->alloc(&b.wpk2, n));
+    CK(s->alloc(&b.aux, n));
+    CK(s->alloc(&b.fvel, n));
+    CK(s->alloc(&b.ftemp, n));
     CK(s->alloc(&b.pressure, n));
     CK(s->alloc(&b.pinc, n));
     CK(s->alloc(&b.rho_near, n));
@@ -775,6 +774,7 @@ int32_t fluid_sim_run(FluidSim *s, const FluidStep *steps, uint32_t count) {
                 if (rc != FLUID_OK) return rc;
             }
             CK(cudaGraphLaunch(g, s->stream));
+            s->work_after_forces = steps[done + k].dt != 0.0f;
         }
         done += m;
     }
@@ -1011,7 +1011,7 @@ int32_t fluid_sim_read_field(FluidSim *s, int32_t field, void *out, uint64_t byt
     case FLUID_FIELD_STARTS: src = s->b.starts; need = 4ull * (s->keyspace + 1); break;
     case FLUID_FIELD_PERM: src = s->b.perm; need = 4 * n; break;
     case FLUID_FIELD_WORK_POS: src = s->b.wpos; need = 16 * n; break;
-    case FLUID_FIELD_WORK_VEL: src = s->b.wvel; need = 16 * n; break;
+    case FLUID_FIELD_WORK_VEL: src = s->work_after_forces ? s->b.fvel : s->b.wvel; need = 16 * n; break;
     case FLUID_FIELD_ACCEL: src = s->b.accel; need = 16 * n; break;
     case FLUID_FIELD_XSPH: src = s->b.xsph; need = 16 * n; break;
     case FLUID_FIELD_WALL_GRAD: src = s->b.wgrad; need = 16 * n; break;
@@ -1044,10 +1044,10 @@ uint32_t fluid_sim_kernels_per_substep(const FluidSim *s) {
     if (!s) return 0;
     const uint32_t passes = (uint32_t)radix_passes(s->keyspace);
     // keys + one per radix pass + starts scan + gather + density_div
-    //   + div applies (+ div_kappa after the first) + forces pair
+    //   + div applies (+ div_kappa after the first) + forces
     //   + den pairs + integrate
     const uint32_t d = s->cfg.div_iters, k = s->cfg.den_iters;
-    return 2 + passes + 1 + 1 + (d ? 2 * d - 1 : 0) + 2 + 2 * k + 1;
+    return 2 + passes + 1 + 1 + (d ? 2 * d - 1 : 0) + 1 + 2 * k + 1;
 }
 
 int32_t fluid_sim_profile_step(FluidSim *s, const FluidStep *step, float *ms, const char **names,
@@ -1072,6 +1072,7 @@ int32_t fluid_sim_profile_step(FluidSim *s, const FluidStep *step, float *ms, co
     };
     if (step->dt == 0.0f) err = enqueue_substep(s, s->stream, 0, 0, true, mark);
     else err = enqueue_substep(s, s->stream, s->cfg.div_iters, s->cfg.den_iters, false, mark);
+    s->work_after_forces = step->dt != 0.0f;
     CK(err);
     CK(cudaStreamSynchronize(s->stream));
     uint32_t k = 0;

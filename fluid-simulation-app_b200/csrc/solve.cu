@@ -18,7 +18,7 @@
 
 // Neighbour batches of the list sweeps (see walk below): entries whose
 // records are loaded before any is used. Position + kappa records, position
-// + velocity records, and forces_eval's five records; FCU_MINB is the
+// + velocity records, and forces_eval's three records; FCU_MINB is the
 // minimum resident blocks per SM the sweeps are compiled for (0: none).
 #ifndef FCU_B_KD
 #define FCU_B_KD 4
@@ -26,8 +26,8 @@
 #ifndef FCU_B_PV
 #define FCU_B_PV 4
 #endif
-#ifndef FCU_B_N5
-#define FCU_B_N5 1
+#ifndef FCU_B_N3
+#define FCU_B_N3 1
 #endif
 // Minimum resident blocks per SM that density_div (at 128 threads a block;
 // scaled for other block sizes; a batch too: its instance measured 3 %
@@ -64,17 +64,13 @@ constexpr int kBatchKappaThreads = 768;
 #ifndef FCU_MINB
 #define FCU_MINB 0
 #endif
-// One box's forces_eval (plain and with the divergence prediction) at 8
-// blocks of 128 threads per SM (64 registers; the fused one spills 24
-// bytes): frames 1.1 % shorter on the 1M workload than at its 72 / 76
-// registers (7 / 6 blocks). Scaled for other block sizes like density_div.
+// The forces sweep (plain and with the divergence prediction) of one box at
+// 6 blocks of 128 threads per SM (80 registers, no spills): 488 us on the 1M
+// workload against 500 at 7 (56 bytes spilled), 596 at 8 (128) and 523 at 5.
+// A batch likewise: 2.739 ms a substep of 64 boxes at 6, 2.850 at 7, 2.750
+// at 5. Scaled for other block sizes like density_div.
 #ifndef FCU_MINB_FORCES
-#define FCU_MINB_FORCES 8
-#endif
-// The batch's forces_eval at 7 blocks of 128 per SM (scaled likewise):
-// batched_256 8.88 against 9.05 ms a substep with no floor, 9.12 at 8.
-#ifndef FCU_MINB_FORCES_BATCH
-#define FCU_MINB_FORCES_BATCH 7
+#define FCU_MINB_FORCES 6
 #endif
 
 namespace fcu {
@@ -339,14 +335,13 @@ struct PosKd {
 struct PosVel {
     float4 p, v;
 };
-struct Nbr5 {
-    float4 p, v;
-    float rho, temp, near;
+struct Nbr3 {
+    float4 p, v, a;  // position, velocity, (density, near density, temperature, warm kd)
 };
 
 // Particle counts stay below 2^28 (the host rejects more), so masking a list
 // entry's slot changes no slot. forces_eval's loader applies the mask before
-// forming its five record addresses: measured 13 % faster on the 1M-particle
+// forming its record addresses: measured 13 % faster on the 1M-particle
 // workload (0.58 against 0.67 ms); in the kappa sweeps it measured slower and
 // is left out.
 constexpr uint32_t kSlotMask = (1u << 28) - 1u;
@@ -737,6 +732,10 @@ __global__ void __launch_bounds__(TPB, (kB ? FCU_MINB_DD_BATCH : FCU_MINB_DD) * 
         grad_sum = grad_sum + wg;
         b.density[i] = rho;
         b.rho_near[i] = rho_near;
+        // the warm start's kd, half the last pressure over rho^2, so that
+        // forces_eval can form forces_den_apply's sum in its own walk
+        const float half = 0.5f * __ldg(&b.wpp[i]);
+        b.aux[i] = make_float4(rho, rho_near, __ldg(&b.wtemp[i]), half / (rho * rho));
         const float a = rho / fmaxf(dot(grad_sum, grad_sum) + grad_sq, 1e-4f);
         b.alpha[i] = a;
         drho += dot(vel, wg);
@@ -830,116 +829,6 @@ __global__ void __launch_bounds__(TPB, FCU_MINB) k_apply(Geo g, SimBufs b, int a
     if (i < g.n) apply_at<kB>(g, b, i, add_pressure, gate);
 }
 
-// ---- forces_eval (sim_solve.wgsl:524-592) ---------------------------------
-// With kDiv, the same walk also forms the divergence prediction of
-// k_div_kappa (the same pair terms, in the same order, so the same sums):
-// its kappa goes to kd2 / wpk2 and its residual term to acc_div[slot], and
-// boxes whose divergence loop has stopped (gate) are skipped. The tolerance
-// schedule runs this after each divergence apply, so the prediction that
-// only decides whether the loop stops costs no sweep of its own.
-template <bool kB, bool kDiv>
-__device__ __forceinline__ void forces_eval_body(const Geo &g, const SimBufs &b, uint32_t i, bool live,
-                                                 int slot, int gate) {
-    const uint32_t n = g.n;
-    if (!kDiv && !live) return;
-    const uint32_t bi = box_index<kB>(g, live ? i : n - 1);
-    unsigned long long term = 0;
-    if (live && !(kDiv && gated_out<kB>(g, bi, gate))) {
-    // a batch reads its box's constants from the box's entry where they are
-    // used, keeping the pair loop's few in registers; one box copies them
-    // from parameter space as before
-    DevParams Pc;
-    if (!kB) Pc = g.one;
-    const DevParams &P = kB ? g.box[bi] : Pc;
-    const KernelConsts K = kernel_consts(P);
-    const float mass = P.mass, inv_h = P.inv_h, rho0 = P.rho0, soft = 0.01f * P.h * P.h;
-    const float coh_c = 2.0f * P.h;
-    const float c3 = coh_c * coh_c * coh_c;
-    const float coh_k = 32.0f / (3.14159265f * c3 * c3 * c3);
-    const float coh_near = c3 * c3 / 64.0f;
-    const float c = 2.0f * P.h;
-    const float gamma = SIGMA_WATER * 7040.0f / (21.0f * LATTICE_SIGMA * P.rho0 * P.rho0 * c * c);
-    const float beta =
-        SIGMA_WATER * (1.0f + COS_CONTACT) * 1558.4f / (LATTICE_SIGMA * P.rho0 * P.rho0 * c * c);
-    const float visc_k = 2.0f * DYNAMIC_VISCOSITY;
-    const float heat_k = 2.0f * CONDUCTIVITY / HEAT_CAPACITY;
-    const float diss_k = 0.5f * DYNAMIC_VISCOSITY / HEAT_CAPACITY;
-
-    const F3 pos = xyz(__ldg(&b.wpos[i]));
-    const float near_i = __ldg(&b.rho_near[i]);
-    const F3 vel = xyz(__ldg(&b.wvel[i]));
-    const float temp = __ldg(&b.wtemp[i]);
-    const float rho_i = __ldg(&b.density[i]);
-    const uint32_t cnt = __ldg(&b.nbr_n[i]);
-    F3 visc = f3(0.f, 0.f, 0.f), blend = f3(0.f, 0.f, 0.f), near = f3(0.f, 0.f, 0.f),
-       tension = f3(0.f, 0.f, 0.f);
-    float heat = 0.0f, drho = 0.0f;
-    auto load = [&](uint32_t code) {
-        const uint32_t j = list_slot(code);
-        return Nbr5{__ldg(&b.wpos[j]), __ldg(&b.wvel[j]), __ldg(&b.density[j]), __ldg(&b.wtemp[j]),
-                    __ldg(&b.rho_near[j])};
-    };
-    walk<FCU_B_N5, Nbr5>(b.nbr, n, i, cnt, load, [&](float gs, const Nbr5 &q) {
-        const float4 pj = q.p;
-        const F3 e = pair_grad(gs, pos, pj);
-        const F3 x = pos - xyz(pj);
-        const float r2 = dot(x, x);
-        const float r = sqrtf(r2);
-        const float rho_j = q.rho;
-        const float f = dot(x, e) / (r2 + soft);
-        const float pair = mass / (rho_i * rho_j) * f;
-        const F3 dv = vel - xyz(q.v);
-        if (kDiv) drho += dot(dv, e);
-        const float wn = fmaxf(1.0f - r * inv_h, 0.0f);
-        near = near + ((near_i + q.near) * wn * wn) * (x / fmaxf(r, 1e-5f));
-        visc = visc + (visc_k * pair) * dv;
-        blend = blend - (mass / rho_j * kernel_q(K, r * inv_h)) * dv;
-        heat += heat_k * pair * (temp - q.temp);
-        heat -= diss_k * pair * dot(dv, dv);
-        const float corr = 2.0f * rho0 / (rho_i + rho_j);
-        tension = tension - ((corr * mass * cohesion(r, coh_c, coh_k, coh_near)) * x) / fmaxf(r, 1e-9f);
-    });
-    const F3 adh = (beta * P.rho0) * wall_adh_sum(P, pos);
-    const F3 acc = visc + K_NEAR * near + gamma * tension + adh;
-    b.accel[i] = make_float4(acc.x, acc.y, acc.z, heat);
-    b.xsph[i] = make_float4(blend.x, blend.y, blend.z, 0.0f);
-    const float half = 0.5f * __ldg(&b.wpp[i]);
-    const float kdv = half / (rho_i * rho_i);
-    b.kd[i] = kdv;
-    b.wpk[i] = make_float4(pos.x, pos.y, pos.z, kdv);
-    b.pressure[i] = half;
-    if (kDiv) {  // k_div_kappa's prediction
-        const float dt = g.st[bi].s.dt;
-        drho = P.mass * drho;
-        drho += dot(vel, xyz(__ldg(&b.wgrad[i])));
-        const float kdd = fmaxf(drho, 0.0f) * __ldg(&b.alpha[i]) / fmaxf(dt, 1e-9f) / rho_i;
-        b.kd2[i] = kdd;
-        b.wpk2[i] = make_float4(pos.x, pos.y, pos.z, kdd);
-        term = fixed_term((double)fmaxf(drho, 0.0f) * (double)dt / (double)P.rho0);
-    }
-    }
-    if (kDiv) add_term<kB>(&g.solve[bi].acc_div[slot], term);
-}
-
-template <bool kB, int TPB>
-__global__ void __launch_bounds__(TPB, kB ? FCU_MINB_FORCES_BATCH * 128 / TPB : FCU_MINB_FORCES * 128 / TPB) k_forces_plain(Geo g, SimBufs b, int slot, int gate) {
-#if FCU_SORTED_FORCES
-    const uint32_t i = slot_by_count<TPB>(b.nbr_n, g.n);
-#else
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-#endif
-    forces_eval_body<kB, false>(g, b, i, i < g.n, slot, gate);
-}
-template <bool kB, int TPB>
-__global__ void __launch_bounds__(TPB, kB ? FCU_MINB_FORCES_BATCH * 128 / TPB : FCU_MINB_FORCES * 128 / TPB) k_forces_fused(Geo g, SimBufs b, int slot, int gate) {
-#if FCU_SORTED_FORCES
-    const uint32_t i = slot_by_count<TPB>(b.nbr_n, g.n);
-#else
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-#endif
-    forces_eval_body<kB, true>(g, b, i, i < g.n, slot, gate);
-}
-
 // fingers (sim_solve.wgsl:103-127)
 __device__ __forceinline__ F3 fingers(const FluidStep &st, F3 pos, F3 v) {
     float px = 0.0f, py = 0.0f, weight = 0.0f;
@@ -960,33 +849,188 @@ __device__ __forceinline__ F3 fingers(const FluidStep &st, F3 pos, F3 v) {
     return f3(mixf(v.x, px / weight, a), mixf(v.y, py / weight, a), v.z);
 }
 
-// ---- forces_den_apply (sim_solve.wgsl:630-663) -----------------------------
-template <bool kB, int TPB>
-__global__ void __launch_bounds__(TPB, FCU_MINB) k_forces_apply(Geo g, SimBufs b) {
-    const uint32_t n = g.n;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t bi = box_index<kB>(g, i);
-    const float mass = params_of<kB>(g, bi).mass;
+// ---- forces_eval and forces_den_apply (sim_solve.wgsl:524-592, :630-663) ---
+// One walk of the neighbour list forms both kernels' sums: the forces of
+// forces_eval, and the pressure push of forces_den_apply, whose warm-start
+// kd is a function of each particle's own density and last pressure (in
+// `aux` since density_div) and so does not wait for the forces. The updated
+// velocity and temperature go to fvel / ftemp, since other particles' walks
+// still read the old ones.
+// With kDiv, the same walk also forms the divergence prediction of
+// k_div_kappa (the same pair terms, in the same order, so the same sums):
+// its kappa goes to kd2 / wpk2 and its residual term to acc_div[slot], and
+// boxes whose divergence loop has stopped (gate) are skipped. The tolerance
+// schedule runs this after each divergence apply, so the prediction that
+// only decides whether the loop stops costs no sweep of its own.
+// Measured on the 1M workload (37 neighbours): 488 us against 443 + 107 us
+// for the two kernels apart, the substep 1.953 -> 1.892 ms.
+
+// What a pair needs of its particle and its box.
+struct ForceCtx {
+    KernelConsts K;
+    float mass, inv_h, rho0, soft, coh_c, coh_k, coh_near;
+    F3 pos, vel;
+    float rho, near, temp, kd;
+};
+struct ForceSums {
+    F3 visc, blend, near, tension, push;
+    float heat, drho;
+};
+// One pair's terms, each to be added (or subtracted: blend, tension and
+// heat_out are subtracted) to its sum.
+struct ForceTerms {
+    F3 visc, blend, near, tension, push;
+    float heat_in, heat_out, drho;
+};
+
+template <bool kB>
+__device__ __forceinline__ ForceCtx force_ctx(const Geo &g, const SimBufs &b, const DevParams &P, uint32_t i) {
+    ForceCtx c;
+    c.K = kernel_consts(P);
+    c.mass = P.mass;
+    c.inv_h = P.inv_h;
+    c.rho0 = P.rho0;
+    c.soft = 0.01f * P.h * P.h;
+    c.coh_c = 2.0f * P.h;
+    const float c3 = c.coh_c * c.coh_c * c.coh_c;
+    c.coh_k = 32.0f / (3.14159265f * c3 * c3 * c3);
+    c.coh_near = c3 * c3 / 64.0f;
+    c.pos = xyz(__ldg(&b.wpos[i]));
+    c.vel = xyz(__ldg(&b.wvel[i]));
+    const float4 a = __ldg(&b.aux[i]);
+    c.rho = a.x;
+    c.near = a.y;
+    c.temp = a.z;
+    c.kd = a.w;
+    return c;
+}
+
+template <bool kDiv>
+__device__ __forceinline__ ForceTerms force_pair(const ForceCtx &c, float gs, const Nbr3 &q) {
+    constexpr float visc_k = 2.0f * DYNAMIC_VISCOSITY;
+    constexpr float heat_k = 2.0f * CONDUCTIVITY / HEAT_CAPACITY;
+    constexpr float diss_k = 0.5f * DYNAMIC_VISCOSITY / HEAT_CAPACITY;
+    ForceTerms t;
+    const F3 e = pair_grad(gs, c.pos, q.p);
+    const F3 x = c.pos - xyz(q.p);
+    const float r2 = dot(x, x);
+    const float r = sqrtf(r2);
+    const float rho_j = q.a.x;
+    const float f = dot(x, e) / (r2 + c.soft);
+    const float pair = c.mass / (c.rho * rho_j) * f;
+    const F3 dv = c.vel - xyz(q.v);
+    t.drho = kDiv ? dot(dv, e) : 0.0f;
+    const float wn = fmaxf(1.0f - r * c.inv_h, 0.0f);
+    t.near = ((c.near + q.a.y) * wn * wn) * (x / fmaxf(r, 1e-5f));
+    t.visc = (visc_k * pair) * dv;
+    t.blend = (c.mass / rho_j * kernel_q(c.K, r * c.inv_h)) * dv;
+    t.heat_in = heat_k * pair * (c.temp - q.a.z);
+    t.heat_out = diss_k * pair * dot(dv, dv);
+    const float corr = 2.0f * c.rho0 / (c.rho + rho_j);
+    t.tension = ((corr * c.mass * cohesion(r, c.coh_c, c.coh_k, c.coh_near)) * x) / fmaxf(r, 1e-9f);
+    t.push = (c.kd + q.a.w) * e;
+    return t;
+}
+
+// The particle's own part, from its finished sums: writes every output and,
+// with kDiv, returns the residual term.
+template <bool kB, bool kDiv>
+__device__ __forceinline__ unsigned long long force_finish(const Geo &g, const SimBufs &b, const DevParams &P,
+                                                           uint32_t bi, uint32_t i, const ForceCtx &c, ForceSums s) {
+    const float cc = 2.0f * P.h;
+    const float gamma = SIGMA_WATER * 7040.0f / (21.0f * LATTICE_SIGMA * P.rho0 * P.rho0 * cc * cc);
+    const float beta =
+        SIGMA_WATER * (1.0f + COS_CONTACT) * 1558.4f / (LATTICE_SIGMA * P.rho0 * P.rho0 * cc * cc);
+    const F3 pos = c.pos;
+    const F3 adh = (beta * P.rho0) * wall_adh_sum(P, pos);
+    const F3 acc = s.visc + K_NEAR * s.near + gamma * s.tension + adh;
+    b.accel[i] = make_float4(acc.x, acc.y, acc.z, s.heat);
+    b.xsph[i] = make_float4(s.blend.x, s.blend.y, s.blend.z, 0.0f);
+    b.kd[i] = c.kd;
+    b.pressure[i] = 0.5f * __ldg(&b.wpp[i]);
+    const F3 wg = xyz(__ldg(&b.wgrad[i]));
     const DevStep *stp = &g.st[bi];
     const FluidStep &st = stp->s;
     const float dt = st.dt;
-    const F3 pos = xyz(__ldg(&b.wpos[i]));
-    const float kd_i = b.kd[i];
-    const F3 total = kappa_sum(b, i, n, pos, kd_i);
-    const float4 a = __ldg(&b.accel[i]);
-    const F3 r = pos;
-    const float4 was = b.wvel[i];
+    unsigned long long term = 0;
+    if (kDiv) {  // k_div_kappa's prediction
+        float drho = P.mass * s.drho;
+        drho += dot(c.vel, wg);
+        const float kdd = fmaxf(drho, 0.0f) * __ldg(&b.alpha[i]) / fmaxf(dt, 1e-9f) / c.rho;
+        b.kd2[i] = kdd;
+        b.wpk2[i] = make_float4(pos.x, pos.y, pos.z, kdd);
+        term = fixed_term((double)fmaxf(drho, 0.0f) * (double)dt / (double)P.rho0);
+    }
+    // forces_den_apply
+    const float4 was = __ldg(&b.wvel[i]);
     const F3 v = xyz(was);
     const F3 force = f3(st.force[0], st.force[1], st.force[2]);
     const F3 omega = f3(st.omega[0], st.omega[1], st.omega[2]);
     const F3 domega = f3(st.domega[0], st.domega[1], st.domega[2]);
-    const F3 fict = -cross(domega, r) - cross(omega, cross(omega, r)) - 2.0f * cross(omega, v);
-    const F3 forced = fingers(st, r, v + dt * (force + fict + xyz(a)) + stp->xsph_blend * xyz(__ldg(&b.xsph[i])));
-    b.wtemp[i] += dt * a.w;
-    const F3 dv_full = mass * total + kd_i * xyz(__ldg(&b.wgrad[i]));
+    const F3 fict = -cross(domega, pos) - cross(omega, cross(omega, pos)) - 2.0f * cross(omega, v);
+    const F3 forced = fingers(st, pos, v + dt * (force + fict + acc) + stp->xsph_blend * s.blend);
+    b.ftemp[i] = c.temp + dt * s.heat;
+    const F3 dv_full = P.mass * s.push + c.kd * wg;
     const F3 o = forced - dt * dv_full;
-    b.wvel[i] = make_float4(o.x, o.y, o.z, was.w);
+    b.fvel[i] = make_float4(o.x, o.y, o.z, was.w);
+    return term;
+}
+
+template <bool kB, bool kDiv>
+__device__ __forceinline__ void forces_eval_body(const Geo &g, const SimBufs &b, uint32_t i, bool live,
+                                                 int slot, int gate) {
+    const uint32_t n = g.n;
+    if (!kDiv && !live) return;
+    const uint32_t bi = box_index<kB>(g, live ? i : n - 1);
+    unsigned long long term = 0;
+    if (live && !(kDiv && gated_out<kB>(g, bi, gate))) {
+        // a batch reads its box's constants from the box's entry where they
+        // are used, keeping the pair loop's few in registers; one box copies
+        // them from parameter space
+        DevParams Pc;
+        if (!kB) Pc = g.one;
+        const DevParams &P = kB ? g.box[bi] : Pc;
+        const ForceCtx c = force_ctx<kB>(g, b, P, i);
+        const uint32_t cnt = __ldg(&b.nbr_n[i]);
+        const F3 zero = f3(0.f, 0.f, 0.f);
+        ForceSums s{zero, zero, zero, zero, zero, 0.0f, 0.0f};
+        auto load = [&](uint32_t code) {
+            const uint32_t j = list_slot(code);
+            return Nbr3{__ldg(&b.wpos[j]), __ldg(&b.wvel[j]), __ldg(&b.aux[j])};
+        };
+        walk<FCU_B_N3, Nbr3>(b.nbr, n, i, cnt, load, [&](float gs, const Nbr3 &q) {
+            const ForceTerms t = force_pair<kDiv>(c, gs, q);
+            s.visc = s.visc + t.visc;
+            s.blend = s.blend - t.blend;
+            s.near = s.near + t.near;
+            s.tension = s.tension - t.tension;
+            s.push = s.push + t.push;
+            s.heat += t.heat_in;
+            s.heat -= t.heat_out;
+            if (kDiv) s.drho += t.drho;
+        });
+        term = force_finish<kB, kDiv>(g, b, P, bi, i, c, s);
+    }
+    if (kDiv) add_term<kB>(&g.solve[bi].acc_div[slot], term);
+}
+
+template <bool kB, int TPB>
+__global__ void __launch_bounds__(TPB, FCU_MINB_FORCES * 128 / TPB) k_forces_plain(Geo g, SimBufs b, int slot, int gate) {
+#if FCU_SORTED_FORCES
+    const uint32_t i = slot_by_count<TPB>(b.nbr_n, g.n);
+#else
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+#endif
+    forces_eval_body<kB, false>(g, b, i, i < g.n, slot, gate);
+}
+template <bool kB, int TPB>
+__global__ void __launch_bounds__(TPB, FCU_MINB_FORCES * 128 / TPB) k_forces_fused(Geo g, SimBufs b, int slot, int gate) {
+#if FCU_SORTED_FORCES
+    const uint32_t i = slot_by_count<TPB>(b.nbr_n, g.n);
+#else
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+#endif
+    forces_eval_body<kB, true>(g, b, i, i < g.n, slot, gate);
 }
 
 // ---- den_kappa (sim_solve.wgsl:674-698) ------------------------------------
@@ -1427,9 +1471,6 @@ void launch_forces_eval(cudaStream_t s, const Geo &g, const SimBufs &b) {
 }
 void launch_forces_div(cudaStream_t s, const Geo &g, const SimBufs &b, int slot, int gate) {
     FCU_SWEEP(k_forces_fused, kTuneForcesEval, kSolveThreads, g, b, slot, gate);
-}
-void launch_forces_apply(cudaStream_t s, const Geo &g, const SimBufs &b) {
-    FCU_SWEEP(k_forces_apply, kTuneForcesApply, kSolveThreads, g, b);
 }
 void launch_den_kappa(cudaStream_t s, const Geo &g, const SimBufs &b, int slot, int gate) {
     FCU_SWEEP(k_den_kappa, kTuneDenKappa, kSolveThreads, g, b, slot, gate);

@@ -24,10 +24,18 @@ struct SimBufs {
     float *density, *alpha, *kd, *pressure, *pinc, *rho_near;
     float4 *accel, *xsph, *wgrad;
     float4 *wpk;  // position and kd of the last prediction: apply's one record per neighbour
-    // the divergence loop's own kd and (position, kd) in the tolerance
-    // schedule, where forces_eval also forms the divergence prediction
+    // the divergence solve's own kd and (position, kd): forces_eval, which
+    // writes the warm start's kd, also forms the divergence prediction
     float *kd2;
     float4 *wpk2;
+    // forces_eval's one record per neighbour beside position and velocity:
+    // density, near density, temperature and the warm start's kd
+    float4 *aux;
+    // velocity and temperature after the forces: forces_eval writes them
+    // while other particles still read wvel / wtemp, and the density solve
+    // and integrate go on from them
+    float4 *fvel;
+    float *ftemp;
     // Neighbour list, slot-major (entry k of particle i at k * n + i): the
     // neighbour's slot and the bits of its kernel-gradient scale dw / r,
     // so a sweep forms the gradient (dw / r) * (x_i - x_j) without the
@@ -87,12 +95,26 @@ void launch_gather(cudaStream_t s, const SimBufs &b, uint32_t n);
 void launch_density_div(cudaStream_t s, const Geo &g, const SimBufs &b, int slot);
 void launch_div_kappa(cudaStream_t s, const Geo &g, const SimBufs &b, int slot, int gate);
 void launch_apply(cudaStream_t s, const Geo &g, const SimBufs &b, bool add_pressure, int gate);
+// forces_eval and forces_den_apply in one sweep: reads wvel / wtemp, writes
+// fvel / ftemp.
 void launch_forces_eval(cudaStream_t s, const Geo &g, const SimBufs &b);
-// forces_eval that also forms the divergence prediction (kappa into kd2 /
-// wpk2, residual term into acc_div[slot]), skipping boxes whose divergence
+// The same, also forming the divergence prediction (kappa into kd2 /
+// wpk2, residual term into acc_div[slot]) and skipping boxes whose divergence
 // loop has stopped.
 void launch_forces_div(cudaStream_t s, const Geo &g, const SimBufs &b, int slot, int gate);
-void launch_forces_apply(cudaStream_t s, const Geo &g, const SimBufs &b);
+// The buffers of a sweep after the forces: velocity and temperature from
+// fvel / ftemp.
+inline SimBufs after_forces(SimBufs b) {
+    b.wvel = b.fvel;
+    b.wtemp = b.ftemp;
+    return b;
+}
+// The buffers of the divergence solve's sweeps: kd2 / wpk2.
+inline SimBufs divergence_bufs(SimBufs b) {
+    b.kd = b.kd2;
+    b.wpk = b.wpk2;
+    return b;
+}
 
 void launch_den_kappa(cudaStream_t s, const Geo &g, const SimBufs &b, int slot, int gate);
 // div_slot >= 0: record each box's residuals from those accumulator slots
