@@ -1,4 +1,5 @@
-// solve.cu — DFSPH sweeps for sm_100a, one thread per particle.
+// solve.cu — DFSPH sweeps for sm_100a, one thread per particle (several
+// lanes, in solve_wide.cuh, for counts too small to fill the GPU that way).
 //
 // Reference: crates/fluid-core/src/sim_solve.wgsl (whole file). The reference
 // splits each particle over 8 subgroup lanes; here a particle is one thread
@@ -589,6 +590,35 @@ __device__ __forceinline__ uint32_t density_scan_all(const DevParams &P, uint32_
     return found;
 }
 
+// The particle's own part of density_div (sim_solve.wgsl:475-517), from its
+// finished sums, the walls' fill and their gradient: writes every output and
+// returns the divergence residual's term.
+__device__ __forceinline__ unsigned long long density_finish(const Geo &g, const SimBufs &b, const DevParams &P,
+                                                             uint32_t bi, uint32_t i, F3 pos, F3 vel,
+                                                             const DensitySums &d, float fill, F3 wg) {
+    const float dt = g.st[bi].s.dt;
+    float rho = P.mass * d.w_sum;
+    const float grad_sq = P.mass * P.mass * d.grad_sq;
+    float drho = P.mass * d.drho;
+    F3 grad_sum = P.mass * d.grad_sum;
+    rho += P.rho0 * fill;
+    b.wgrad[i] = make_float4(wg.x, wg.y, wg.z, 0.0f);
+    grad_sum = grad_sum + wg;
+    b.density[i] = rho;
+    b.rho_near[i] = d.rho_near;
+    // the warm start's kd, half the last pressure over rho^2, so that
+    // forces_eval can form forces_den_apply's sum in its own walk
+    const float half = 0.5f * __ldg(&b.wpp[i]);
+    b.aux[i] = make_float4(rho, d.rho_near, __ldg(&b.wtemp[i]), half / (rho * rho));
+    const float a = rho / fmaxf(dot(grad_sum, grad_sum) + grad_sq, 1e-4f);
+    b.alpha[i] = a;
+    drho += dot(vel, wg);
+    const float kdv = fmaxf(drho, 0.0f) * a / fmaxf(dt, 1e-9f) / rho;
+    b.kd[i] = kdv;
+    b.wpk[i] = make_float4(pos.x, pos.y, pos.z, kdv);
+    return fixed_term((double)fmaxf(drho, 0.0f) * (double)dt / (double)P.rho0);
+}
+
 template <bool kB, int TPB>
 __global__ void __launch_bounds__(TPB, (kB ? FCU_MINB_DD_BATCH : FCU_MINB_DD) * 128 / TPB)
     k_density_div(const __grid_constant__ Geo g, SimBufs b, int slot) {
@@ -605,7 +635,6 @@ __global__ void __launch_bounds__(TPB, (kB ? FCU_MINB_DD_BATCH : FCU_MINB_DD) * 
         const DevParams &P = params_ref<kB>(g, bi);
         const KernelConsts K = kernel_consts(P);
         const uint32_t base = cell_base_of<kB>(g, bi);
-        const float dt = g.st[bi].s.dt;
         const F3 pos = xyz(__ldg(&b.wpos[i]));
         const F3 vel = xyz(__ldg(&b.wvel[i]));
         const Stencil t = stencil_of(P, pos);
@@ -710,14 +739,8 @@ __global__ void __launch_bounds__(TPB, (kB ? FCU_MINB_DD_BATCH : FCU_MINB_DD) * 
         } else {
             found = density_scan_all<(int)kSimSlabs>(P, base, b, n, i, pos, vel, t, d);
         }
-        // sim_solve.wgsl:475-517
         b.nbr_n[i] = found < cap ? found : cap;
         if (found > cap) atomicAdd(&g.solve[bi].nbr_over, found - cap);
-        float rho = P.mass * d.w_sum;
-        const float rho_near = d.rho_near;
-        const float grad_sq = P.mass * P.mass * d.grad_sq;
-        float drho = P.mass * d.drho;
-        F3 grad_sum = P.mass * d.grad_sum;
         const F3 lo = wall_lo(P), hi = wall_hi(P);
         const F3 tl = (pos - lo) * P.inv_h;
         const F3 th = (hi - pos) * P.inv_h;
@@ -726,23 +749,7 @@ __global__ void __launch_bounds__(TPB, (kB ? FCU_MINB_DD_BATCH : FCU_MINB_DD) * 
         fill += wall_density(tl.y) + wall_density(th.y);
         fill += wall_density(tl.z) + wall_density(th.z);
         fill -= wedge_sum(tl, th);
-        rho += P.rho0 * fill;
-        const F3 wg = wall_grad_sum(P, pos);
-        b.wgrad[i] = make_float4(wg.x, wg.y, wg.z, 0.0f);
-        grad_sum = grad_sum + wg;
-        b.density[i] = rho;
-        b.rho_near[i] = rho_near;
-        // the warm start's kd, half the last pressure over rho^2, so that
-        // forces_eval can form forces_den_apply's sum in its own walk
-        const float half = 0.5f * __ldg(&b.wpp[i]);
-        b.aux[i] = make_float4(rho, rho_near, __ldg(&b.wtemp[i]), half / (rho * rho));
-        const float a = rho / fmaxf(dot(grad_sum, grad_sum) + grad_sq, 1e-4f);
-        b.alpha[i] = a;
-        drho += dot(vel, wg);
-        const float kdv = fmaxf(drho, 0.0f) * a / fmaxf(dt, 1e-9f) / rho;
-        b.kd[i] = kdv;
-        b.wpk[i] = make_float4(pos.x, pos.y, pos.z, kdv);
-        term = fixed_term((double)fmaxf(drho, 0.0f) * (double)dt / (double)P.rho0);
+        term = density_finish(g, b, P, bi, i, pos, vel, d, fill, wall_grad_sum(P, pos));
     }
     add_term<kB>(&g.solve[bi].acc_div[slot], term);
 }
@@ -759,6 +766,31 @@ __device__ __forceinline__ bool gated_out(const Geo &g, uint32_t bi, int gate) {
 // ---- divergence predictor for a later divergence iteration ---------------
 // density_div's divergence sums again over the list, with this
 // iteration's velocities.
+__device__ __forceinline__ unsigned long long div_kappa_finish(const Geo &g, const SimBufs &b, const DevParams &P,
+                                                               uint32_t bi, uint32_t i, float sum) {
+    const float dt = g.st[bi].s.dt;
+    const F3 pos = xyz(__ldg(&b.wpos[i]));
+    const F3 vel = xyz(__ldg(&b.wvel[i]));
+    float drho = P.mass * sum;
+    drho += dot(vel, xyz(__ldg(&b.wgrad[i])));
+    const float rho = __ldg(&b.density[i]);
+    const float kdv = fmaxf(drho, 0.0f) * __ldg(&b.alpha[i]) / fmaxf(dt, 1e-9f) / rho;
+    b.kd[i] = kdv;
+    b.wpk[i] = make_float4(pos.x, pos.y, pos.z, kdv);
+    return fixed_term((double)fmaxf(drho, 0.0f) * (double)dt / (double)P.rho0);
+}
+
+// The sum both predictions form: (v_i - v_j) . grad W over the list.
+__device__ __forceinline__ float divergence_sum(const SimBufs &b, uint32_t n, uint32_t i, F3 pos, F3 vel) {
+    const uint32_t cnt = __ldg(&b.nbr_n[i]);
+    float drho = 0.0f;
+    walk<FCU_B_PV, PosVel>(
+        b.nbr, n, i, cnt,
+        [&](uint32_t j) { return PosVel{__ldg(&b.wpos[j]), __ldg(&b.wvel[j])}; },
+        [&](float gs, const PosVel &q) { drho += dot(vel - xyz(q.v), pair_grad(gs, pos, q.p)); });
+    return drho;
+}
+
 template <bool kB, int TPB>
 __global__ void __launch_bounds__(TPB, kB ? kBatchKappaThreads / TPB : FCU_MINB_KAPPA) k_div_kappa(Geo g, SimBufs b, int slot,
                                                                        int gate) {
@@ -769,22 +801,9 @@ __global__ void __launch_bounds__(TPB, kB ? kBatchKappaThreads / TPB : FCU_MINB_
     unsigned long long term = 0;
     if (live && !gated_out<kB>(g, bi, gate)) {
         const DevParams P = params_of<kB>(g, bi);
-        const float dt = g.st[bi].s.dt;
         const F3 pos = xyz(__ldg(&b.wpos[i]));
         const F3 vel = xyz(__ldg(&b.wvel[i]));
-        const uint32_t cnt = __ldg(&b.nbr_n[i]);
-        float drho = 0.0f;
-        walk<FCU_B_PV, PosVel>(
-            b.nbr, n, i, cnt,
-            [&](uint32_t j) { return PosVel{__ldg(&b.wpos[j]), __ldg(&b.wvel[j])}; },
-            [&](float gs, const PosVel &q) { drho += dot(vel - xyz(q.v), pair_grad(gs, pos, q.p)); });
-        drho = P.mass * drho;
-        drho += dot(vel, xyz(__ldg(&b.wgrad[i])));
-        const float rho = __ldg(&b.density[i]);
-        const float kdv = fmaxf(drho, 0.0f) * __ldg(&b.alpha[i]) / fmaxf(dt, 1e-9f) / rho;
-        b.kd[i] = kdv;
-        b.wpk[i] = make_float4(pos.x, pos.y, pos.z, kdv);
-        term = fixed_term((double)fmaxf(drho, 0.0f) * (double)dt / (double)P.rho0);
+        term = div_kappa_finish(g, b, P, bi, i, divergence_sum(b, n, i, pos, vel));
     }
     add_term<kB>(&g.solve[bi].acc_div[slot], term);
 }
@@ -805,6 +824,15 @@ __device__ __forceinline__ F3 kappa_sum(const SimBufs &b, uint32_t i, uint32_t n
 // ---- apply_kappa_wide: div_apply / den_apply (sim_solve.wgsl:608-621) -----
 // For the density iterations the applied pressure k*rho that den_kappa held
 // back joins the pressure here, with the kappa it belongs to.
+__device__ __forceinline__ void apply_finish(const Geo &g, const SimBufs &b, float mass, uint32_t bi, uint32_t i,
+                                             float kd_i, F3 total, int add_pressure) {
+    const float dt = g.st[bi].s.dt;
+    const F3 dv_full = mass * total + kd_i * xyz(__ldg(&b.wgrad[i]));
+    const float4 was = b.wvel[i];
+    const F3 v = xyz(was) - dt * dv_full;
+    b.wvel[i] = make_float4(v.x, v.y, v.z, was.w);
+    if (add_pressure) b.pressure[i] += b.pinc[i];
+}
 template <bool kB>
 __device__ __forceinline__ void apply_at(const Geo &g, const SimBufs &b, uint32_t i, int add_pressure,
                                          int gate) {
@@ -812,15 +840,9 @@ __device__ __forceinline__ void apply_at(const Geo &g, const SimBufs &b, uint32_
     const uint32_t bi = box_index<kB>(g, i);
     if (gated_out<kB>(g, bi, gate)) return;
     const float mass = params_of<kB>(g, bi).mass;
-    const float dt = g.st[bi].s.dt;
     const F3 pos = xyz(__ldg(&b.wpos[i]));
     const float kd_i = b.kd[i];
-    const F3 total = kappa_sum(b, i, n, pos, kd_i);
-    const F3 dv_full = mass * total + kd_i * xyz(__ldg(&b.wgrad[i]));
-    const float4 was = b.wvel[i];
-    const F3 v = xyz(was) - dt * dv_full;
-    b.wvel[i] = make_float4(v.x, v.y, v.z, was.w);
-    if (add_pressure) b.pressure[i] += b.pinc[i];
+    apply_finish(g, b, mass, bi, i, kd_i, kappa_sum(b, i, n, pos, kd_i), add_pressure);
 }
 
 template <bool kB, int TPB>
@@ -883,8 +905,7 @@ struct ForceTerms {
     float heat_in, heat_out, drho;
 };
 
-template <bool kB>
-__device__ __forceinline__ ForceCtx force_ctx(const Geo &g, const SimBufs &b, const DevParams &P, uint32_t i) {
+__device__ __forceinline__ ForceCtx force_ctx(const SimBufs &b, const DevParams &P, uint32_t i) {
     ForceCtx c;
     c.K = kernel_consts(P);
     c.mass = P.mass;
@@ -934,7 +955,7 @@ __device__ __forceinline__ ForceTerms force_pair(const ForceCtx &c, float gs, co
 
 // The particle's own part, from its finished sums: writes every output and,
 // with kDiv, returns the residual term.
-template <bool kB, bool kDiv>
+template <bool kDiv>
 __device__ __forceinline__ unsigned long long force_finish(const Geo &g, const SimBufs &b, const DevParams &P,
                                                            uint32_t bi, uint32_t i, const ForceCtx &c, ForceSums s) {
     const float cc = 2.0f * P.h;
@@ -990,7 +1011,7 @@ __device__ __forceinline__ void forces_eval_body(const Geo &g, const SimBufs &b,
         DevParams Pc;
         if (!kB) Pc = g.one;
         const DevParams &P = kB ? g.box[bi] : Pc;
-        const ForceCtx c = force_ctx<kB>(g, b, P, i);
+        const ForceCtx c = force_ctx(b, P, i);
         const uint32_t cnt = __ldg(&b.nbr_n[i]);
         const F3 zero = f3(0.f, 0.f, 0.f);
         ForceSums s{zero, zero, zero, zero, zero, 0.0f, 0.0f};
@@ -1009,7 +1030,7 @@ __device__ __forceinline__ void forces_eval_body(const Geo &g, const SimBufs &b,
             s.heat -= t.heat_out;
             if (kDiv) s.drho += t.drho;
         });
-        term = force_finish<kB, kDiv>(g, b, P, bi, i, c, s);
+        term = force_finish<kDiv>(g, b, P, bi, i, c, s);
     }
     if (kDiv) add_term<kB>(&g.solve[bi].acc_div[slot], term);
 }
@@ -1034,42 +1055,38 @@ __global__ void __launch_bounds__(TPB, FCU_MINB_FORCES * 128 / TPB) k_forces_fus
 }
 
 // ---- den_kappa (sim_solve.wgsl:674-698) ------------------------------------
-template <bool kB>
-__device__ __forceinline__ void den_kappa_at(const Geo &g, const SimBufs &b, uint32_t i, bool live, int slot,
-                                             int gate) {
-    const uint32_t n = g.n;
-    const uint32_t bi = box_index<kB>(g, live ? i : n - 1);
-    unsigned long long term = 0;
-    if (live && !gated_out<kB>(g, bi, gate)) {
-        const DevParams P = params_of<kB>(g, bi);
-        const float mass = P.mass, rho0 = P.rho0;
-        const float dt = g.st[bi].s.dt;
-        const F3 pos = xyz(__ldg(&b.wpos[i]));
-        const F3 vel = xyz(__ldg(&b.wvel[i]));
-        const uint32_t cnt = __ldg(&b.nbr_n[i]);
-        float drho = 0.0f;
-        walk<FCU_B_PV, PosVel>(
-            b.nbr, n, i, cnt,
-            [&](uint32_t j) { return PosVel{__ldg(&b.wpos[j]), __ldg(&b.wvel[j])}; },
-            [&](float gs, const PosVel &q) { drho += dot(vel - xyz(q.v), pair_grad(gs, pos, q.p)); });
-        const float rho = __ldg(&b.density[i]);
-        drho = mass * drho + dot(vel, xyz(__ldg(&b.wgrad[i])));
-        const float rho_star = rho + dt * drho;
-        const float kk = fmaxf(rho_star - rho0, 0.0f) * __ldg(&b.alpha[i]) / (dt * dt);
-        const float kdv = kk / rho;
-        b.kd[i] = kdv;
-        b.wpk[i] = make_float4(pos.x, pos.y, pos.z, kdv);
-        b.pinc[i] = kk * rho;
-        term = fixed_term((double)rho_star / (double)rho0 - 1.0);
-    }
-    add_term<kB>(&g.solve[bi].acc_den[slot], term);
+__device__ __forceinline__ unsigned long long den_kappa_finish(const Geo &g, const SimBufs &b, const DevParams &P,
+                                                               uint32_t bi, uint32_t i, float sum) {
+    const float mass = P.mass, rho0 = P.rho0;
+    const float dt = g.st[bi].s.dt;
+    const F3 pos = xyz(__ldg(&b.wpos[i]));
+    const F3 vel = xyz(__ldg(&b.wvel[i]));
+    const float rho = __ldg(&b.density[i]);
+    const float drho = mass * sum + dot(vel, xyz(__ldg(&b.wgrad[i])));
+    const float rho_star = rho + dt * drho;
+    const float kk = fmaxf(rho_star - rho0, 0.0f) * __ldg(&b.alpha[i]) / (dt * dt);
+    const float kdv = kk / rho;
+    b.kd[i] = kdv;
+    b.wpk[i] = make_float4(pos.x, pos.y, pos.z, kdv);
+    b.pinc[i] = kk * rho;
+    return fixed_term((double)rho_star / (double)rho0 - 1.0);
 }
 
 template <bool kB, int TPB>
 __global__ void __launch_bounds__(TPB, kB ? kBatchKappaThreads / TPB : FCU_MINB_KAPPA) k_den_kappa(Geo g, SimBufs b, int slot,
                                                                        int gate) {
+    const uint32_t n = g.n;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    den_kappa_at<kB>(g, b, i, i < g.n, slot, gate);
+    const bool live = i < n;
+    const uint32_t bi = box_index<kB>(g, live ? i : n - 1);
+    unsigned long long term = 0;
+    if (live && !gated_out<kB>(g, bi, gate)) {
+        const DevParams P = params_of<kB>(g, bi);
+        const F3 pos = xyz(__ldg(&b.wpos[i]));
+        const F3 vel = xyz(__ldg(&b.wvel[i]));
+        term = den_kappa_finish(g, b, P, bi, i, divergence_sum(b, n, i, pos, vel));
+    }
+    add_term<kB>(&g.solve[bi].acc_den[slot], term);
 }
 
 // ---- integrate (sim_solve.wgsl:709-756) ------------------------------------
@@ -1431,6 +1448,8 @@ __global__ void __launch_bounds__(256) k_advect(DevParams P, SimBufs b, DevStep 
     store_tracer(P, b.tracers, i, tracer_clamp(P, pos), fmaxf(len(v), old[3] * stp->decay));
 }
 
+#include "solve_wide.cuh"
+
 inline uint32_t blocks_for(uint32_t n, uint32_t t) { return (n + t - 1) / t; }
 
 }  // namespace
@@ -1450,37 +1469,78 @@ void launch_gather(cudaStream_t s, const SimBufs &b, uint32_t n) {
     } while (0)
 #define FCU_SWEEP(kern, slot_id, deflt, ...)                                            \
     do {                                                                                \
-        if (!g.n) return;                                                               \
         const int tpb_ = g.tpb[slot_id] ? (int)g.tpb[slot_id] : (deflt);                \
         if (tpb_ == 64) FCU_SWEEP_AT(kern, 64, __VA_ARGS__);                            \
         else if (tpb_ == 256) FCU_SWEEP_AT(kern, 256, __VA_ARGS__);                     \
         else FCU_SWEEP_AT(kern, 128, __VA_ARGS__);                                      \
     } while (0)
 
+// Lanes per particle of the sweeps at this particle count: the most (up to a
+// warp) that keep the launch within about one block wave of the GPU, 1 (the
+// one-thread sweeps) when even four do not. More lanes shorten one particle's
+// walk but add work (idle places of the last chunk, the fold); once the GPU
+// is full they only cost. Measured, us a substep by lanes 1 / 4 / 8 / 16 / 32:
+// 1,620 particles 212 / 154 / 135 / 125 / 123, 16,384 207 / 152 / 147 / 161 /
+// 174, 41,796 (a batch) 267 / 249 / 253 / 290 / 355, 72,072 260 / 285 / 309 /
+// 390 / 503.
+constexpr uint32_t kWideMost = 148u * 1200u;
+inline int lanes_for(uint32_t n) {
+    for (int lanes = 32; lanes >= 4; lanes >>= 1)
+        if ((uint64_t)n * lanes <= kWideMost) return lanes;
+    return 1;
+}
+#define FCU_WIDE_AT(L, one, batch, ...)                                                                     \
+    do {                                                                                                    \
+        const uint32_t blocks_ = blocks_for(g.n, kWideThreads / L);                                         \
+        if (g.box_of) batch<<<blocks_, kWideThreads, 0, s>>>(__VA_ARGS__);                                  \
+        else one<<<blocks_, kWideThreads, 0, s>>>(__VA_ARGS__);                                             \
+    } while (0)
+// A sweep at lanes_for(n) lanes: `wide` with each particle's list shared by
+// that many lanes, or the one-thread kernel.
+#define FCU_SWEEP_WIDE(wide, kern, slot_id, ...)                                                            \
+    do {                                                                                                    \
+        if (!g.n) return;                                                                                   \
+        switch (lanes_for(g.n)) {                                                                           \
+        case 32: FCU_WIDE_AT(32, (wide<false, 32>), (wide<true, 32>), __VA_ARGS__); break;                  \
+        case 16: FCU_WIDE_AT(16, (wide<false, 16>), (wide<true, 16>), __VA_ARGS__); break;                  \
+        case 8: FCU_WIDE_AT(8, (wide<false, 8>), (wide<true, 8>), __VA_ARGS__); break;                      \
+        case 4: FCU_WIDE_AT(4, (wide<false, 4>), (wide<true, 4>), __VA_ARGS__); break;                      \
+        default: FCU_SWEEP(kern, slot_id, kSolveThreads, __VA_ARGS__);                                      \
+        }                                                                                                   \
+    } while (0)
+
+template <bool kB, int L>
+constexpr auto k_forces_plain_wide = k_forces_wide<kB, false, L>;
+template <bool kB, int L>
+constexpr auto k_forces_fused_wide = k_forces_wide<kB, true, L>;
+
 void launch_density_div(cudaStream_t s, const Geo &g, const SimBufs &b, int slot) {
-    FCU_SWEEP(k_density_div, kTuneDensity, kSolveThreads, g, b, slot);
+    FCU_SWEEP_WIDE(k_density_wide, k_density_div, kTuneDensity, g, b, slot);
 }
 void launch_div_kappa(cudaStream_t s, const Geo &g, const SimBufs &b, int slot, int gate) {
-    FCU_SWEEP(k_div_kappa, kTuneDivKappa, kSolveThreads, g, b, slot, gate);
+    FCU_SWEEP_WIDE(k_div_kappa_wide, k_div_kappa, kTuneDivKappa, g, b, slot, gate);
 }
 void launch_apply(cudaStream_t s, const Geo &g, const SimBufs &b, bool add_pressure, int gate) {
-    FCU_SWEEP(k_apply, kTuneApply, kSolveThreads, g, b, add_pressure ? 1 : 0, gate);
+    FCU_SWEEP_WIDE(k_apply_wide, k_apply, kTuneApply, g, b, add_pressure ? 1 : 0, gate);
 }
 void launch_forces_eval(cudaStream_t s, const Geo &g, const SimBufs &b) {
-    FCU_SWEEP(k_forces_plain, kTuneForcesEval, kSolveThreads, g, b, 0, kGateNone);
+    FCU_SWEEP_WIDE(k_forces_plain_wide, k_forces_plain, kTuneForcesEval, g, b, 0, kGateNone);
 }
 void launch_forces_div(cudaStream_t s, const Geo &g, const SimBufs &b, int slot, int gate) {
-    FCU_SWEEP(k_forces_fused, kTuneForcesEval, kSolveThreads, g, b, slot, gate);
+    FCU_SWEEP_WIDE(k_forces_fused_wide, k_forces_fused, kTuneForcesEval, g, b, slot, gate);
 }
 void launch_den_kappa(cudaStream_t s, const Geo &g, const SimBufs &b, int slot, int gate) {
-    FCU_SWEEP(k_den_kappa, kTuneDenKappa, kSolveThreads, g, b, slot, gate);
+    FCU_SWEEP_WIDE(k_den_kappa_wide, k_den_kappa, kTuneDenKappa, g, b, slot, gate);
 }
 void launch_integrate(cudaStream_t s, const Geo &g, const SimBufs &b, int div_slot, int den_slot,
                       int div_iters, int den_iters) {
+    if (!g.n) return;
     FCU_SWEEP(k_integrate, kTuneIntegrate, 256, g, b, div_slot, den_slot, div_iters, den_iters);
 }
 #undef FCU_SWEEP_AT
 #undef FCU_SWEEP
+#undef FCU_WIDE_AT
+#undef FCU_SWEEP_WIDE
 
 void launch_tol_finish(cudaStream_t s, const Geo &g, int which, int first, float tol,
                        uint32_t max_iters, cudaGraphConditionalHandle handle) {
