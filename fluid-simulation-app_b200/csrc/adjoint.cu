@@ -1385,8 +1385,7 @@ struct AdjImpl : AdjBase {
     cudaStream_t stream = nullptr;
     std::vector<void *> allocs;
     // grid
-    GridWork gw{};
-    void *grid_ws = nullptr;
+    CountGrid gw{};
     float4 *pos4 = nullptr;
     uint32_t *keys = nullptr, *starts = nullptr, *perm = nullptr, *over = nullptr;
     // state and its checkpoints
@@ -1431,7 +1430,6 @@ struct AdjImpl : AdjBase {
         cudaSetDevice(device);
         if (stream) cudaStreamSynchronize(stream);
         for (void *p : allocs) cudaFree(p);
-        if (grid_ws) cudaFree(grid_ws);
         if (stream) cudaStreamDestroy(stream);
     }
 
@@ -1492,8 +1490,13 @@ struct AdjImpl : AdjBase {
         AK(alloc(&starts, (size_t)cells + 1));
         AK(alloc(&perm, N));
         AK(alloc(&over, 1));
-        AK(cudaMalloc(&grid_ws, grid_work_bytes(n, cells)));
-        gw = grid_work_carve(grid_ws, n, cells, nullptr);
+        char *grid_ws = nullptr;
+        uint32_t *grid_err = nullptr;
+        AK(alloc(&grid_err, 1));
+        AK(alloc(&grid_ws, count_grid_bytes(n, cells)));
+        AK(cudaMemset(grid_ws, 0, count_grid_bytes(n, cells)));
+        AK(cudaMemset(grid_err, 0, 4));
+        gw = count_grid_carve(grid_ws, n, cells, keys, starts, perm, grid_err);
         AK(alloc(&x, N));
         AK(alloc(&v, N));
         AK(alloc(&pp, N));
@@ -1569,9 +1572,8 @@ struct AdjImpl : AdjBase {
             g.dims[a] = P.dims[a];
         }
         g.cell = P.cell;
-        g.slabs = kAdjSlabs;
-        AK(cudaMemsetAsync(gw.err, 0, 4, stream));
-        AK(grid_build_enqueue(stream, pos4, n, g, keys, starts, perm, gw, nullptr, nullptr, nullptr, 1));
+        AK(count_grid_enqueue(stream, pos4, g, nullptr, gw, StepRing{}));
+        AK(count_grid_order(stream, gw, nullptr));
         return FLUID_OK;
     }
 

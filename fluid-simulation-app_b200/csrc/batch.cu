@@ -54,15 +54,6 @@ namespace {
 constexpr uint32_t kBatchRing = 128;  // substeps of Step blocks in flight
 constexpr uint32_t kMaxBoxes = 65535;
 
-// Clears every box's residual accumulators (the substep's first launch).
-__global__ void __launch_bounds__(128) k_clear_acc(DevSolve *solve) {
-    DevSolve *sv = &solve[blockIdx.x];
-    for (int k = threadIdx.x; k < kAccSlots; k += blockDim.x) {
-        sv->acc_div[k] = 0ull;
-        sv->acc_den[k] = 0ull;
-    }
-}
-
 }  // namespace
 
 struct FluidBatch {
@@ -75,8 +66,7 @@ struct FluidBatch {
     int device = 0;
     cudaStream_t stream = nullptr, side = nullptr;
     SimBufs b{};
-    GridWork gw{};
-    void *grid_ws = nullptr;
+    CountGrid gw{};
     DevParams *d_box = nullptr;
     uint16_t *d_box_of = nullptr;
     uint32_t *d_cell_base = nullptr, *d_first = nullptr;
@@ -101,7 +91,16 @@ struct FluidBatch {
         for (int k = 0; k < 8; ++k) g.tpb[k] = tpb[k];
         return g;
     }
-    BoxKeys keys() const { return BoxKeys{d_box_of, d_box, d_cell_base, nboxes, kSimSlabs}; }
+    BoxKeys keys() const { return BoxKeys{d_box_of, d_box, d_cell_base}; }
+    // The grid of every box and the records in cell order; with `steps` the
+    // substep's Step blocks come from the ring.
+    cudaError_t build_grid(cudaStream_t st, bool steps) const {
+        const BoxKeys bk = keys();
+        const StepRing r{steps ? ring : nullptr, cur, solve, kBatchRing, nboxes};
+        const cudaError_t e = count_grid_enqueue(st, b.pos, GridGeom{}, &bk, gw, r);
+        const GridGather records = gather_of(b);
+        return e == cudaSuccess ? count_grid_order(st, gw, &records) : e;
+    }
 
     template <class T>
     cudaError_t alloc(T **p, size_t cnt) {
@@ -119,14 +118,10 @@ namespace {
 
 // One substep of every box at a fixed schedule (the one-box sequence).
 cudaError_t batch_enqueue(FluidBatch *s, cudaStream_t st, uint32_t div_iters, uint32_t den_iters) {
-    k_clear_acc<<<s->nboxes, 128, 0, st>>>(s->solve);
-    const BoxKeys bk = s->keys();
-    cudaError_t e = grid_build_enqueue(st, s->b.pos, s->n, GridGeom{}, s->b.keys, s->b.starts, s->b.perm,
-                                       s->gw, s->ring, s->cur, s->solve, kBatchRing, &bk);
+    cudaError_t e = s->build_grid(st, true);
     if (e != cudaSuccess) return e;
     const Geo g = s->geo();
     const SimBufs bd = divergence_bufs(s->b), bf = after_forces(s->b);
-    launch_gather(st, s->b, s->n);
     launch_density_div(st, g, bd, 0);
     for (uint32_t d = 0; d < div_iters; ++d) {
         if (d > 0) launch_div_kappa(st, g, bd, (int)d, kGateNone);
@@ -183,17 +178,13 @@ int32_t batch_graph_tolerance(FluidBatch *s, cudaGraphExec_t *out) {
     cudaGraph_t bdiv = nullptr, bden = nullptr;
     BK(cudaStreamBeginCaptureToGraph(st, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     int32_t rc = FLUID_OK;
-    k_clear_acc<<<s->nboxes, 128, 0, st>>>(s->solve);
-    const BoxKeys bk = s->keys();
-    cudaError_t e = grid_build_enqueue(st, s->b.pos, s->n, GridGeom{}, s->b.keys, s->b.starts, s->b.perm,
-                                       s->gw, s->ring, s->cur, s->solve, kBatchRing, &bk);
+    cudaError_t e = s->build_grid(st, true);
     const Geo geo = s->geo();
     // forces_eval after every divergence apply, forming the prediction that
     // decides the loop (as the one-box tolerance substep)
     const bool fused = c.max_iters >= 1;
     const SimBufs bd = divergence_bufs(s->b), bf = after_forces(s->b);
     if (e == cudaSuccess) {
-        launch_gather(st, s->b, s->n);
         launch_density_div(st, geo, bd, 0);
         launch_tol_finish(st, geo, 0, 1, c.div_tol, c.max_iters, hdiv);
         rc = host_add_while(st, g, hdiv, &bdiv);
@@ -362,9 +353,10 @@ int32_t batch_create_into(FluidBatch *s, const FluidSimConfig *boxes, uint32_t n
     BK(s->alloc(&s->cur, nb));
     BK(s->alloc(&s->solve, nb));
 
-    const size_t wsb = grid_work_bytes(s->n, s->cells);
-    BK(cudaMalloc(&s->grid_ws, wsb));
-    s->gw = grid_work_carve(s->grid_ws, s->n, s->cells, &s->solve[0].error);
+    const size_t wsb = count_grid_bytes(s->n, s->cells);
+    char *grid_ws = nullptr;
+    BK(s->alloc(&grid_ws, wsb));
+    s->gw = count_grid_carve(grid_ws, s->n, s->cells, b.keys, b.starts, b.perm, &s->solve[0].error);
     BK(cudaMallocHost(&s->h_ring, (size_t)kBatchRing * nb * sizeof(DevStep)));
 
     std::vector<float> zeros4(4 * n, 0.0f), zeros(n, 0.0f);
@@ -376,6 +368,7 @@ int32_t batch_create_into(FluidBatch *s, const FluidSimConfig *boxes, uint32_t n
     BK(cudaMemcpy(b.id, ids.data(), 4 * n, cudaMemcpyHostToDevice));
     for (float *z : {b.density, b.alpha, b.kd, b.pressure, b.pinc, b.rho_near}) BK(cudaMemset(z, 0, 4 * n));
     BK(cudaMemset(b.nbr_n, 0, 4 * n));
+    BK(cudaMemset(grid_ws, 0, wsb));
     BK(cudaMemset(b.stats_acc, 0, 8 * nb));
     BK(cudaMemset(b.stats, 0, 64 * nb));
     BK(cudaMemcpy(s->d_box, s->P.data(), nb * sizeof(DevParams), cudaMemcpyHostToDevice));
@@ -399,7 +392,6 @@ void fluid_batch_destroy(FluidBatch *s) {
     for (auto &kv : s->graphs) cudaGraphExecDestroy(kv.second);
     if (s->tol_graph) cudaGraphExecDestroy(s->tol_graph);
     for (void *p : s->allocs) cudaFree(p);
-    if (s->grid_ws) cudaFree(s->grid_ws);
     if (s->h_ring) cudaFreeHost(s->h_ring);
     if (s->side) cudaStreamDestroy(s->side);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -574,11 +566,7 @@ int32_t timed_substep(FluidBatch *s, int tpb, float *ms, cudaEvent_t *ev) {
     cudaStream_t st = s->stream;
     Geo g = s->geo();
     for (int k = 0; k < kTuneCount; ++k) g.tpb[k] = (uint16_t)tpb;
-    k_clear_acc<<<s->nboxes, 128, 0, st>>>(s->solve);
-    const BoxKeys bk = s->keys();
-    BK(grid_build_enqueue(st, s->b.pos, s->n, GridGeom{}, s->b.keys, s->b.starts, s->b.perm, s->gw,
-                          nullptr, nullptr, s->solve, kBatchRing, &bk));
-    launch_gather(st, s->b, s->n);
+    BK(s->build_grid(st, false));
     int e = 0;
     auto timed = [&](int slot, auto &&launch) {
         cudaEventRecord(ev[e], st);

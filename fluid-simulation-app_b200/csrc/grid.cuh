@@ -9,9 +9,6 @@ struct GridGeom {
     float min[3];
     float cell;
     uint32_t dims[3];
-    // slabs > 1: each cell is cut into that many slabs along x and the key
-    // is cell * slabs + slab, so a cell's slots are in slab order
-    uint32_t slabs = 1;
 };
 
 constexpr int kScanThreads = 256;
@@ -67,27 +64,65 @@ int32_t read_build_status(const uint32_t *err, cudaStream_t stream, const char *
 // publishes: its bounded look-back waits give up and set w.err.
 cudaError_t enqueue_stalled_radix_pass(const GridWork &w, cudaStream_t stream);
 
+// Enqueues keys -> stable radix sort -> starts on `stream`. `keys` receives
+// each input's cell key, `starts` the exclusive scan of the cell counts with
+// starts[cells] = n, `perm` the stable permutation.
+cudaError_t grid_build_enqueue(cudaStream_t stream, const float4 *pos, uint32_t n, const GridGeom &g, uint32_t *keys,
+                               uint32_t *starts, uint32_t *perm, GridWork &w);
+
+// ---- the simulations' grid, by counting ----------------------------------------
+// Keys are cell * kSimSlabs + x slab, so a cell's slots are in slab order.
+constexpr int kCountThreads = 256;
+constexpr int kCountItems = 4;  // positions per thread of the key kernel
+
 // A batch of boxes sharing one grid: slot i belongs to box box_of[i], whose
-// keys are cell_base[b] .. cell_base[b] + its cells * slabs - 1 (the boxes'
-// key ranges laid end to end, in box order; key cell * slabs + x slab).
+// keys are cell_base[b] .. cell_base[b] + its cells * kSimSlabs - 1 (the
+// boxes' key ranges laid end to end, in box order).
 struct BoxKeys {
     const uint16_t *box_of;     // [n]
     const DevParams *box;       // [nboxes]
     const uint32_t *cell_base;  // [nboxes]
-    uint32_t nboxes;
-    uint32_t slabs = 1;
 };
 
-// Enqueues keys -> stable radix sort -> starts on `stream`. `keys` receives
-// each input's cell key, `starts` the exclusive scan of the cell counts with
-// starts[cells] = n, `perm` the stable permutation. `ring`/`cur`/`solve`
-// (may be null) let the key kernel
-// also fetch the substep's Step block from the ring. With `boxes`, the keys
-// are the batch's (`g` unused) and every box's Step block of the substep
-// (ring entry cursor holds nboxes of them) moves to cur[0 .. nboxes-1].
-cudaError_t grid_build_enqueue(cudaStream_t stream, const float4 *pos, uint32_t n,
-                               const GridGeom &g, uint32_t *keys, uint32_t *starts,
-                               uint32_t *perm, GridWork &w, const DevStep *ring, DevStep *cur,
-                               DevSolve *solve, uint32_t ring_size, const BoxKeys *boxes = nullptr);
+// Buffers of a counting build of `cells` keys: `count` and `ctl` are zero
+// between builds (each build leaves them so), `order` holds indices below n.
+struct CountGrid {
+    uint32_t *keys, *count, *rank, *order, *starts, *perm;
+    unsigned long long *ctl;  // the scan's look-back words
+    uint32_t ctl_words;
+    uint32_t *err;
+    uint32_t n, cells;
+};
+// One allocation for count, rank, order and ctl; zero it once.
+size_t count_grid_bytes(uint32_t n, uint32_t cells);
+CountGrid count_grid_carve(void *ws, uint32_t n, uint32_t cells, uint32_t *keys, uint32_t *starts, uint32_t *perm,
+                           uint32_t *err);
+
+// What the key kernel does for the substep beside the keys: with `solve`,
+// clears every box's residual accumulators, and with `ring` moves the
+// substep's nboxes Step blocks (ring entry `cursor`) into cur[0 .. nboxes-1].
+struct StepRing {
+    const DevStep *ring = nullptr;
+    DevStep *cur = nullptr;
+    DevSolve *solve = nullptr;
+    uint32_t size = 1, nboxes = 1;
+};
+
+// The particle records k_order moves into cell order with the permutation.
+struct GridGather {
+    const float4 *pos, *vel, *pvel;
+    const float *pp, *temp;
+    const uint32_t *id;
+    float4 *wpos, *wvel, *wpvel;
+    float *wpp, *wtemp;
+    uint32_t *wid;
+};
+
+// Keys, starts (starts[cells] = n) and every index at a slot of its key's
+// run; with `boxes` the keys are the batch's (`g` unused). n > 0.
+cudaError_t count_grid_enqueue(cudaStream_t stream, const float4 *pos, const GridGeom &g, const BoxKeys *boxes,
+                               const CountGrid &w, const StepRing &r);
+// Then the stable permutation and, with `gather`, the records in its order.
+cudaError_t count_grid_order(cudaStream_t stream, const CountGrid &w, const GridGather *gather);
 
 }  // namespace fcu

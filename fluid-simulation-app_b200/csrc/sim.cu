@@ -104,8 +104,7 @@ struct FluidSim {
     int device = 0;
     cudaStream_t stream = nullptr;
     SimBufs b{};
-    GridWork gw{};
-    void *grid_ws = nullptr;
+    CountGrid gw{};
     DevStep *ring = nullptr, *cur = nullptr;
     DevSolve *solve = nullptr;
     DevStep *h_ring = nullptr;  // pinned mirror of the ring
@@ -139,6 +138,7 @@ struct FluidSim {
         g.nboxes = 1;
         return g;
     }
+    StepRing step_ring() const;
     uint32_t stats_chunks() const {
         const uint32_t c = (n + kStatsThreads - 1) / kStatsThreads;
         return c < 1u ? 1u : (c > (uint32_t)kStatsChunks ? (uint32_t)kStatsChunks : c);
@@ -155,6 +155,8 @@ struct FluidSim {
         return e;
     }
 };
+
+StepRing FluidSim::step_ring() const { return StepRing{ring, cur, solve, kRing, 1}; }
 
 namespace {
 
@@ -292,7 +294,6 @@ GridGeom geom_of(const DevParams &P) {
         g.dims[i] = P.dims[i];
     }
     g.cell = P.cell;
-    g.slabs = kSimSlabs;
     return g;
 }
 
@@ -303,14 +304,13 @@ GridGeom geom_of(const DevParams &P) {
 template <class Mark>
 cudaError_t enqueue_substep(FluidSim *s, cudaStream_t st, uint32_t div_iters, uint32_t den_iters,
                             bool density_only, Mark mark) {
-    cudaError_t e = cudaMemsetAsync(s->solve->acc_div, 0, 2 * kAccSlots * sizeof(unsigned long long), st);
-    if (e != cudaSuccess) return e;
-    e = grid_build_enqueue(st, s->b.pos, s->n, geom_of(s->P), s->b.keys, s->b.starts, s->b.perm, s->gw,
-                           s->ring, s->cur, s->solve, kRing);
+    cudaError_t e = count_grid_enqueue(st, s->b.pos, geom_of(s->P), nullptr, s->gw, s->step_ring());
     if (e != cudaSuccess) return e;
     mark("grid");
     const Geo g = s->geo();
-    launch_gather(st, s->b, s->n);
+    const GridGather records = gather_of(s->b);
+    e = count_grid_order(st, s->gw, &records);
+    if (e != cudaSuccess) return e;
     mark("gather");
     const SimBufs bd = divergence_bufs(s->b), bf = after_forces(s->b);
     launch_density_div(st, g, density_only ? s->b : bd, 0);
@@ -398,10 +398,9 @@ int32_t capture_tolerance(FluidSim *s, cudaGraphExec_t *out) {
     cudaGraph_t bdiv = nullptr, bden = nullptr;
     CK(cudaStreamBeginCaptureToGraph(st, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     int32_t rc = FLUID_OK;
-    cudaError_t e = cudaMemsetAsync(s->solve->acc_div, 0, 2 * kAccSlots * sizeof(unsigned long long), st);
-    if (e == cudaSuccess)
-        e = grid_build_enqueue(st, s->b.pos, s->n, geom_of(s->P), s->b.keys, s->b.starts, s->b.perm, s->gw,
-                               s->ring, s->cur, s->solve, kRing);
+    cudaError_t e = count_grid_enqueue(st, s->b.pos, geom_of(s->P), nullptr, s->gw, s->step_ring());
+    const GridGather records = gather_of(s->b);
+    if (e == cudaSuccess) e = count_grid_order(st, s->gw, &records);
     const Geo geo = s->geo();
     // With at least one divergence apply, forces_eval runs after every one
     // and also forms the divergence prediction that decides whether the
@@ -409,7 +408,6 @@ int32_t capture_tolerance(FluidSim *s, cudaGraphExec_t *out) {
     const bool fused = c.max_iters >= 1;
     const SimBufs bd = divergence_bufs(s->b), bf = after_forces(s->b);
     if (e == cudaSuccess) {
-        launch_gather(st, s->b, s->n);
         launch_density_div(st, geo, bd, 0);
         launch_tol_finish(st, geo, 0, 1, c.div_tol, c.max_iters, hdiv);
         rc = add_while(st, g, hdiv, &bdiv);
@@ -609,7 +607,6 @@ void fluid_sim_destroy(FluidSim *s) {
     if (s->density_graph) cudaGraphExecDestroy(s->density_graph);
     if (s->tol_graph) cudaGraphExecDestroy(s->tol_graph);
     for (void *p : s->allocs) cudaFree(p);
-    if (s->grid_ws) cudaFree(s->grid_ws);
     if (s->h_ring) cudaFreeHost(s->h_ring);
     if (s->h_stats_stale) cudaFreeHost(s->h_stats_stale);
     if (s->stats_ready) cudaEventDestroy(s->stats_ready);
@@ -686,9 +683,10 @@ static int32_t create_into(FluidSim *s, const FluidSimConfig *cfg) {
     CK(s->alloc(&s->ring, kRing));
     CK(s->alloc(&s->cur, 1));
     CK(s->alloc(&s->solve, 1));
-    const size_t wsb = grid_work_bytes(s->n, s->keyspace);
-    CK(cudaMalloc(&s->grid_ws, wsb));
-    s->gw = grid_work_carve(s->grid_ws, s->n, s->keyspace, &s->solve->error);
+    const size_t wsb = count_grid_bytes(s->n, s->keyspace);
+    char *grid_ws = nullptr;
+    CK(s->alloc(&grid_ws, wsb));
+    s->gw = count_grid_carve(grid_ws, s->n, s->keyspace, b.keys, b.starts, b.perm, &s->solve->error);
     CK(cudaMallocHost(&s->h_ring, kRing * sizeof(DevStep)));
     CK(cudaMallocHost(&s->h_stats_stale, 16 * sizeof(float)));
     CK(cudaEventCreateWithFlags(&s->stats_ready, cudaEventDisableTiming));
@@ -705,6 +703,7 @@ static int32_t create_into(FluidSim *s, const FluidSimConfig *cfg) {
     CK(cudaMemcpy(b.id, ids.data(), 4 * n, cudaMemcpyHostToDevice));
     for (float *z : {b.density, b.alpha, b.kd, b.pressure, b.pinc, b.rho_near}) CK(cudaMemset(z, 0, 4 * n));
     CK(cudaMemset(b.nbr_n, 0, 4 * n));
+    CK(cudaMemset(grid_ws, 0, wsb));
     CK(cudaMemset(b.vel_grid, 0, 16 * C));
     CK(cudaMemset(b.vel_flat, 0, 16 * C));
     CK(cudaMemset(b.stats_acc, 0, 8));
@@ -1042,12 +1041,11 @@ uint32_t fluid_sim_grid_slabs(void) { return kSimSlabs; }
 
 uint32_t fluid_sim_kernels_per_substep(const FluidSim *s) {
     if (!s) return 0;
-    const uint32_t passes = (uint32_t)radix_passes(s->keyspace);
-    // keys + one per radix pass + starts scan + gather + density_div
+    // keys + starts scan + place + order with gather + density_div
     //   + div applies (+ div_kappa after the first) + forces
     //   + den pairs + integrate
     const uint32_t d = s->cfg.div_iters, k = s->cfg.den_iters;
-    return 2 + passes + 1 + 1 + (d ? 2 * d - 1 : 0) + 1 + 2 * k + 1;
+    return 5 + (d ? 2 * d - 1 : 0) + 1 + 2 * k + 1;
 }
 
 int32_t fluid_sim_profile_step(FluidSim *s, const FluidStep *step, float *ms, const char **names,
@@ -1168,8 +1166,7 @@ int32_t fluid_grid_build(const float *pos4, uint32_t n, const FluidGrid *grid, u
         g.dims[i] = grid->dims[i];
     }
     g.cell = grid->cell;
-    CK(grid_build_enqueue(st, (const float4 *)pos4, n, g, k, starts, perm, w, nullptr, nullptr, nullptr,
-                          kRing));
+    CK(grid_build_enqueue(st, (const float4 *)pos4, n, g, k, starts, perm, w));
     return FLUID_OK;
 }
 

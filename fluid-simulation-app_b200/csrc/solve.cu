@@ -348,20 +348,6 @@ struct Nbr3 {
 constexpr uint32_t kSlotMask = (1u << 28) - 1u;
 __device__ __forceinline__ uint32_t list_slot(uint32_t code) { return code & kSlotMask; }
 
-// ---- gather into the working set (sim_grid.wgsl:52-63) -------------------
-__global__ void __launch_bounds__(256) k_gather(SimBufs b, uint32_t n) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    uint32_t i = __ldg(&b.perm[k]);
-    if (i >= n) i = k;  // only after a grid build that gave up; keeps reads in bounds
-    b.wpos[k] = __ldg(&b.pos[i]);
-    b.wvel[k] = __ldg(&b.vel[i]);
-    b.wpvel[k] = __ldg(&b.pvel[i]);
-    b.wpp[k] = __ldg(&b.pp[i]);
-    b.wtemp[k] = __ldg(&b.temp[i]);
-    b.wid[k] = __ldg(&b.id[i]);
-}
-
 // Per-box views of a Geo. kB (batch) is a template flag so the one-box
 // kernels keep their constants in parameter space and their sums on the
 // plain warp-aggregated atomics.
@@ -1453,10 +1439,6 @@ __global__ void __launch_bounds__(256) k_advect(DevParams P, SimBufs b, DevStep 
 inline uint32_t blocks_for(uint32_t n, uint32_t t) { return (n + t - 1) / t; }
 
 }  // namespace
-
-void launch_gather(cudaStream_t s, const SimBufs &b, uint32_t n) {
-    if (n) k_gather<<<blocks_for(n, 256), 256, 0, s>>>(b, n);
-}
 
 // One launch of `kern` over g.n particles: the batch instance when the
 // geometry has a box map, the one-box instance otherwise, at the block size

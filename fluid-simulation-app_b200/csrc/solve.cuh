@@ -1,10 +1,9 @@
 // solve.cuh — the DFSPH substep's sweeps, integrate, statistics, tracers.
 #pragma once
 
-#include "common.cuh"
+#include "grid.cuh"
 
 namespace fcu {
-
 
 // Device pointers of the particle state and scratch: one box, or a batch of
 // boxes laid end to end (box b owns slots first[b] .. first[b] + count - 1 in
@@ -20,7 +19,7 @@ struct SimBufs {
     float *wpp, *wtemp;
     uint32_t *wid;
     // scratch
-    uint32_t *keys, *starts, *perm;
+    uint32_t *keys, *starts, *perm;  // perm: slot -> slot of the resting set
     float *density, *alpha, *kd, *pressure, *pinc, *rho_near;
     float4 *accel, *xsph, *wgrad;
     float4 *wpk;  // position and kd of the last prediction: apply's one record per neighbour
@@ -91,7 +90,6 @@ constexpr int kStatsThreads = 256;
 enum Gate : int { kGateNone = 0, kGateDiv = 1, kGateDen = 2 };
 
 // Enqueue helpers: each launches one kernel on `s`.
-void launch_gather(cudaStream_t s, const SimBufs &b, uint32_t n);
 void launch_density_div(cudaStream_t s, const Geo &g, const SimBufs &b, int slot);
 void launch_div_kappa(cudaStream_t s, const Geo &g, const SimBufs &b, int slot, int gate);
 void launch_apply(cudaStream_t s, const Geo &g, const SimBufs &b, bool add_pressure, int gate);
@@ -102,6 +100,10 @@ void launch_forces_eval(cudaStream_t s, const Geo &g, const SimBufs &b);
 // wpk2, residual term into acc_div[slot]) and skipping boxes whose divergence
 // loop has stopped.
 void launch_forces_div(cudaStream_t s, const Geo &g, const SimBufs &b, int slot, int gate);
+// The resting set's records into cell order.
+inline GridGather gather_of(const SimBufs &b) {
+    return GridGather{b.pos, b.vel, b.pvel, b.pp, b.temp, b.id, b.wpos, b.wvel, b.wpvel, b.wpp, b.wtemp, b.wid};
+}
 // The buffers of a sweep after the forces: velocity and temperature from
 // fvel / ftemp.
 inline SimBufs after_forces(SimBufs b) {
