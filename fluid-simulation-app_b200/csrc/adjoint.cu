@@ -39,6 +39,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "arena.cuh"
 #include "grid.cuh"
 
 namespace fcu {
@@ -1383,7 +1384,7 @@ struct AdjImpl : AdjBase {
     float div_tol = 0.01f, den_tol = 0.001f;
     uint32_t max_iters = 100;
     cudaStream_t stream = nullptr;
-    std::vector<void *> allocs;
+    Arena arena;
     // grid
     CountGrid gw{};
     float4 *pos4 = nullptr;
@@ -1392,7 +1393,8 @@ struct AdjImpl : AdjBase {
     V3<T> *x = nullptr, *v = nullptr;
     T *pp = nullptr;
     uint32_t *id = nullptr, *id2 = nullptr;  // particle ids of the state's order
-    std::vector<float> x0;
+    V3<T> *x_init = nullptr;  // the initial state (at rest, ids in order)
+    uint32_t *id_init = nullptr;
     std::vector<V3<T> *> ck_x, ck_v;
     std::vector<T *> ck_pp;
     std::vector<uint32_t *> ck_id;
@@ -1416,48 +1418,37 @@ struct AdjImpl : AdjBase {
     V3<T> *gbar = nullptr;
     double *fbar = nullptr, *cbar = nullptr;
 
-    template <class U>
-    cudaError_t alloc(U **p, size_t cnt) {
-        void *q = nullptr;
-        cudaError_t e = cudaMalloc(&q, (cnt ? cnt : 1) * sizeof(U));
-        if (e == cudaSuccess) {
-            allocs.push_back(q);
-            *p = (U *)q;
-        }
-        return e;
-    }
     ~AdjImpl() override {
         cudaSetDevice(device);
         if (stream) cudaStreamSynchronize(stream);
-        for (void *p : allocs) cudaFree(p);
+        arena.release();
         if (stream) cudaStreamDestroy(stream);
     }
 
-    int32_t alloc_tape(Tape<T> &t, uint32_t ndiv, uint32_t nden, bool with_x) {
+    void want_tape(Tape<T> &t, uint32_t ndiv, uint32_t nden, bool with_x) {
         const size_t N = n;
         if (with_x) {
-            AK(alloc(&t.x, N));
-            AK(alloc(&t.pp, N));
-            AK(alloc(&t.perm, N));
+            arena.want(&t.x, N);
+            arena.want(&t.pp, N);
+            arena.want(&t.perm, N);
         }
-        AK(alloc(&t.nbr, N * kModelCap));
-        AK(alloc(&t.nbr_n, N));
-        AK(alloc(&t.rho, N));
-        AK(alloc(&t.rhon, N));
-        AK(alloc(&t.alpha, N));
-        AK(alloc(&t.wg, N));
-        AK(alloc(&t.blend, N));
-        AK(alloc(&t.accel, N));
-        AK(alloc(&t.kdf, N));
+        arena.want(&t.nbr, N * kModelCap);
+        arena.want(&t.nbr_n, N);
+        arena.want(&t.rho, N);
+        arena.want(&t.rhon, N);
+        arena.want(&t.alpha, N);
+        arena.want(&t.wg, N);
+        arena.want(&t.blend, N);
+        arena.want(&t.accel, N);
+        arena.want(&t.kdf, N);
         t.vdiv.assign(ndiv + 1, nullptr);
         t.vden.assign(nden + 1, nullptr);
         t.kddiv.assign(ndiv, nullptr);
         t.kdden.assign(nden, nullptr);
-        for (auto &p : t.vdiv) AK(alloc(&p, N));
-        for (auto &p : t.vden) AK(alloc(&p, N));
-        for (auto &p : t.kddiv) AK(alloc(&p, N));
-        for (auto &p : t.kdden) AK(alloc(&p, N));
-        return FLUID_OK;
+        for (auto &p : t.vdiv) arena.want(&p, N);
+        for (auto &p : t.vden) arena.want(&p, N);
+        for (auto &p : t.kddiv) arena.want(&p, N);
+        for (auto &p : t.kdden) arena.want(&p, N);
     }
 
     int32_t create(const FluidSimConfig &c, uint32_t frames_, uint32_t spf_, float frame_dt, float vclamp_,
@@ -1471,6 +1462,7 @@ struct AdjImpl : AdjBase {
         den_tol = c.den_tol;
         max_iters = c.max_iters;
         AK(cudaSetDevice(device));
+        std::vector<float> x0;
         host_seed(c, x0);
         const uint64_t n64 = x0.size() / 4;
         if (n64 == 0 || n64 > (1u << 26)) return report_error(FLUID_ERR_ARG, "adjoint: 1..2^26 particles");
@@ -1485,81 +1477,84 @@ struct AdjImpl : AdjBase {
         cells = (uint32_t)(c64 * kAdjSlabs);  // grid keys: cell * slabs + x slab
         AK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         const size_t N = n;
-        AK(alloc(&pos4, N));
-        AK(alloc(&keys, N));
-        AK(alloc(&starts, (size_t)cells + 1));
-        AK(alloc(&perm, N));
-        AK(alloc(&over, 1));
+        arena.want(&pos4, N);
+        arena.want(&keys, N);
+        arena.want(&starts, (size_t)cells + 1);
+        arena.want(&perm, N);
+        arena.want(&over, 1);
         char *grid_ws = nullptr;
         uint32_t *grid_err = nullptr;
-        AK(alloc(&grid_err, 1));
-        AK(alloc(&grid_ws, count_grid_bytes(n, cells)));
-        AK(cudaMemset(grid_ws, 0, count_grid_bytes(n, cells)));
-        AK(cudaMemset(grid_err, 0, 4));
-        gw = count_grid_carve(grid_ws, n, cells, keys, starts, perm, grid_err);
-        AK(alloc(&x, N));
-        AK(alloc(&v, N));
-        AK(alloc(&pp, N));
-        AK(alloc(&id, N));
-        AK(alloc(&id2, N));
+        arena.want(&grid_err, 1);
+        arena.want(&grid_ws, count_grid_bytes(n, cells));
+        arena.want(&x_init, N);
+        arena.want(&id_init, N);
+        arena.want(&x, N);
+        arena.want(&v, N);
+        arena.want(&pp, N);
+        arena.want(&id, N);
+        arena.want(&id2, N);
         const uint32_t nck = (frames + ce - 1) / ce + 1;
         ck_x.assign(nck, nullptr);
         ck_v.assign(nck, nullptr);
         ck_pp.assign(nck, nullptr);
         ck_id.assign(nck, nullptr);
         for (uint32_t k = 0; k < nck; ++k) {
-            AK(alloc(&ck_x[k], N));
-            AK(alloc(&ck_v[k], N));
-            AK(alloc(&ck_pp[k], N));
-            AK(alloc(&ck_id[k], N));
+            arena.want(&ck_x[k], N);
+            arena.want(&ck_v[k], N);
+            arena.want(&ck_pp[k], N);
+            arena.want(&ck_id[k], N);
         }
         // the forward's scratch substep holds the longest schedule any substep may take
-        int32_t rc = alloc_tape(work, kMaxIters + 1, kMaxIters + 1, true);
-        if (rc != FLUID_OK) return rc;
-        rc = alloc_tape(fin, 0, 0, false);
-        if (rc != FLUID_OK) return rc;
-        AK(alloc(&kd, N));
-        AK(alloc(&gsl, N * kModelCap));
-        AK(alloc(&pinc, N));
-        AK(alloc(&pressure, N));
-        AK(alloc(&acc, 8));
-        AK(alloc(&res_acc, 1));
-        AK(alloc(&part, 4 * (size_t)std::max(nblk(n * kLanes, kAdjThreads), nblk(n, 256))));
-        AK(alloc(&xbar, N));
-        AK(alloc(&vbar, N));
-        AK(alloc(&xbar2, N));
-        AK(alloc(&vbar2, N));
-        AK(alloc(&abar, N));
-        AK(alloc(&bbar, N));
-        AK(alloc(&rhobar, N));
-        AK(alloc(&rhonbar, N));
-        AK(alloc(&alphabar, N));
-        AK(alloc(&kdbar, N));
-        AK(alloc(&dbar, N));
-        AK(alloc(&rbt, N));
-        AK(alloc(&sbar, N));
-        AK(alloc(&gbar, N));
-        AK(alloc(&pbar, N));
-        AK(alloc(&ppbar, N));
-        AK(alloc(&ppbar_next, N));
-        AK(alloc(&fbar, (size_t)frames * spf * 3));
-        AK(alloc(&cbar, 1));
+        want_tape(work, kMaxIters + 1, kMaxIters + 1, true);
+        want_tape(fin, 0, 0, false);
+        arena.want(&kd, N);
+        arena.want(&gsl, N * kModelCap);
+        arena.want(&pinc, N);
+        arena.want(&pressure, N);
+        arena.want(&acc, 8);
+        arena.want(&res_acc, 1);
+        arena.want(&part, 4 * (size_t)std::max(nblk(n * kLanes, kAdjThreads), nblk(n, 256)));
+        arena.want(&xbar, N);
+        arena.want(&vbar, N);
+        arena.want(&xbar2, N);
+        arena.want(&vbar2, N);
+        arena.want(&abar, N);
+        arena.want(&bbar, N);
+        arena.want(&rhobar, N);
+        arena.want(&rhonbar, N);
+        arena.want(&alphabar, N);
+        arena.want(&kdbar, N);
+        arena.want(&dbar, N);
+        arena.want(&rbt, N);
+        arena.want(&sbar, N);
+        arena.want(&gbar, N);
+        arena.want(&pbar, N);
+        arena.want(&ppbar, N);
+        arena.want(&ppbar_next, N);
+        arena.want(&fbar, (size_t)frames * spf * 3);
+        arena.want(&cbar, 1);
+        AK(arena.commit());
+        AK(cudaMemset(grid_ws, 0, count_grid_bytes(n, cells)));
+        AK(cudaMemset(grid_err, 0, 4));
+        gw = count_grid_carve(grid_ws, n, cells, keys, starts, perm, grid_err);
+        // the initial state, which every forward starts from
+        std::vector<V3<T>> xs(n);
+        std::vector<uint32_t> ids(n);
+        for (uint32_t i = 0; i < n; ++i) {
+            xs[i] = V3<T>{T(x0[4 * i]), T(x0[4 * i + 1]), T(x0[4 * i + 2])};
+            ids[i] = i;
+        }
+        AK(cudaMemcpy(x_init, xs.data(), sizeof(V3<T>) * n, cudaMemcpyHostToDevice));
+        AK(cudaMemcpy(id_init, ids.data(), 4ull * n, cudaMemcpyHostToDevice));
+        AK(cudaDeviceSynchronize());  // the handle's stream does not wait for the default one
         return FLUID_OK;
     }
 
     int32_t load_initial() {
-        std::vector<V3<T>> xs(n), zs(n);
-        std::vector<uint32_t> ids(n);
-        for (uint32_t i = 0; i < n; ++i) {
-            xs[i] = V3<T>{T(x0[4 * i]), T(x0[4 * i + 1]), T(x0[4 * i + 2])};
-            zs[i] = V3<T>{T(0), T(0), T(0)};
-            ids[i] = i;
-        }
-        AK(cudaMemcpyAsync(id, ids.data(), 4ull * n, cudaMemcpyHostToDevice, stream));
-        AK(cudaMemcpyAsync(x, xs.data(), sizeof(V3<T>) * n, cudaMemcpyHostToDevice, stream));
-        AK(cudaMemcpyAsync(v, zs.data(), sizeof(V3<T>) * n, cudaMemcpyHostToDevice, stream));
+        AK(cudaMemcpyAsync(id, id_init, 4ull * n, cudaMemcpyDeviceToDevice, stream));
+        AK(cudaMemcpyAsync(x, x_init, sizeof(V3<T>) * n, cudaMemcpyDeviceToDevice, stream));
+        AK(cudaMemsetAsync(v, 0, sizeof(V3<T>) * n, stream));
         AK(cudaMemsetAsync(pp, 0, sizeof(T) * n, stream));
-        AK(cudaStreamSynchronize(stream));
         return FLUID_OK;
     }
 
@@ -1752,10 +1747,10 @@ struct AdjImpl : AdjBase {
         const uint32_t len = ce * spf;
         if (seg.size() == len && md <= seg_div_cap && me <= seg_den_cap) return FLUID_OK;
         seg.assign(len, Tape<T>());
-        for (auto &t : seg) {
-            int32_t rc = alloc_tape(t, md, me, true);
-            if (rc != FLUID_OK) return rc;
-        }
+        for (auto &t : seg) want_tape(t, md, me, true);
+        const cudaError_t e = arena.commit();
+        if (e != cudaSuccess) seg.clear();
+        AK(e);
         seg_div_cap = md;
         seg_den_cap = me;
         return FLUID_OK;

@@ -359,11 +359,10 @@ int32_t batch_create_into(FluidBatch *s, const FluidSimConfig *boxes, uint32_t n
     s->gw = count_grid_carve(grid_ws, s->n, s->cells, b.keys, b.starts, b.perm, &s->solve[0].error);
     BK(cudaMallocHost(&s->h_ring, (size_t)kBatchRing * nb * sizeof(DevStep)));
 
-    std::vector<float> zeros4(4 * n, 0.0f), zeros(n, 0.0f);
     BK(cudaMemcpy(b.pos, pos.data(), 16 * n, cudaMemcpyHostToDevice));
-    BK(cudaMemcpy(b.vel, zeros4.data(), 16 * n, cudaMemcpyHostToDevice));
-    BK(cudaMemcpy(b.pvel, zeros4.data(), 16 * n, cudaMemcpyHostToDevice));
-    BK(cudaMemcpy(b.pp, zeros.data(), 4 * n, cudaMemcpyHostToDevice));
+    BK(cudaMemset(b.vel, 0, 16 * n));
+    BK(cudaMemset(b.pvel, 0, 16 * n));
+    BK(cudaMemset(b.pp, 0, 4 * n));
     BK(cudaMemcpy(b.temp, temp.data(), 4 * n, cudaMemcpyHostToDevice));
     BK(cudaMemcpy(b.id, ids.data(), 4 * n, cudaMemcpyHostToDevice));
     for (float *z : {b.density, b.alpha, b.kd, b.pressure, b.pinc, b.rho_near}) BK(cudaMemset(z, 0, 4 * n));

@@ -692,13 +692,13 @@ static int32_t create_into(FluidSim *s, const FluidSimConfig *cfg) {
     CK(cudaEventCreateWithFlags(&s->stats_ready, cudaEventDisableTiming));
 
     // Initial state (render.rs:1484-1555): the seed, at rest, at temperature.
-    std::vector<float> zeros4(4 * n, 0.0f), zeros(n, 0.0f), temp(n, cfg->temperature);
+    std::vector<float> temp(n, cfg->temperature);
     std::vector<uint32_t> ids(n);
     for (size_t i = 0; i < n; ++i) ids[i] = (uint32_t)i;
     CK(cudaMemcpy(b.pos, pos.data(), 16 * n, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(b.vel, zeros4.data(), 16 * n, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(b.pvel, zeros4.data(), 16 * n, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(b.pp, zeros.data(), 4 * n, cudaMemcpyHostToDevice));
+    CK(cudaMemset(b.vel, 0, 16 * n));
+    CK(cudaMemset(b.pvel, 0, 16 * n));
+    CK(cudaMemset(b.pp, 0, 4 * n));
     CK(cudaMemcpy(b.temp, temp.data(), 4 * n, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(b.id, ids.data(), 4 * n, cudaMemcpyHostToDevice));
     for (float *z : {b.density, b.alpha, b.kd, b.pressure, b.pinc, b.rho_near}) CK(cudaMemset(z, 0, 4 * n));
@@ -900,16 +900,15 @@ int32_t fluid_sim_set_state(FluidSim *s, const float *pos4, const float *vel4, c
 
 int32_t fluid_sim_read_particles(FluidSim *s, float *pos4, float *vel4) {
     if (!s) return fail(FLUID_ERR_ARG, "null handle");
+    CK(cudaSetDevice(s->device));
+    // ordered on the device, into buffers that hold nothing between substeps
     const size_t n = s->n;
-    std::vector<float> p(4 * n), v(4 * n);
-    std::vector<uint32_t> id(n);
-    int32_t rc = fluid_sim_get_state(s, p.data(), v.data(), nullptr, nullptr, nullptr, id.data());
-    if (rc != FLUID_OK) return rc;
-    for (size_t k = 0; k < n; ++k) {
-        const uint32_t i = id[k];
-        if (pos4) std::memcpy(pos4 + 4 * (size_t)i, &p[4 * k], 16);
-        if (vel4) std::memcpy(vel4 + 4 * (size_t)i, &v[4 * k], 16);
-    }
+    float4 *pos = s->b.wpk, *vel = s->b.wpk2;
+    launch_by_id(s->stream, s->b, s->n, pos, vel);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(s->stream));
+    if (pos4) CK(cudaMemcpy(pos4, pos, 16 * n, cudaMemcpyDeviceToHost));
+    if (vel4) CK(cudaMemcpy(vel4, vel, 16 * n, cudaMemcpyDeviceToHost));
     return FLUID_OK;
 }
 

@@ -100,6 +100,8 @@ void launch_forces_eval(cudaStream_t s, const Geo &g, const SimBufs &b);
 // wpk2, residual term into acc_div[slot]) and skipping boxes whose divergence
 // loop has stopped.
 void launch_forces_div(cudaStream_t s, const Geo &g, const SimBufs &b, int slot, int gate);
+// The resting positions and velocities ordered by particle id.
+void launch_by_id(cudaStream_t s, const SimBufs &b, uint32_t n, float4 *pos, float4 *vel);
 // The resting set's records into cell order.
 inline GridGather gather_of(const SimBufs &b) {
     return GridGather{b.pos, b.vel, b.pvel, b.pp, b.temp, b.id, b.wpos, b.wvel, b.wpvel, b.wpp, b.wtemp, b.wid};

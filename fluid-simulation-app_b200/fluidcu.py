@@ -337,8 +337,8 @@ class Adjoint:
         check(lib().fluid_adjoint_set_schedule(self.h, _p(d), _p(e)), "adjoint_set_schedule")
 
     def final_state(self):
-        p = np.zeros((self.n, 3), np.float64)
-        v = np.zeros((self.n, 3), np.float64)
+        p = np.empty((self.n, 3), np.float64)
+        v = np.empty((self.n, 3), np.float64)
         check(lib().fluid_adjoint_final_state(self.h, _p(p), _p(v)), "adjoint_final_state")
         return p, v
 
@@ -428,9 +428,9 @@ class Batch:
 
     def state(self, box):
         n = self.counts[box]
-        out = dict(pos=np.zeros((n, 4), np.float32), vel=np.zeros((n, 4), np.float32),
-                   prev_vel=np.zeros((n, 4), np.float32), prev_p=np.zeros(n, np.float32),
-                   temp=np.zeros(n, np.float32), id=np.zeros(n, np.uint32))
+        out = dict(pos=np.empty((n, 4), np.float32), vel=np.empty((n, 4), np.float32),
+                   prev_vel=np.empty((n, 4), np.float32), prev_p=np.empty(n, np.float32),
+                   temp=np.empty(n, np.float32), id=np.empty(n, np.uint32))
         check(lib().fluid_batch_get_state(self.h, box, *[_p(out[k]) for k in
                                                          ("pos", "vel", "prev_vel", "prev_p",
                                                           "temp", "id")]), "batch_get_state")
@@ -512,9 +512,9 @@ class Sim:
 
     def state(self):
         n = self.n
-        out = dict(pos=np.zeros((n, 4), np.float32), vel=np.zeros((n, 4), np.float32),
-                   prev_vel=np.zeros((n, 4), np.float32), prev_p=np.zeros(n, np.float32),
-                   temp=np.zeros(n, np.float32), id=np.zeros(n, np.uint32))
+        out = dict(pos=np.empty((n, 4), np.float32), vel=np.empty((n, 4), np.float32),
+                   prev_vel=np.empty((n, 4), np.float32), prev_p=np.empty(n, np.float32),
+                   temp=np.empty(n, np.float32), id=np.empty(n, np.uint32))
         check(lib().fluid_sim_get_state(self.h, *[_p(out[k]) for k in
                                                   ("pos", "vel", "prev_vel", "prev_p", "temp",
                                                    "id")]), "get_state")
@@ -527,8 +527,8 @@ class Sim:
         return check(lib().fluid_sim_set_state(self.h, *[_p(a) for a in arrs]), "set_state")
 
     def read_particles(self):
-        pos = np.zeros((self.n, 4), np.float32)
-        vel = np.zeros((self.n, 4), np.float32)
+        pos = np.empty((self.n, 4), np.float32)
+        vel = np.empty((self.n, 4), np.float32)
         check(lib().fluid_sim_read_particles(self.h, _p(pos), _p(vel)), "read_particles")
         return pos, vel
 
@@ -551,8 +551,8 @@ class Sim:
 
     def field_read(self):
         h, w = self._field_shape
-        f2 = np.zeros((h, w, 2), np.float32)
-        f4 = np.zeros((h, w, 4), np.float32)
+        f2 = np.empty((h, w, 2), np.float32)
+        f4 = np.empty((h, w, 4), np.float32)
         check(lib().fluid_sim_field_read(self.h, _p(f2), _p(f4)), "field_read")
         return f2, f4
 
@@ -565,7 +565,7 @@ class Sim:
                       accel=((n, 4), np.float32), xsph=((n, 4), np.float32),
                       wall_grad=((n, 4), np.float32), counters=(2, np.uint32))
         shape, dt = shapes[name]
-        out = np.zeros(shape, dt)
+        out = np.empty(shape, dt)
         check(lib().fluid_sim_read_field(self.h, FIELDS[name], _p(out), out.nbytes), name)
         return out
 
