@@ -21,14 +21,19 @@
 //   * the branch of every clamp (speed ceiling, wall clamp, max(., 0)).
 //
 // The backward pass is reverse mode over the substeps. Every sweep has an
-// adjoint kernel, one thread per particle: the particle's own terms are
-// accumulated directly, its neighbours' shares go out by atomic adds. Pair
-// terms use the analytic derivatives of the cubic spline (gradient and
-// Hessian: d(gs x)/dx = gs I + (gs'/r) x x^T); the wall polynomials are
-// differentiated by a three-slot forward-mode dual over the particle's
-// position. The state is checkpointed every `checkpoint_every` frames and
-// each segment is recomputed (storing its substeps' tapes) before it is
-// reversed.
+// adjoint kernel, four lanes per particle: each particle gathers, over its
+// own (symmetric) list, the shares of its neighbours' equations, so nothing
+// is added atomically. Pair terms use the analytic derivatives of the cubic
+// spline (gradient and Hessian: d(gs x)/dx = gs I + (gs'/r) x x^T); the wall
+// polynomials are differentiated by a three-slot forward-mode dual over the
+// particle's position. What depends on positions alone, each pair's gs and
+// gs'/r and the walls' derivatives, is formed once a substep. The state is
+// checkpointed every `checkpoint_every` frames and each segment is recomputed
+// (storing its substeps' tapes) before it is reversed.
+//
+// What bounds the sweeps at 64k particles: the reversed forces' divisions
+// (30 a pair) at five blocks an SM, 150 us of a substep's 640; the others
+// latency and L1, 20-30 us each.
 //
 // The reference has no adjoint; nothing here replaces a reference call.
 #include <algorithm>
@@ -74,11 +79,13 @@ constexpr uint32_t kAdjSlabs = kSimSlabs;
 #endif
 
 // ---- small vector and dual types --------------------------------------------
+// Padded to four values, so that a record is one 16-byte load (two for
+// double) instead of three words.
 template <class T>
-struct V3 {
-    T x, y, z;
+struct alignas(4 * sizeof(T)) V3 {
+    T x, y, z, w;
 };
-template <class T> DEV V3<T> mk(T x, T y, T z) { return V3<T>{x, y, z}; }
+template <class T> DEV V3<T> mk(T x, T y, T z) { return V3<T>{x, y, z, T(0)}; }
 template <class T> DEV V3<T> operator+(V3<T> a, V3<T> b) { return mk(a.x + b.x, a.y + b.y, a.z + b.z); }
 template <class T> DEV V3<T> operator-(V3<T> a, V3<T> b) { return mk(a.x - b.x, a.y - b.y, a.z - b.z); }
 template <class T> DEV V3<T> operator-(V3<T> a) { return mk(-a.x, -a.y, -a.z); }
@@ -404,10 +411,20 @@ template <class T> DEV Radial<T> radial(const MP<T> &p, T r2) {
     }
     return o;
 }
+// What the reverse sweeps need of a pair: gs and gs' / r, both 0 below the
+// guard radius.
+template <class T>
+struct alignas(2 * sizeof(T)) PairG {
+    T gs, h;
+};
+template <class T> DEV PairG<T> pair_g(const Radial<T> &R) {
+    if (R.r < T(1e-9f)) return PairG<T>{T(0), T(0)};
+    return PairG<T>{R.gs, R.dgs / R.r};
+}
 // H u, H = d(gs x)/dx = gs I + (gs'/r) x x^T
-template <class T> DEV V3<T> hess(const Radial<T> &R, V3<T> x, V3<T> u) {
-    if (R.r < T(1e-9f)) return zero3<T>();
-    return R.gs * u + (R.dgs / R.r * dot(x, u)) * x;
+template <class T> DEV V3<T> hess(PairG<T> g, V3<T> x, V3<T> u) {
+    if (g.gs == T(0) && g.h == T(0)) return zero3<T>();
+    return g.gs * u + (g.h * dot(x, u)) * x;
 }
 
 // ---- forward kernels -----------------------------------------------------------
@@ -550,7 +567,8 @@ __global__ void __launch_bounds__(256) k_m_gather(uint32_t n, const uint32_t *__
 // (load(j)), and only then use(gs, record) for each, so a batch's loads
 // overlap.
 constexpr int kMB = 4;
-constexpr int kRB = 2;  // the reverse sweeps with wide records
+constexpr int kPB = 2;  // the reverse sweeps on stored pair values (4: 12.15 ms a backward against 11.96)
+constexpr int kRB = 1;  // the sweeps with wide records (2: 12.15 against 11.69)
 // Each particle's list is shared by kLanes adjacent lanes of a warp: lane l
 // takes entries l, l + kLanes, ... and the lanes' partial sums are folded by
 // lane_sum (the model fixes its own summation order; at 64k particles one
@@ -585,9 +603,9 @@ DEV LaneOf lane_of(uint32_t n) {
 template <class T, class R, class Load, class Use>
 DEV void mwalk(const uint32_t *__restrict__ nbr, const T *__restrict__ gsl, uint32_t n, uint32_t i,
                uint32_t cnt, uint32_t lane, Load load, Use use) {
-    for (uint32_t k = lane; k < cnt; k += kLanes * kMB) {
-        uint32_t j[kMB];
-        T g[kMB];
+    uint32_t j[kMB];
+    T g[kMB];
+    auto entries = [&](uint32_t k) {
 #pragma unroll
         for (int u = 0; u < kMB; ++u) {
             const uint32_t kk = k + u * kLanes;
@@ -595,12 +613,20 @@ DEV void mwalk(const uint32_t *__restrict__ nbr, const T *__restrict__ gsl, uint
             j[u] = ok ? nbr[(size_t)kk * n + i] : i;
             g[u] = ok ? gsl[(size_t)kk * n + i] : T(0);
         }
+    };
+    entries(lane);
+    for (uint32_t k = lane; k < cnt; k += kLanes * kMB) {
         R r[kMB];
+        T gu[kMB];
 #pragma unroll
-        for (int u = 0; u < kMB; ++u) r[u] = load(j[u]);
+        for (int u = 0; u < kMB; ++u) {
+            r[u] = load(j[u]);
+            gu[u] = g[u];
+        }
+        entries(k + kLanes * kMB);  // the next batch's, before this one's records are used
 #pragma unroll
         for (int u = 0; u < kMB; ++u)
-            if (k + u * kLanes < cnt) use(g[u], r[u]);
+            if (k + u * kLanes < cnt) use(gu[u], r[u]);
     }
 }
 template <class T> struct XV {
@@ -611,21 +637,56 @@ template <class T> struct XK {
     T kd;
 };
 
-// mwalk for the reverse sweeps, which keep no gradient scales: kB entries,
-// then their records, then use(j, record) for each, in the lane's order.
+// mwalk without the scales: kB entries, then their records, then use(record)
+// for each, in the lane's order.
 template <int kB, class R, class Load, class Use>
 DEV void rwalk(const uint32_t *__restrict__ nbr, uint32_t n, uint32_t i, uint32_t cnt, uint32_t lane, Load load,
                Use use) {
-    for (uint32_t k = lane; k < cnt; k += kLanes * kB) {
-        uint32_t j[kB];
+    uint32_t j[kB];
+    auto entries = [&](uint32_t k) {
 #pragma unroll
         for (int u = 0; u < kB; ++u) j[u] = k + u * kLanes < cnt ? nbr[(size_t)(k + u * kLanes) * n + i] : i;
+    };
+    entries(lane);
+    for (uint32_t k = lane; k < cnt; k += kLanes * kB) {
         R r[kB];
 #pragma unroll
         for (int u = 0; u < kB; ++u) r[u] = load(j[u]);
+        entries(k + kLanes * kB);
 #pragma unroll
         for (int u = 0; u < kB; ++u)
-            if (k + u * kLanes < cnt) use(j[u], r[u]);
+            if (k + u * kLanes < cnt) use(r[u]);
+    }
+}
+// mwalk for the reverse sweeps, with each pair's gs and gs' / r beside the
+// list (k_r_pairs).
+template <class T, class R, class Load, class Use>
+DEV void pwalk(const uint32_t *__restrict__ nbr, const PairG<T> *__restrict__ pair, uint32_t n, uint32_t i,
+               uint32_t cnt, uint32_t lane, Load load, Use use) {
+    uint32_t j[kPB];
+    PairG<T> g[kPB];
+    auto entries = [&](uint32_t k) {
+#pragma unroll
+        for (int u = 0; u < kPB; ++u) {
+            const uint32_t kk = k + u * kLanes;
+            const bool ok = kk < cnt;
+            j[u] = ok ? nbr[(size_t)kk * n + i] : i;
+            g[u] = ok ? pair[(size_t)kk * n + i] : PairG<T>{T(0), T(0)};
+        }
+    };
+    entries(lane);
+    for (uint32_t k = lane; k < cnt; k += kLanes * kPB) {
+        R r[kPB];
+        PairG<T> gu[kPB];
+#pragma unroll
+        for (int u = 0; u < kPB; ++u) {
+            r[u] = load(j[u]);
+            gu[u] = g[u];
+        }
+        entries(k + kLanes * kPB);
+#pragma unroll
+        for (int u = 0; u < kPB; ++u)
+            if (k + u * kLanes < cnt) use(gu[u], r[u]);
     }
 }
 template <class T> struct XVK {
@@ -646,21 +707,16 @@ DEV T div_of(const MP<T> &p, uint32_t n, uint32_t i, const V3<T> *__restrict__ x
     return p.m * lane_sum(d) + dot(vi, wgi);
 }
 
-// div_of with each pair's gradient scale recomputed (the reverse sweeps,
-// which keep no scales): the same values, so the same sum.
+// div_of in the reverse sweeps, whose scales are in `pair`.
 template <class T>
-DEV T div_of_radial(const MP<T> &p, uint32_t n, uint32_t i, const V3<T> *__restrict__ x,
-                    const V3<T> *__restrict__ v, const uint32_t *__restrict__ nbr, uint32_t cnt, V3<T> wgi,
-                    uint32_t lane) {
+DEV T div_of_pairs(const MP<T> &p, uint32_t n, uint32_t i, const V3<T> *__restrict__ x,
+                   const V3<T> *__restrict__ v, const uint32_t *__restrict__ nbr,
+                   const PairG<T> *__restrict__ pair, uint32_t cnt, V3<T> wgi, uint32_t lane) {
     const V3<T> xi = x[i], vi = v[i];
     T d = T(0);
-    rwalk<kMB, XV<T>>(
-        nbr, n, i, cnt, lane, [&](uint32_t j) { return XV<T>{x[j], v[j]}; },
-        [&](uint32_t, const XV<T> &q) {
-            const V3<T> xij = xi - q.x;
-            const Radial<T> R = radial(p, dot(xij, xij));
-            d += dot(vi - q.v, R.gs * xij);
-        });
+    pwalk<T, XV<T>>(
+        nbr, pair, n, i, cnt, lane, [&](uint32_t j) { return XV<T>{x[j], v[j]}; },
+        [&](PairG<T> g, const XV<T> &q) { d += dot(vi - q.v, g.gs * (xi - q.x)); });
     return p.m * lane_sum(d) + dot(vi, wgi);
 }
 
@@ -751,7 +807,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_m_forces_eval(MP<T> p, uint32_t
         T rho, near;
     };
     rwalk<kRB, Rec>(nbr, n, i, cnt, L.lane, [&](uint32_t j) { return Rec{x[j], v[j], rho[j], rhon[j]}; },
-                    [&](uint32_t, const Rec &q) {
+                    [&](const Rec &q) {
         const V3<T> xij = xi - q.x;
         const T r2 = dot(xij, xij);
         const Radial<T> R = radial(p, r2);
@@ -856,13 +912,20 @@ __global__ void __launch_bounds__(256) k_m_loss(MP<T> p, uint32_t n, const V3<T>
 
 // integrate: x' = clamp(x + v_c dt), v' = v_c zeroed where clamped, v_c the
 // speed-clamped v. In place: xbar, vbar hold the adjoints of x', v' on entry
-// and of x, v on exit.
+// and of x, v on exit. The pressure's adjoint is the next substep's previous
+// pressure's; the adjoints the substep accumulates start at 0.
 template <class T>
 __global__ void __launch_bounds__(256) k_r_integrate(MP<T> p, uint32_t n, T dt, T vclamp,
                                                      const V3<T> *__restrict__ x, const V3<T> *__restrict__ v_pre,
-                                                     const T *__restrict__ rho, V3<T> *xbar, V3<T> *vbar) {
+                                                     const T *__restrict__ rho, V3<T> *xbar, V3<T> *vbar,
+                                                     const T *__restrict__ ppbar, T *pbar, T *rhobar, T *rhonbar,
+                                                     T *alphabar) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    pbar[i] = ppbar[i];
+    rhobar[i] = T(0);
+    rhonbar[i] = T(0);
+    alphabar[i] = T(0);
     V3<T> v = v_pre[i];
     const T speed = sqrt(dot(v, v));
     const T ceiling = rho[i] < p.rho0_half ? T(3) * vclamp : vclamp;
@@ -900,15 +963,74 @@ __global__ void __launch_bounds__(256) k_r_integrate(MP<T> p, uint32_t n, T dt, 
 // Every reverse sweep below writes only its own particle's entries, with no
 // atomics; the pair terms are evaluated once from each end.
 
+// Each pair's gs and gs' / r beside the list, once a substep: the sweeps of
+// the divergence and density iterations, of the forces' push and of the
+// density would each redo the square root and three divisions.
+template <class T>
+__global__ void __launch_bounds__(kAdjThreads) k_r_pairs(MP<T> p, uint32_t n, const V3<T> *__restrict__ x,
+                                                         const uint32_t *__restrict__ nbr,
+                                                         const uint32_t *__restrict__ nbr_n, PairG<T> *pair) {
+    const LaneOf L = lane_of(n);
+    const uint32_t i = L.i;
+    const V3<T> xi = x[i];
+    const uint32_t cnt = L.live ? nbr_n[i] : 0u;
+    for (uint32_t k = L.lane; k < cnt; k += kLanes * kMB) {
+        V3<T> xj[kMB];
+#pragma unroll
+        for (int u = 0; u < kMB; ++u) {
+            const uint32_t kk = k + u * kLanes;
+            xj[u] = x[kk < cnt ? nbr[(size_t)kk * n + i] : i];
+        }
+#pragma unroll
+        for (int u = 0; u < kMB; ++u) {
+            const uint32_t kk = k + u * kLanes;
+            const V3<T> xij = xi - xj[u];
+            if (kk < cnt) pair[(size_t)kk * n + i] = pair_g(radial(p, dot(xij, xij)));
+        }
+    }
+}
+
+// The walls' derivatives at every particle, once a substep: the rows of the
+// Jacobians of the wall gradient and of the adhesion, and the fill's gradient.
+// They depend on positions alone; every sweep evaluated its own (24 edge
+// polynomials over duals near a wall) on one lane of a particle's four.
+template <class T>
+struct WallDerivs {
+    V3<T> *grad[3], *adh[3], *fill;
+};
+template <class T> DEV J3<T> rows_of(V3<T> *const (&r)[3], uint32_t i) {
+    const V3<T> a = r[0][i], b = r[1][i], c = r[2][i];
+    J3<T> J;
+    J.a[0][0] = a.x; J.a[0][1] = a.y; J.a[0][2] = a.z;
+    J.a[1][0] = b.x; J.a[1][1] = b.y; J.a[1][2] = b.z;
+    J.a[2][0] = c.x; J.a[2][1] = c.y; J.a[2][2] = c.z;
+    return J;
+}
+template <class T>
+__global__ void __launch_bounds__(kAdjThreads) k_r_walls(MP<T> p, uint32_t n, const V3<T> *__restrict__ x,
+                                                         WallDerivs<T> o) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const V3<T> xi = x[i];
+    const J3<T> G = wall_grad_jac(p, xi);
+    const J3<T> A = wall_adh_jac(p, xi);
+    for (int r = 0; r < 3; ++r) {
+        o.grad[r][i] = mk(G.a[r][0], G.a[r][1], G.a[r][2]);
+        o.adh[r][i] = mk(A.a[r][0], A.a[r][1], A.a[r][2]);
+    }
+    o.fill[i] = fill_grad(p, xi);
+}
+
 // apply (v_out = v_in - dt (m sum (kd_i + kd_j) grad W_ij + kd_i wg_i)):
 // given vbar (the adjoint of v_out, and of v_in), write the adjoint of kd and
 // add the adjoint of x.
 template <class T>
 __global__ void __launch_bounds__(kAdjThreads) k_r_apply(MP<T> p, uint32_t n, T dt, const V3<T> *__restrict__ x,
                                                          const uint32_t *__restrict__ nbr,
+                                                         const PairG<T> *__restrict__ pair,
                                                          const uint32_t *__restrict__ nbr_n, const T *__restrict__ kd,
                                                          const V3<T> *__restrict__ wg, const V3<T> *__restrict__ vbar,
-                                                         T *kdbar, V3<T> *xbar) {
+                                                         WallDerivs<T> wd, T *kdbar, V3<T> *xbar) {
     const LaneOf L = lane_of(n);
     const uint32_t i = L.i;
     const V3<T> xi = x[i], vb = vbar[i];
@@ -917,21 +1039,20 @@ __global__ void __launch_bounds__(kAdjThreads) k_r_apply(MP<T> p, uint32_t n, T 
     const uint32_t cnt = L.live ? nbr_n[i] : 0u;
     T s = T(0);
     V3<T> xs = zero3<T>();
-    rwalk<kMB, XVK<T>>(
-        nbr, n, i, cnt, L.lane, [&](uint32_t j) { return XVK<T>{x[j], vbar[j], kd[j]}; },
-        [&](uint32_t, const XVK<T> &q) {
+    pwalk<T, XVK<T>>(
+        nbr, pair, n, i, cnt, L.lane, [&](uint32_t j) { return XVK<T>{x[j], vbar[j], kd[j]}; },
+        [&](PairG<T> g, const XVK<T> &q) {
             const V3<T> xij = xi - q.x;
-            const Radial<T> R = radial(p, dot(xij, xij));
             const V3<T> dvb = vb - q.v;
-            s += dot(R.gs * xij, dvb);
-            xs = xs + (c * (kdi + q.k)) * hess(R, xij, dvb);
+            s += dot(g.gs * xij, dvb);
+            xs = xs + (c * (kdi + q.k)) * hess(g, xij, dvb);
         });
     s = lane_sum(s);
     xs = lane_sum(xs);
     if (!L.live || L.lane != 0) return;
     const V3<T> wgi = wg[i];
     kdbar[i] = -dt * (p.m * s + dot(wgi, vb));
-    const J3<T> J = wall_grad_jac(p, xi);
+    const J3<T> J = rows_of(wd.grad, i);
     xbar[i] = xbar[i] + xs + (-dt * kdi) * jt_mul(J, vb);
 }
 
@@ -943,6 +1064,7 @@ template <class T>
 __global__ void __launch_bounds__(kAdjThreads) k_r_kappa_a(MP<T> p, uint32_t n, int den, T dt,
                                                            const V3<T> *__restrict__ x, const V3<T> *__restrict__ v,
                                                            const uint32_t *__restrict__ nbr,
+                                                           const PairG<T> *__restrict__ pair,
                                                            const uint32_t *__restrict__ nbr_n,
                                                            const T *__restrict__ rho, const T *__restrict__ alpha,
                                                            const V3<T> *__restrict__ wg, const T *__restrict__ kdbar,
@@ -950,7 +1072,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_r_kappa_a(MP<T> p, uint32_t n, 
                                                            T *alphabar) {
     const LaneOf L = lane_of(n);
     const uint32_t i = L.i;
-    const T d = div_of_radial(p, n, i, x, v, nbr, L.live ? nbr_n[i] : 0u, wg[i], L.lane);
+    const T d = div_of_pairs(p, n, i, x, v, nbr, pair, L.live ? nbr_n[i] : 0u, wg[i], L.lane);
     if (!L.live || L.lane != 0) return;
     const T r = rho[i], a = alpha[i], kb = kdbar[i];
     T db = T(0), rb = T(0), ab = T(0);
@@ -985,31 +1107,31 @@ template <class T>
 __global__ void __launch_bounds__(kAdjThreads) k_r_kappa_b(MP<T> p, uint32_t n, const V3<T> *__restrict__ x,
                                                            const V3<T> *__restrict__ v,
                                                            const uint32_t *__restrict__ nbr,
+                                                           const PairG<T> *__restrict__ pair,
                                                            const uint32_t *__restrict__ nbr_n,
                                                            const V3<T> *__restrict__ wg, const T *__restrict__ dbar,
-                                                           V3<T> *vbar, V3<T> *xbar) {
+                                                           WallDerivs<T> wd, V3<T> *vbar, V3<T> *xbar) {
     const LaneOf L = lane_of(n);
     const uint32_t i = L.i;
     const V3<T> xi = x[i], vi = v[i];
     const T di = dbar[i];
     const uint32_t cnt = L.live ? nbr_n[i] : 0u;
     V3<T> vs = zero3<T>(), xs = zero3<T>();
-    rwalk<kMB, XVK<T>>(
-        nbr, n, i, cnt, L.lane, [&](uint32_t j) { return XVK<T>{x[j], v[j], dbar[j]}; },
-        [&](uint32_t, const XVK<T> &q) {
+    pwalk<T, XVK<T>>(
+        nbr, pair, n, i, cnt, L.lane, [&](uint32_t j) { return XVK<T>{x[j], v[j], dbar[j]}; },
+        [&](PairG<T> g, const XVK<T> &q) {
             const T c = p.m * (di + q.k);
             if (c == T(0)) return;
             const V3<T> xij = xi - q.x;
-            const Radial<T> R = radial(p, dot(xij, xij));
-            vs = vs + (c * R.gs) * xij;
-            xs = xs + c * hess(R, xij, vi - q.v);
+            vs = vs + (c * g.gs) * xij;
+            xs = xs + c * hess(g, xij, vi - q.v);
         });
     vs = lane_sum(vs);
     xs = lane_sum(xs);
     if (!L.live || L.lane != 0) return;
     vbar[i] = vbar[i] + vs + di * wg[i];
     if (di != T(0)) {
-        const J3<T> J = wall_grad_jac(p, xi);
+        const J3<T> J = rows_of(wd.grad, i);
         xs = xs + di * jt_mul(J, vi);
     }
     xbar[i] = xbar[i] + xs;
@@ -1023,9 +1145,11 @@ __global__ void __launch_bounds__(kAdjThreads) k_r_forces_apply(MP<T> p, uint32_
                                                                 const V3<T> *__restrict__ x,
                                                                 const V3<T> *__restrict__ blend,
                                                                 const uint32_t *__restrict__ nbr,
+                                                                const PairG<T> *__restrict__ pair,
                                                                 const uint32_t *__restrict__ nbr_n,
                                                                 const T *__restrict__ kd, const V3<T> *__restrict__ wg,
-                                                                const V3<T> *__restrict__ vbar, V3<T> *abar, V3<T> *bbar,
+                                                                const V3<T> *__restrict__ vbar, WallDerivs<T> wd,
+                                                                V3<T> *abar, V3<T> *bbar,
                                                                 T *kdbar, V3<T> *xbar, double *part) {
     const LaneOf L = lane_of(n);
     const uint32_t i = L.i;
@@ -1036,14 +1160,13 @@ __global__ void __launch_bounds__(kAdjThreads) k_r_forces_apply(MP<T> p, uint32_
     const uint32_t cnt = L.live ? nbr_n[i] : 0u;
     T s = T(0);
     V3<T> xs = zero3<T>();
-    rwalk<kMB, XVK<T>>(
-        nbr, n, i, cnt, L.lane, [&](uint32_t j) { return XVK<T>{x[j], vbar[j], kd[j]}; },
-        [&](uint32_t, const XVK<T> &q) {
+    pwalk<T, XVK<T>>(
+        nbr, pair, n, i, cnt, L.lane, [&](uint32_t j) { return XVK<T>{x[j], vbar[j], kd[j]}; },
+        [&](PairG<T> g, const XVK<T> &q) {
             const V3<T> xij = xi - q.x;
-            const Radial<T> R = radial(p, dot(xij, xij));
             const V3<T> dvb = vb - q.v;
-            s += dot(R.gs * xij, dvb);
-            xs = xs + (cc * (kdi + q.k)) * hess(R, xij, dvb);
+            s += dot(g.gs * xij, dvb);
+            xs = xs + (cc * (kdi + q.k)) * hess(g, xij, dvb);
         });
     s = lane_sum(s);
     xs = lane_sum(xs);
@@ -1056,97 +1179,127 @@ __global__ void __launch_bounds__(kAdjThreads) k_r_forces_apply(MP<T> p, uint32_
         red[3] = (double)dot(blend[i], vb);
         const V3<T> wgi = wg[i];
         kdbar[i] = -dt * (p.m * s + dot(wgi, vb));
-        const J3<T> J = wall_grad_jac(p, xi);
+        const J3<T> J = rows_of(wd.grad, i);
         xbar[i] = xbar[i] + xs + (-dt * kdi) * jt_mul(J, vb);
     }
     block_sums4(red, part);
 }
 
+// What both ends of a pair share of forces_eval reversed: the radial factors
+// and their derivatives, symmetric in the two particles. (Formed apart for
+// each end, under its own branches, they cost 46 divisions a pair; together
+// 30.)
+template <class T>
+struct ForcePair {
+    bool far;                   // r >= 1e-9: the radial derivatives exist
+    T r, W, dW;
+    T rr, Q, s, dphi;           // rho_a rho_b; visc_k m / rr; viscosity's factor and phi'
+    T psi, sn_psi, sn_dpsi_r;   // near pressure: psi, (near_a + near_b) psi and (..) psi' / r
+    T cmc, cmd_r, m_chi, sr;    // tension: corr m chi, corr m chi' / r, -m chi, rho_a + rho_b
+};
+template <class T>
+DEV ForcePair<T> force_pair_of(const MP<T> &p, T r2, const Radial<T> &R, T rho_a, T rho_b, T near_a, T near_b) {
+    ForcePair<T> f;
+    const T r = R.r;
+    f.r = r;
+    f.W = R.W;
+    f.dW = R.dW;
+    f.far = r >= T(1e-9f);
+    f.dphi = f.sn_dpsi_r = f.cmd_r = T(0);
+    // viscosity: visc_k m / (rho_a rho_b) phi(r) dv, phi = gs r^2 / (r^2 + eps)
+    const T den = r2 + p.eps;
+    f.rr = rho_a * rho_b;
+    f.Q = p.visc_k * p.m / f.rr;
+    f.s = f.Q * (R.gs * r2 / den);
+    // near pressure: (near_a + near_b) psi(r) x, psi = wn^2 / max(r, 1e-5)
+    const T wn = R.q < T(1) ? T(1) - R.q : T(0);
+    const T rn = r > T(1e-5f) ? r : T(1e-5f);
+    f.psi = wn * wn / rn;
+    const T sn = near_a + near_b;
+    f.sn_psi = sn * f.psi;
+    // surface tension: -corr m chi(r) x, chi = C(r) / max(r, 1e-9)
+    T C = T(0), dC = T(0);
+    if (r < p.coh_c && f.far) {
+        const T cr = p.coh_c - r;
+        const T a = cr * cr * cr * r * r * r;
+        const T da = T(-3) * cr * cr * r * r * r + T(3) * cr * cr * cr * r * r;
+        if (T(2) * r > p.coh_c) {
+            C = p.coh_k * a;
+            dC = p.coh_k * da;
+        } else {
+            C = p.coh_k * (T(2) * a - p.coh_near);
+            dC = p.coh_k * T(2) * da;
+        }
+    }
+    const T rt = r > T(1e-9f) ? r : T(1e-9f);
+    const T chi = C / rt;
+    f.sr = rho_a + rho_b;
+    const T corr = T(2) * p.rho0 / f.sr;
+    f.cmc = corr * p.m * chi;
+    f.m_chi = -p.m * chi;
+    if (f.far) {
+        // dphi/dr = (gs' r^2 + 2 gs r) / den - gs r^2 2 r / den^2
+        f.dphi = (R.dgs * r2 + T(2) * R.gs * r) / den - R.gs * r2 * T(2) * r / (den * den);
+        T dpsi = T(0);
+        if (wn > T(0)) {
+            dpsi = T(2) * wn * (-p.inv_h) / rn;
+            if (r > T(1e-5f)) dpsi -= wn * wn / (r * r);
+        }
+        f.sn_dpsi_r = sn * dpsi / r;
+        const T dchi = r > T(1e-9f) ? dC / r - C / (r * r) : T(0);
+        f.cmd_r = corr * p.m * dchi / r;
+    }
+    return f;
+}
+
 // One pair's share of forces_eval in particle a's equation (neighbour b,
 // x_ab = x_a - x_b, dv = v_a - v_b), reversed: given a's accel and blend
-// adjoints, the adjoints of x_ab, dv, rho_a, rho_b and of (near_a + near_b).
+// adjoints and m / rho_b, the adjoints of x_ab, dv, rho_a, rho_b and of
+// (near_a + near_b).
 template <class T>
 struct PairBar {
     V3<T> gx, gdv;
     T rb_a, rb_b, nb;
 };
 template <class T>
-DEV PairBar<T> forces_pair_bar(const MP<T> &p, V3<T> xab, T r2, const Radial<T> &R, V3<T> dv, T rho_a, T rho_b,
-                               T near_a, T near_b, V3<T> ab, V3<T> bb) {
+DEV PairBar<T> forces_pair_bar(const MP<T> &p, const ForcePair<T> &f, V3<T> xab, V3<T> dv, T rho_a, T rho_b,
+                               T m_rho_b, V3<T> ab, V3<T> bb) {
     PairBar<T> o;
-    o.gx = zero3<T>();
-    o.gdv = zero3<T>();
-    o.rb_a = T(0);
-    o.rb_b = T(0);
-    const T r = R.r;
     const V3<T> ab_near = p.k_near * ab, ab_ten = p.gamma * ab;
-    // viscosity: visc_k m / (rho_a rho_b) phi(r) dv, phi = gs r^2 / (r^2 + eps)
-    {
-        const T den = r2 + p.eps;
-        const T phi = R.gs * r2 / den;
-        const T s = p.visc_k * p.m / (rho_a * rho_b) * phi;
-        o.gdv = o.gdv + s * ab;
-        const T sb = dot(ab, dv);
-        o.rb_a += -sb * s / rho_a;
-        o.rb_b += -sb * s / rho_b;
-        if (r >= T(1e-9f)) {
-            // dphi/dr = (gs' r^2 + 2 gs r) / den - gs r^2 2 r / den^2
-            const T dphi = (R.dgs * r2 + T(2) * R.gs * r) / den - R.gs * r2 * T(2) * r / (den * den);
-            const T phib = sb * p.visc_k * p.m / (rho_a * rho_b);
-            o.gx = o.gx + (phib * dphi / r) * xab;
-        }
+    // viscosity
+    o.gdv = f.s * ab;
+    const T sb = dot(ab, dv);
+    o.rb_a = -sb * f.s / rho_a;
+    o.rb_b = -sb * f.s / rho_b;
+    o.gx = zero3<T>();
+    if (f.far) {
+        const T phib = sb * p.visc_k * p.m / f.rr;
+        o.gx = (phib * f.dphi / f.r) * xab;
     }
-    // near pressure: (near_a + near_b) psi(r) x, psi = wn^2 / max(r, 1e-5)
+    // near pressure
     {
-        const T wn = R.q < T(1) ? T(1) - R.q : T(0);
-        const T rr = r > T(1e-5f) ? r : T(1e-5f);
-        const T psi = wn * wn / rr;
-        const T sn = near_a + near_b;
         const T xa = dot(xab, ab_near);
-        o.nb = psi * xa;
-        T dpsi = T(0);
-        if (wn > T(0)) {
-            dpsi = T(2) * wn * (-p.inv_h) / rr;
-            if (r > T(1e-5f)) dpsi -= wn * wn / (r * r);
-        }
-        o.gx = o.gx + (sn * psi) * ab_near;
-        if (r >= T(1e-9f)) o.gx = o.gx + (sn * dpsi / r * xa) * xab;
+        o.nb = f.psi * xa;
+        o.gx = o.gx + f.sn_psi * ab_near;
+        if (f.far) o.gx = o.gx + (f.sn_dpsi_r * xa) * xab;
     }
     // XSPH blend: -(m / rho_b) W dv
     {
-        const T s = p.m / rho_b * R.W;
+        const T s = m_rho_b * f.W;
         o.gdv = o.gdv - s * bb;
         const T bdv = dot(bb, dv);
         o.rb_b += s / rho_b * bdv;
-        if (r >= T(1e-9f)) o.gx = o.gx + (-(p.m / rho_b) * bdv * R.dW / r) * xab;
+        if (f.far) o.gx = o.gx + (-m_rho_b * bdv * f.dW / f.r) * xab;
     }
-    // surface tension: -corr m chi(r) x, chi = C(r) / max(r, 1e-9)
+    // surface tension
     {
-        T C = T(0), dC = T(0);
-        if (r < p.coh_c && r >= T(1e-9f)) {
-            const T cr = p.coh_c - r;
-            const T a = cr * cr * cr * r * r * r;
-            const T da = T(-3) * cr * cr * r * r * r + T(3) * cr * cr * cr * r * r;
-            if (T(2) * r > p.coh_c) {
-                C = p.coh_k * a;
-                dC = p.coh_k * da;
-            } else {
-                C = p.coh_k * (T(2) * a - p.coh_near);
-                dC = p.coh_k * T(2) * da;
-            }
-        }
-        const T rt = r > T(1e-9f) ? r : T(1e-9f);
-        const T chi = C / rt;
-        const T dchi = r > T(1e-9f) ? dC / r - C / (r * r) : T(0);
-        const T sr = rho_a + rho_b;
-        const T corr = T(2) * p.rho0 / sr;
         const T xa = dot(xab, ab_ten);
-        const T corrb = -p.m * chi * xa;
-        const T srb = -corrb * T(2) * p.rho0 / (sr * sr);
+        const T corrb = f.m_chi * xa;
+        const T srb = -corrb * T(2) * p.rho0 / (f.sr * f.sr);
         o.rb_a += srb;
         o.rb_b += srb;
-        o.gx = o.gx - (corr * p.m * chi) * ab_ten;
-        if (r >= T(1e-9f)) o.gx = o.gx - (corr * p.m * dchi / r * xa) * xab;
+        o.gx = o.gx - f.cmc * ab_ten;
+        if (f.far) o.gx = o.gx - (f.cmd_r * xa) * xab;
     }
     return o;
 }
@@ -1156,8 +1309,11 @@ DEV PairBar<T> forces_pair_bar(const MP<T> &p, V3<T> xab, T r2, const Radial<T> 
 // adjoints of x, v, rho and near density, and write that of the previous
 // pressure. Each pair is reversed in the particle's own equation and in the
 // neighbour's.
+// In 32 bits held to 5 blocks per SM (102 registers instead of 145: 12.15
+// against 11.63 ms a backward of the 64k-particle workload; in 64 bits the
+// spills cost more).
 template <class T>
-__global__ void __launch_bounds__(kAdjThreads) k_r_forces_eval(MP<T> p, uint32_t n, const V3<T> *__restrict__ x,
+__global__ void __launch_bounds__(kAdjThreads, sizeof(T) == 4 ? 5 : 1) k_r_forces_eval(MP<T> p, uint32_t n, const V3<T> *__restrict__ x,
                                                                const V3<T> *__restrict__ v,
                                                                const uint32_t *__restrict__ nbr,
                                                                const uint32_t *__restrict__ nbr_n,
@@ -1165,13 +1321,15 @@ __global__ void __launch_bounds__(kAdjThreads) k_r_forces_eval(MP<T> p, uint32_t
                                                                const T *__restrict__ pp, const V3<T> *__restrict__ abar,
                                                                const V3<T> *__restrict__ bbar,
                                                                const T *__restrict__ kdbar, const T *__restrict__ pbar,
-                                                               V3<T> *xbar, V3<T> *vbar, T *rhobar, T *rhonbar,
+                                                               WallDerivs<T> wd, V3<T> *xbar, V3<T> *vbar, T *rhobar,
+                                                               T *rhonbar,
                                                                T *ppbar) {
     const LaneOf L = lane_of(n);
     const uint32_t i = L.i;
     const V3<T> xi = x[i], vi = v[i];
     const T rho_i = rho[i], near_i = rhon[i];
     const V3<T> ab = abar[i], bb = bbar[i];
+    const T m_rho_i = p.m / rho_i;
     T rb_i = T(0);
     T nb_i = T(0);
     V3<T> xs = zero3<T>(), vs = zero3<T>();
@@ -1182,13 +1340,14 @@ __global__ void __launch_bounds__(kAdjThreads) k_r_forces_eval(MP<T> p, uint32_t
     };
     rwalk<kRB, Rec>(
         nbr, n, i, cnt, L.lane, [&](uint32_t j) { return Rec{x[j], v[j], abar[j], bbar[j], rho[j], rhon[j]}; },
-        [&](uint32_t, const Rec &q) {
+        [&](const Rec &q) {
             const V3<T> xij = xi - q.x;
             const T r2 = dot(xij, xij);
             const Radial<T> R = radial(p, r2);
             const V3<T> dv = vi - q.v;
-            const PairBar<T> own = forces_pair_bar(p, xij, r2, R, dv, rho_i, q.rho, near_i, q.near, ab, bb);
-            const PairBar<T> oth = forces_pair_bar(p, -xij, r2, R, -dv, q.rho, rho_i, q.near, near_i, q.ab, q.bb);
+            const ForcePair<T> f = force_pair_of(p, r2, R, rho_i, q.rho, near_i, q.near);
+            const PairBar<T> own = forces_pair_bar(p, f, xij, dv, rho_i, q.rho, p.m / q.rho, ab, bb);
+            const PairBar<T> oth = forces_pair_bar(p, f, -xij, -dv, q.rho, rho_i, m_rho_i, q.ab, q.bb);
             xs = xs + own.gx - oth.gx;
             vs = vs + own.gdv - oth.gdv;
             rb_i += own.rb_a + oth.rb_b;
@@ -1203,7 +1362,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_r_forces_eval(MP<T> p, uint32_t
     const T kb = kdbar[i];
     ppbar[i] = T(0.5f) * kb / (rho_i * rho_i) + T(0.5f) * pbar[i];
     rb_i += -kb * pp[i] / (rho_i * rho_i * rho_i);
-    const J3<T> Ja = wall_adh_jac(p, xi);
+    const J3<T> Ja = rows_of(wd.adh, i);
     xs = xs + (p.beta * p.rho0) * jt_mul(Ja, ab);
     xbar[i] = xbar[i] + xs;
     vbar[i] = vbar[i] + vs;
@@ -1217,6 +1376,8 @@ __global__ void __launch_bounds__(kAdjThreads) k_r_forces_eval(MP<T> p, uint32_t
 template <class T>
 __global__ void __launch_bounds__(kAdjThreads) k_r_density_a(MP<T> p, uint32_t n, const V3<T> *__restrict__ x,
                                                              const uint32_t *__restrict__ nbr,
+                                                             const PairG<T> *__restrict__ pair,
+                                                             const V3<T> *__restrict__ wg,
                                                              const uint32_t *__restrict__ nbr_n,
                                                              const T *__restrict__ rho, const T *__restrict__ rhobar,
                                                              const T *__restrict__ alphabar, T *rbt, V3<T> *gbar,
@@ -1227,19 +1388,17 @@ __global__ void __launch_bounds__(kAdjThreads) k_r_density_a(MP<T> p, uint32_t n
     const uint32_t cnt = L.live ? nbr_n[i] : 0u;
     V3<T> gsum = zero3<T>();
     T gsq = T(0);
-    rwalk<kMB, V3<T>>(
-        nbr, n, i, cnt, L.lane, [&](uint32_t j) { return x[j]; },
-        [&](uint32_t, const V3<T> &xj) {
-            const V3<T> xij = xi - xj;
-            const Radial<T> R = radial(p, dot(xij, xij));
-            const V3<T> gw = R.gs * xij;
+    pwalk<T, V3<T>>(
+        nbr, pair, n, i, cnt, L.lane, [&](uint32_t j) { return x[j]; },
+        [&](PairG<T> g, const V3<T> &xj) {
+            const V3<T> gw = g.gs * (xi - xj);
             gsum = gsum + gw;
             gsq += dot(gw, gw);
         });
     gsum = lane_sum(gsum);
     gsq = lane_sum(gsq);
     if (!L.live || L.lane != 0) return;
-    const V3<T> G = p.m * gsum + wall_grad(p, xi);
+    const V3<T> G = p.m * gsum + wg[i];  // the forward's wall gradient at x
     const T den = dot(G, G) + p.m * p.m * gsq;
     const T r = rho[i];
     const T ab = alphabar[i];
@@ -1263,11 +1422,11 @@ __global__ void __launch_bounds__(kAdjThreads) k_r_density_a(MP<T> p, uint32_t n
 // weighted by its adjoints: rho (rb m grad W), G (m H Gb), S (2 Sb m^2 H
 // grad W) and near density (nb 3 wn^2 d wn / d x).
 template <class T>
-DEV V3<T> density_pair_bar(const MP<T> &p, V3<T> xab, const Radial<T> &R, T rb, V3<T> Gb, T Sb, T nb) {
+DEV V3<T> density_pair_bar(const MP<T> &p, V3<T> xab, const Radial<T> &R, PairG<T> pg, T rb, V3<T> Gb, T Sb, T nb) {
     const V3<T> gw = R.gs * xab;
     V3<T> g = (rb * p.m) * gw;
-    g = g + p.m * hess(R, xab, Gb);
-    g = g + (Sb * p.m * p.m * T(2)) * hess(R, xab, gw);
+    g = g + p.m * hess(pg, xab, Gb);
+    g = g + (Sb * p.m * p.m * T(2)) * hess(pg, xab, gw);
     if (R.q < T(1) && R.r >= T(1e-9f)) {
         const T wn = T(1) - R.q;
         g = g + (nb * T(3) * wn * wn * (-p.inv_h) / R.r) * xab;
@@ -1283,7 +1442,8 @@ __global__ void __launch_bounds__(kAdjThreads) k_r_density_b(MP<T> p, uint32_t n
                                                              const uint32_t *__restrict__ nbr_n,
                                                              const T *__restrict__ rbt, const V3<T> *__restrict__ gbar,
                                                              const T *__restrict__ sbar,
-                                                             const T *__restrict__ rhonbar, V3<T> *xbar) {
+                                                             const T *__restrict__ rhonbar, WallDerivs<T> wd,
+                                                             V3<T> *xbar) {
     const LaneOf L = lane_of(n);
     const uint32_t i = L.i;
     const V3<T> xi = x[i];
@@ -1297,15 +1457,17 @@ __global__ void __launch_bounds__(kAdjThreads) k_r_density_b(MP<T> p, uint32_t n
     };
     rwalk<kRB, Rec>(
         nbr, n, i, cnt, L.lane, [&](uint32_t j) { return Rec{x[j], gbar[j], rbt[j], sbar[j], rhonbar[j]}; },
-        [&](uint32_t, const Rec &q) {
+        [&](const Rec &q) {
             const V3<T> xij = xi - q.x;
             const Radial<T> R = radial(p, dot(xij, xij));
-            xs = xs + density_pair_bar(p, xij, R, rb, Gb, Sb, nb) - density_pair_bar(p, -xij, R, q.rb, q.gb, q.sb, q.nb);
+            const PairG<T> pg = pair_g(R);
+            xs = xs + density_pair_bar(p, xij, R, pg, rb, Gb, Sb, nb) -
+                 density_pair_bar(p, -xij, R, pg, q.rb, q.gb, q.sb, q.nb);
         });
     xs = lane_sum(xs);
     if (!L.live || L.lane != 0) return;
-    const J3<T> J = wall_grad_jac(p, xi);
-    xs = xs + jt_mul(J, Gb) + (rb * p.rho0) * fill_grad(p, xi);
+    const J3<T> J = rows_of(wd.grad, i);
+    xs = xs + jt_mul(J, Gb) + (rb * p.rho0) * wd.fill[i];
     xbar[i] = xbar[i] + xs;
 }
 
@@ -1416,6 +1578,8 @@ struct AdjImpl : AdjBase {
     T *rhobar = nullptr, *rhonbar = nullptr, *alphabar = nullptr, *kdbar = nullptr, *pbar = nullptr,
       *ppbar = nullptr, *ppbar_next = nullptr, *dbar = nullptr, *rbt = nullptr, *sbar = nullptr;
     V3<T> *gbar = nullptr;
+    PairG<T> *pair = nullptr;  // the reversed substep's pair values beside its list
+    WallDerivs<T> walls{};     // and its particles' wall derivatives
     double *fbar = nullptr, *cbar = nullptr;
 
     ~AdjImpl() override {
@@ -1528,6 +1692,12 @@ struct AdjImpl : AdjBase {
         arena.want(&rbt, N);
         arena.want(&sbar, N);
         arena.want(&gbar, N);
+        arena.want(&pair, N * kModelCap);
+        for (int r = 0; r < 3; ++r) {
+            arena.want(&walls.grad[r], N);
+            arena.want(&walls.adh[r], N);
+        }
+        arena.want(&walls.fill, N);
         arena.want(&pbar, N);
         arena.want(&ppbar, N);
         arena.want(&ppbar_next, N);
@@ -1756,46 +1926,51 @@ struct AdjImpl : AdjBase {
         return FLUID_OK;
     }
 
+    // What the reverse sweeps share of positions xs: pair values and walls.
+    void reverse_geometry(const V3<T> *xs, const uint32_t *nb, const uint32_t *nbn) {
+        k_r_pairs<T><<<nblk(n * kLanes, kAdjThreads), kAdjThreads, 0, stream>>>(mp, n, xs, nb, nbn, pair);
+        k_r_walls<T><<<nblk(n, kAdjThreads), kAdjThreads, 0, stream>>>(mp, n, xs, walls);
+    }
+
     // The density pass reversed: total rho, G and S adjoints, then x.
-    void reverse_density(const V3<T> *xs, const uint32_t *nb, const uint32_t *nbn, const T *rho) {
+    void reverse_density(const V3<T> *xs, const Tape<T> &t) {
         const uint32_t B = nblk(n * kLanes, kAdjThreads);
-        k_r_density_a<T><<<B, kAdjThreads, 0, stream>>>(mp, n, xs, nb, nbn, rho, rhobar, alphabar, rbt, gbar, sbar);
-        k_r_density_b<T><<<B, kAdjThreads, 0, stream>>>(mp, n, xs, nb, nbn, rbt, gbar, sbar, rhonbar, xbar);
+        k_r_density_a<T><<<B, kAdjThreads, 0, stream>>>(mp, n, xs, t.nbr, pair, t.wg, t.nbr_n, t.rho, rhobar, alphabar,
+                                                        rbt, gbar, sbar);
+        k_r_density_b<T><<<B, kAdjThreads, 0, stream>>>(mp, n, xs, t.nbr, t.nbr_n, rbt, gbar, sbar, rhonbar, walls,
+                                                        xbar);
     }
 
     void reverse_substep(uint32_t k, const Tape<T> &t) {
         const uint32_t B = nblk(n * kLanes, kAdjThreads), B2 = nblk(n, 256);
         const uint32_t nd = div_it[k], ne = den_it[k];
-        const size_t N = n;
-        k_r_integrate<T><<<B2, 256, 0, stream>>>(mp, n, dt, vclamp, t.x, t.vden[ne], t.rho, xbar, vbar);
-        cudaMemcpyAsync(pbar, ppbar_next, sizeof(T) * N, cudaMemcpyDeviceToDevice, stream);
-        cudaMemsetAsync(rhobar, 0, sizeof(T) * N, stream);
-        cudaMemsetAsync(rhonbar, 0, sizeof(T) * N, stream);
-        cudaMemsetAsync(alphabar, 0, sizeof(T) * N, stream);
+        reverse_geometry(t.x, t.nbr, t.nbr_n);
+        k_r_integrate<T><<<B2, 256, 0, stream>>>(mp, n, dt, vclamp, t.x, t.vden[ne], t.rho, xbar, vbar, ppbar_next,
+                                                 pbar, rhobar, rhonbar, alphabar);
         for (uint32_t q = ne; q-- > 0;) {
-            k_r_apply<T><<<B, kAdjThreads, 0, stream>>>(mp, n, dt, t.x, t.nbr, t.nbr_n, t.kdden[q], t.wg, vbar,
-                                                        kdbar, xbar);
-            k_r_kappa_a<T><<<B, kAdjThreads, 0, stream>>>(mp, n, 1, dt, t.x, t.vden[q], t.nbr, t.nbr_n, t.rho,
+            k_r_apply<T><<<B, kAdjThreads, 0, stream>>>(mp, n, dt, t.x, t.nbr, pair, t.nbr_n, t.kdden[q], t.wg, vbar,
+                                                        walls, kdbar, xbar);
+            k_r_kappa_a<T><<<B, kAdjThreads, 0, stream>>>(mp, n, 1, dt, t.x, t.vden[q], t.nbr, pair, t.nbr_n, t.rho,
                                                           t.alpha, t.wg, kdbar, pbar, dbar, rhobar, alphabar);
-            k_r_kappa_b<T><<<B, kAdjThreads, 0, stream>>>(mp, n, t.x, t.vden[q], t.nbr, t.nbr_n, t.wg, dbar, vbar,
-                                                          xbar);
+            k_r_kappa_b<T><<<B, kAdjThreads, 0, stream>>>(mp, n, t.x, t.vden[q], t.nbr, pair, t.nbr_n, t.wg, dbar,
+                                                          walls, vbar, xbar);
         }
-        k_r_forces_apply<T><<<B, kAdjThreads, 0, stream>>>(mp, n, dt, T(xsph), t.x, t.blend, t.nbr, t.nbr_n, t.kdf,
-                                                           t.wg, vbar, abar, bbar, kdbar, xbar, part);
+        k_r_forces_apply<T><<<B, kAdjThreads, 0, stream>>>(mp, n, dt, T(xsph), t.x, t.blend, t.nbr, pair, t.nbr_n,
+                                                           t.kdf, t.wg, vbar, walls, abar, bbar, kdbar, xbar, part);
         double *fk = fbar + 3 * (size_t)k;
         k_sum_parts<<<1, 256, 0, stream>>>(part, B, Sum4Out{{fk, fk + 1, fk + 2, cbar}, 1});
         k_r_forces_eval<T><<<B, kAdjThreads, 0, stream>>>(mp, n, t.x, t.vdiv[nd], t.nbr, t.nbr_n, t.rho, t.rhon,
-                                                          t.pp, abar, bbar, kdbar, pbar, xbar, vbar, rhobar, rhonbar,
-                                                          ppbar);
+                                                          t.pp, abar, bbar, kdbar, pbar, walls, xbar, vbar, rhobar,
+                                                          rhonbar, ppbar);
         for (uint32_t q = nd; q-- > 0;) {
-            k_r_apply<T><<<B, kAdjThreads, 0, stream>>>(mp, n, dt, t.x, t.nbr, t.nbr_n, t.kddiv[q], t.wg, vbar,
-                                                        kdbar, xbar);
-            k_r_kappa_a<T><<<B, kAdjThreads, 0, stream>>>(mp, n, 0, dt, t.x, t.vdiv[q], t.nbr, t.nbr_n, t.rho,
+            k_r_apply<T><<<B, kAdjThreads, 0, stream>>>(mp, n, dt, t.x, t.nbr, pair, t.nbr_n, t.kddiv[q], t.wg, vbar,
+                                                        walls, kdbar, xbar);
+            k_r_kappa_a<T><<<B, kAdjThreads, 0, stream>>>(mp, n, 0, dt, t.x, t.vdiv[q], t.nbr, pair, t.nbr_n, t.rho,
                                                           t.alpha, t.wg, kdbar, nullptr, dbar, rhobar, alphabar);
-            k_r_kappa_b<T><<<B, kAdjThreads, 0, stream>>>(mp, n, t.x, t.vdiv[q], t.nbr, t.nbr_n, t.wg, dbar, vbar,
-                                                          xbar);
+            k_r_kappa_b<T><<<B, kAdjThreads, 0, stream>>>(mp, n, t.x, t.vdiv[q], t.nbr, pair, t.nbr_n, t.wg, dbar,
+                                                          walls, vbar, xbar);
         }
-        reverse_density(t.x, t.nbr, t.nbr_n, t.rho);
+        reverse_density(t.x, t);
         // back to the order the substep started from
         k_r_unpermute<T><<<B2, 256, 0, stream>>>(n, t.perm, xbar, vbar, ppbar, xbar2, vbar2, ppbar_next);
         std::swap(xbar, xbar2);
@@ -1819,7 +1994,8 @@ struct AdjImpl : AdjBase {
                                  T(2.0 * (com[2] - target[2]) / n)};
         k_r_loss<T><<<nblk(n, 256), 256, 0, stream>>>(mp, n, fin.rho, gcom, xbar, vbar, rhobar, rhonbar, alphabar,
                                                       ppbar_next);
-        reverse_density(x, fin.nbr, fin.nbr_n, fin.rho);
+        reverse_geometry(x, fin.nbr, fin.nbr_n);
+        reverse_density(x, fin);
         AK(cudaGetLastError());
         const uint32_t nseg = (frames + ce - 1) / ce;
         for (uint32_t q = nseg; q-- > 0;) {
