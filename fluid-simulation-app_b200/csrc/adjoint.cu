@@ -46,6 +46,7 @@
 
 #include "arena.cuh"
 #include "grid.cuh"
+#include "wide.cuh"
 
 namespace fcu {
 int32_t report_error(int32_t code, const std::string &msg);
@@ -72,11 +73,12 @@ constexpr int kAdjThreads = 128;
 constexpr uint32_t kModelCap = 128;  // neighbours a particle may have in the model
 // The model's grid keys are cell * kAdjSlabs + the x slab, as a simulation's:
 // each cell's particles in slab order, so the density sweep can skip the
-// stencil cells and x slabs beyond the support (ADJ_CULL).
+// stencil cells and x slabs beyond the support.
 constexpr uint32_t kAdjSlabs = kSimSlabs;
-#ifndef ADJ_CULL
-#define ADJ_CULL 1
-#endif
+// Threads up to which the density sweep takes 8 lanes a particle instead of
+// 4: two block waves. Forward of 8,192 particles in 64 bits 1.007 ms at 8,
+// 1.091 at 4, 1.030 at 16; of 65,536 in 32 bits 4.316, 4.251 and 4.514.
+constexpr uint32_t kDensityMost = 148u * 2048u;
 
 // ---- small vector and dual types --------------------------------------------
 // Padded to four values, so that a record is one 16-byte load (two for
@@ -332,12 +334,6 @@ template <class T, class S> DEV void w_adh(const MP<T> &p, S x, S y, S z, S &ax,
     az = cst<S>(0.0f) - w_adhesion((z - p.lo[2]) * inv_h) + w_adhesion((p.hi[2] - z) * inv_h);
 }
 
-template <class T> DEV V3<T> wall_grad(const MP<T> &p, V3<T> x) {
-    V3<T> g;
-    w_grad<T, T>(p, x.x, x.y, x.z, g.x, g.y, g.z);
-    return g;
-}
-
 // J^T u for the Jacobian of a wall vector field at x (rows = components).
 template <class T> struct J3 {
     T a[3][3];  // a[row][col] = d field_row / d x_col
@@ -439,102 +435,198 @@ __global__ void __launch_bounds__(256) k_m_pos4(const V3<T> *__restrict__ x, flo
 // near density, alpha and the wall gradient. With `perm`
 // null the particles are in the grid's cell order (slot k is particle k);
 // otherwise slot k holds particle perm[k].
-template <class T>
-__global__ void __launch_bounds__(kAdjThreads) k_m_density(MP<T> p, uint32_t n, const V3<T> *__restrict__ x,
-                                                           const float4 *__restrict__ pos4,
-                                                           const uint32_t *__restrict__ starts,
-                                                           const uint32_t *__restrict__ perm, uint32_t *nbr,
-                                                           T *gsl, uint32_t *nbr_n, T *rho, T *rhon, T *alpha,
-                                                           V3<T> *wg, uint32_t *over) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+//
+// L lanes a particle, as the simulations' small density sweep: the lanes form
+// the stencil rows, test candidates side by side (a ballot keeps the hits in
+// stencil order), form the staged hits' terms side by side and add them in
+// order, and share the walls' polynomials. With one thread a particle the
+// model's 8k to 64k particles waited on one particle's walk: a forward of
+// 8,192 in 64 bits 1.61 -> 1.01 ms (8 substeps), of 65,536 in 32 bits 4.65 ->
+// 4.25 (16 substeps).
+template <class T, int L>
+__global__ void __launch_bounds__(kWideThreads) k_m_density(MP<T> p, uint32_t n, const V3<T> *__restrict__ x,
+                                                            const uint32_t *__restrict__ starts,
+                                                            const uint32_t *__restrict__ perm, uint32_t *nbr,
+                                                            T *gsl, uint32_t *nbr_n, T *rho, T *rhon, T *alpha,
+                                                            V3<T> *wg, uint32_t *over) {
+    constexpr int kGroups = 32 / L, U = kWideLoads<L>;
+    __shared__ __align__(16) T s_rows[kWideWarps][6][kRowOf<T>];
+    __shared__ uint32_t s_hit[kWideWarps][kGroups][kWideCap<L>];
+    __shared__ uint32_t s_beg[kWideWarps][kGroups][9], s_len[kWideWarps][kGroups][9];
+    const uint32_t warp = threadIdx.x >> 5, at = threadIdx.x & 31u;
+    const WideLane w = wide_lane<L>(n);
+    const uint32_t i = w.i;
     const V3<T> xi = x[i];
-    const float4 pf = make_float4((float)xi.x, (float)xi.y, (float)xi.z, 0.0f);
-    const int bx = (int)axis_cell(pf.x, p.box_min[0], p.cell, p.dims[0]);
-    const int by = (int)axis_cell(pf.y, p.box_min[1], p.cell, p.dims[1]);
-    const int bz = (int)axis_cell(pf.z, p.box_min[2], p.cell, p.dims[2]);
-    T w_sum = p.sigma, near = T(0), gsq = T(0);
-    V3<T> gsum = zero3<T>();
-    uint32_t cnt = 0;
-#if ADJ_CULL
-    // Stencil cells and x slabs beyond the support skipped, as in the
-    // simulation's density sweep: on the float position the grid was built
-    // from, the distances to the own cell's faces shrunk by a margin far
-    // above both its rounding and the float / T difference of positions.
-    const float cellf = p.cell, sup2f = (float)p.sup2;
-    const float margin = 1e-3f * cellf + 1e-6f * (fabsf(pf.x) + fabsf(pf.y) + fabsf(pf.z));
-    const float fx = pf.x - (p.box_min[0] + (float)bx * cellf);
-    const float fy = pf.y - (p.box_min[1] + (float)by * cellf);
-    const float fz = pf.z - (p.box_min[2] + (float)bz * cellf);
-    const float xl = fmaxf(fx - margin, 0.0f), xh = fmaxf(cellf - fx - margin, 0.0f);
-    const float yl = fmaxf(fy - margin, 0.0f), yh = fmaxf(cellf - fy - margin, 0.0f);
-    const float zl = fmaxf(fz - margin, 0.0f), zh = fmaxf(cellf - fz - margin, 0.0f);
-#endif
-    for (int oz = -1; oz <= 1; ++oz)
-        for (int oy = -1; oy <= 1; ++oy) {
+    uint32_t *beg = s_beg[warp][w.group], *len = s_len[warp][w.group], *hit = s_hit[warp][w.group];
+    {
+        // Stencil cells and x slabs beyond the support are skipped, as in the
+        // simulation's density sweep: on the float position the grid was built
+        // from, the distances to the own cell's faces shrunk by a margin far
+        // above both its rounding and the float / T difference of positions.
+        const float px = (float)xi.x, py = (float)xi.y, pz = (float)xi.z;
+        const int bx = (int)axis_cell(px, p.box_min[0], p.cell, p.dims[0]);
+        const int by = (int)axis_cell(py, p.box_min[1], p.cell, p.dims[1]);
+        const int bz = (int)axis_cell(pz, p.box_min[2], p.cell, p.dims[2]);
+        const float cellf = p.cell, sup2f = (float)p.sup2;
+        const float margin = 1e-3f * cellf + 1e-6f * (fabsf(px) + fabsf(py) + fabsf(pz));
+        const float fx = px - (p.box_min[0] + (float)bx * cellf);
+        const float fy = py - (p.box_min[1] + (float)by * cellf);
+        const float fz = pz - (p.box_min[2] + (float)bz * cellf);
+        const float xl = fmaxf(fx - margin, 0.0f), xh = fmaxf(cellf - fx - margin, 0.0f);
+        const float yl = fmaxf(fy - margin, 0.0f), yh = fmaxf(cellf - fy - margin, 0.0f);
+        const float zl = fmaxf(fz - margin, 0.0f), zh = fmaxf(cellf - fz - margin, 0.0f);
+        for (uint32_t r = w.lane; r < 9u; r += L) {
+            const int oz = (int)(r / 3u) - 1, oy = (int)(r % 3u) - 1;
             const int cz = bz + oz, cy = by + oy;
-            if (cz < 0 || cz >= (int)p.dims[2] || cy < 0 || cy >= (int)p.dims[1]) continue;
-            const uint32_t row = ((uint32_t)cz * p.dims[1] + (uint32_t)cy) * p.dims[0];
-#if ADJ_CULL
+            uint32_t s = 0, e = 0;
             const float dperp = (oz < 0 ? zl * zl : (oz > 0 ? zh * zh : 0.0f)) +
                                 (oy < 0 ? yl * yl : (oy > 0 ? yh * yh : 0.0f));
-            if (dperp >= sup2f) continue;
-            const int cx0 = (bx > 0 && dperp + xl * xl < sup2f) ? bx - 1 : bx;
-            const int cx1 = (bx + 1 < (int)p.dims[0] && dperp + xh * xh < sup2f) ? bx + 1 : bx;
-            const float w = sqrtf(sup2f - dperp) * 1.001f + margin;
-            const float xa = pf.x - w, xb = pf.x + w;
-            const uint32_t ca = axis_cell(xa, p.box_min[0], cellf, p.dims[0]);
-            const uint32_t cb = axis_cell(xb, p.box_min[0], cellf, p.dims[0]);
-            const uint32_t klo = max(ca * kAdjSlabs + axis_slab(xa, p.box_min[0], cellf, ca, kAdjSlabs),
-                                     (uint32_t)cx0 * kAdjSlabs);
-            const uint32_t khi = min(cb * kAdjSlabs + axis_slab(xb, p.box_min[0], cellf, cb, kAdjSlabs),
-                                     (uint32_t)cx1 * kAdjSlabs + (kAdjSlabs - 1));
-            uint32_t s = starts[row * kAdjSlabs + klo], e = starts[row * kAdjSlabs + khi + 1];
-            if (s > e) s = e;
-#else
-            const int cx0 = bx > 0 ? bx - 1 : bx;
-            const int cx1 = bx + 1 < (int)p.dims[0] ? bx + 1 : bx;
-            uint32_t s = starts[(row + cx0) * kAdjSlabs], e = starts[(row + cx1 + 1) * kAdjSlabs];
-#endif
-            if (e > n) e = n;
-            // candidates four at a time: their positions load together
-            for (uint32_t k0 = s; k0 < e; k0 += 4) {
-                uint32_t jj[4];
-                V3<T> xj[4];
+            if (w.live && cz >= 0 && cz < (int)p.dims[2] && cy >= 0 && cy < (int)p.dims[1] && dperp < sup2f) {
+                const uint32_t row = ((uint32_t)cz * p.dims[1] + (uint32_t)cy) * p.dims[0];
+                const int cx0 = (bx > 0 && dperp + xl * xl < sup2f) ? bx - 1 : bx;
+                const int cx1 = (bx + 1 < (int)p.dims[0] && dperp + xh * xh < sup2f) ? bx + 1 : bx;
+                const float half = sqrtf(sup2f - dperp) * 1.001f + margin;
+                const float xa = px - half, xb = px + half;
+                const uint32_t ca = axis_cell(xa, p.box_min[0], cellf, p.dims[0]);
+                const uint32_t cb = axis_cell(xb, p.box_min[0], cellf, p.dims[0]);
+                const uint32_t klo = max(ca * kAdjSlabs + axis_slab(xa, p.box_min[0], cellf, ca, kAdjSlabs),
+                                         (uint32_t)cx0 * kAdjSlabs);
+                const uint32_t khi = min(cb * kAdjSlabs + axis_slab(xb, p.box_min[0], cellf, cb, kAdjSlabs),
+                                         (uint32_t)cx1 * kAdjSlabs + (kAdjSlabs - 1));
+                s = starts[row * kAdjSlabs + klo];
+                e = min(starts[row * kAdjSlabs + khi + 1], n);
+            }
+            beg[r] = s;
+            len[r] = s < e ? e - s : 0u;
+        }
+    }
+    __syncwarp();
+    WideRows c(beg, len, w.lane);
+    const uint32_t mine = group_mask<L>(w), before = mine & ((1u << at) - 1u);
+    WideSums<T, L, 6> sums;
+    if (w.lane == 0) sums.acc[0] = p.sigma;
+    uint32_t cnt = 0;
+    bool more = true;
+    while (__any_sync(0xffffffffu, more)) {
+        uint32_t staged = 0;
+        while (__any_sync(0xffffffffu, more && staged < kWideStage)) {
+            const bool scan = more && staged < kWideStage;
+            uint32_t j[U];
+            V3<T> xj[U];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const uint32_t k = k0 + u;
-                    const uint32_t jr = k < e ? (perm ? perm[k] : k) : i;
-                    jj[u] = jr;
-                    xj[u] = x[jr < n ? jr : i];
+            for (int u = 0; u < U; ++u) {
+                uint32_t k = i;
+                if (scan && c.any()) {
+                    k = c.at();
+                    if (perm) k = perm[k];
+                    if (k >= n) k = i;  // only after a grid build that gave up
                 }
+                j[u] = k;
+                xj[u] = x[k];
+                if (scan) c.next<L>();
+            }
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                const uint32_t j = jj[u];
-                if (k0 + u >= e || j == i || j >= n) continue;
+            for (int u = 0; u < U; ++u) {
                 const V3<T> xij = xi - xj[u];
-                const T r2 = dot(xij, xij);
-                if (r2 >= p.sup2) continue;
-                const Radial<T> R = radial(p, r2);
-                w_sum += R.W;
+                const bool is = j[u] != i && dot(xij, xij) < p.sup2;
+                const uint32_t hits = __ballot_sync(0xffffffffu, is);
+                if (is) hit[staged + __popc(hits & before)] = j[u];
+                staged += __popc(hits & mine);
+            }
+            // the group's first lane has the group's earliest candidate
+            const uint32_t row0 = __shfl_sync(0xffffffffu, c.row, 0, L);
+            if (scan) more = row0 < 9u;
+        }
+        __syncwarp();
+        const uint32_t most = __reduce_max_sync(0xffffffffu, staged);
+        for (uint32_t h0 = 0; h0 < most; h0 += L) {
+            const uint32_t h = h0 + w.lane;
+            T t[6];
+#pragma unroll
+            for (int a = 0; a < 6; ++a) t[a] = T(0);
+            if (h < staged) {
+                const uint32_t jj = hit[h];
+                const V3<T> xij = xi - x[jj];
+                const Radial<T> R = radial(p, dot(xij, xij));
+                t[0] = R.W;
                 const T wn = R.q < T(1) ? T(1) - R.q : T(0);
-                near += wn * wn * wn;
+                t[1] = wn * wn * wn;
                 const V3<T> gw = R.gs * xij;
-                gsum = gsum + gw;
-                gsq += dot(gw, gw);
-                if (cnt < kModelCap) {
-                    nbr[(size_t)cnt * n + i] = j;
-                    if (gsl) gsl[(size_t)cnt * n + i] = R.gs;
-                }
-                cnt++;
+                t[2] = gw.x;
+                t[3] = gw.y;
+                t[4] = gw.z;
+                t[5] = dot(gw, gw);
+                const uint32_t idx = cnt + h;
+                if (idx < kModelCap) {
+                    nbr[(size_t)idx * n + i] = jj;
+                    if (gsl) gsl[(size_t)idx * n + i] = R.gs;
                 }
             }
+#pragma unroll
+            for (int a = 0; a < 6; ++a) s_rows[warp][a][at] = t[a];
+            __syncwarp();
+            sums.add(s_rows[warp], w);
+            __syncwarp();
         }
+        cnt += staged;
+    }
+    const T w_sum = sums.template get<0>(), near = sums.template get<1>();
+    const V3<T> gsum = mk(sums.template get<2>(), sums.template get<3>(), sums.template get<4>());
+    const T gsq = sums.template get<5>();
+
+    // the walls, w_fill and w_grad's terms spread over the lanes: wall q (axis
+    // q % 3, side q / 3) and edge q (axes xy, xz, yz by q / 4)
+    auto to_wall = [&](int a, bool high, T inv) {
+        return high ? (p.hi[a] - comp(xi, a)) * inv : (comp(xi, a) - p.lo[a]) * inv;
+    };
+    const T inv_h = T(1) / p.h;  // as w_grad; w_fill uses the float constant
+    constexpr int kWallPer = (6 + L - 1) / L, kEdgePer = (12 + L - 1) / L;
+    T wd[kWallPer], wgr[kWallPer], edge[kEdgePer];
+#pragma unroll
+    for (int u = 0; u < kWallPer; ++u) {
+        const int q = (int)w.lane + u * L;
+        wd[u] = wgr[u] = T(0);
+        if (q < 6) {
+            const int a = q % 3, c1 = a == 0 ? 1 : 0, c2 = a == 2 ? 1 : 2;
+            wd[u] = w_density(to_wall(a, q >= 3, p.inv_h));
+            const T t = to_wall(a, q >= 3, inv_h);
+            wgr[u] = w_gradient(t) + w_dsum(t, to_wall(c1, false, inv_h), to_wall(c1, true, inv_h),
+                                            to_wall(c2, false, inv_h), to_wall(c2, true, inv_h));
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < kEdgePer; ++u) {
+        const int q = (int)w.lane + u * L;
+        edge[u] = T(0);
+        if (q < 12) {
+            const int a = q / 4 == 2 ? 1 : 0, b = q / 4 == 0 ? 1 : 2;
+            edge[u] = w_wedge(to_wall(a, (q & 2) != 0, p.inv_h), to_wall(b, (q & 1) != 0, p.inv_h));
+        }
+    }
+    T D[6], S[6], E[12];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        D[q] = __shfl_sync(0xffffffffu, wd[q / L], q % L, L);
+        S[q] = __shfl_sync(0xffffffffu, wgr[q / L], q % L, L);
+    }
+#pragma unroll
+    for (int q = 0; q < 12; ++q) E[q] = __shfl_sync(0xffffffffu, edge[q / L], q % L, L);
+    if (!w.live || w.lane != 0) return;
+    T f = T(0);
+    f = f + (D[0] + D[3]);
+    f = f + (D[1] + D[4]);
+    f = f + (D[2] + D[5]);
+    T ws = E[0] + E[1] + E[2] + E[3];
+    ws = ws + (E[4] + E[5] + E[6] + E[7]);
+    ws = ws + (E[8] + E[9] + E[10] + E[11]);
+    const T scale = p.rho0 * inv_h;
+    V3<T> g = mk(T(0) - scale * S[0], T(0) - scale * S[1], T(0) - scale * S[2]);
+    g.x = g.x + scale * S[3];
+    g.y = g.y + scale * S[4];
+    g.z = g.z + scale * S[5];
     nbr_n[i] = cnt < kModelCap ? cnt : kModelCap;
     if (cnt > kModelCap) atomicAdd(over, 1u);
-    const T fill = w_fill<T, T>(p, xi.x, xi.y, xi.z);
-    const T r = p.m * w_sum + p.rho0 * fill;
-    const V3<T> g = wall_grad(p, xi);
+    const T r = p.m * w_sum + p.rho0 * (f - ws);
     wg[i] = g;
     const V3<T> G = p.m * gsum + g;
     T den = dot(G, G) + p.m * p.m * gsq;
@@ -864,11 +956,13 @@ __global__ void __launch_bounds__(kAdjThreads) k_m_forces_apply(MP<T> p, uint32_
     v_out[i] = forced - dt * (p.m * s + kdi * wg[i]);
 }
 
-// integrate without the lenses and temperature (sim_solve.wgsl:709-756)
+// integrate without the lenses and temperature (sim_solve.wgsl:709-756); also
+// leaves the positions the next substep's grid is built from
 template <class T>
 __global__ void __launch_bounds__(256) k_m_integrate(MP<T> p, uint32_t n, T dt, T vclamp, const V3<T> *x_in,
                                                      V3<T> *x_out, const V3<T> *__restrict__ v_in, V3<T> *v_out,
-                                                     const T *__restrict__ pressure, T *pp, const T *__restrict__ rho) {
+                                                     const T *__restrict__ pressure, T *pp, const T *__restrict__ rho,
+                                                     float4 *pos4) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     V3<T> v = v_in[i];
@@ -888,6 +982,7 @@ __global__ void __launch_bounds__(256) k_m_integrate(MP<T> p, uint32_t n, T dt, 
     }
     o = mk(oa[0], oa[1], oa[2]);
     x_out[i] = o;
+    pos4[i] = make_float4((float)o.x, (float)o.y, (float)o.z, 0.0f);  // the next grid's positions
     v_out[i] = mk(va[0], va[1], va[2]);
     pp[i] = pressure[i];
 }
@@ -1725,12 +1820,19 @@ struct AdjImpl : AdjBase {
         AK(cudaMemcpyAsync(x, x_init, sizeof(V3<T>) * n, cudaMemcpyDeviceToDevice, stream));
         AK(cudaMemsetAsync(v, 0, sizeof(V3<T>) * n, stream));
         AK(cudaMemsetAsync(pp, 0, sizeof(T) * n, stream));
+        return grid_positions();
+    }
+
+    // The grid's positions of a state that no integrate left (the initial
+    // one, a checkpoint).
+    int32_t grid_positions() {
+        k_m_pos4<T><<<nblk(n, 256), 256, 0, stream>>>(x, pos4, n);
+        AK(cudaGetLastError());
         return FLUID_OK;
     }
 
-    // Neighbour grid of positions xs (the state's order): starts and perm.
-    int32_t grid(const V3<T> *xs) {
-        k_m_pos4<T><<<nblk(n, 256), 256, 0, stream>>>(xs, pos4, n);
+    // Neighbour grid of the state's positions (pos4): starts and perm.
+    int32_t grid() {
         GridGeom g;
         for (int a = 0; a < 3; ++a) {
             g.min[a] = P.box_min[a];
@@ -1742,13 +1844,22 @@ struct AdjImpl : AdjBase {
         return FLUID_OK;
     }
 
-    // Neighbour grid of positions xs, then lists and densities into t (the
+    // k_m_density at 8 or 4 lanes a particle (kDensityMost).
+    void launch_density(const V3<T> *xs, const uint32_t *pm, T *scales, Tape<T> &t) {
+        auto at = [&](auto kernel, uint32_t lanes) {
+            kernel<<<nblk(n, kWideThreads / lanes), kWideThreads, 0, stream>>>(
+                mp, n, xs, starts, pm, t.nbr, scales, t.nbr_n, t.rho, t.rhon, t.alpha, t.wg, over);
+        };
+        if ((uint64_t)n * 8 <= kDensityMost) at(k_m_density<T, 8>, 8);
+        else at(k_m_density<T, 4>, 4);
+    }
+
+    // Neighbour grid of the state's positions xs, then lists and densities into t (the
     // loss's pass over the final state, which is not in its own cell order).
     int32_t density(const V3<T> *xs, Tape<T> &t) {
-        const int32_t rc = grid(xs);
+        const int32_t rc = grid();
         if (rc != FLUID_OK) return rc;
-        k_m_density<T><<<nblk(n, kAdjThreads), kAdjThreads, 0, stream>>>(
-            mp, n, xs, pos4, starts, perm, t.nbr, nullptr, t.nbr_n, t.rho, t.rhon, t.alpha, t.wg, over);
+        launch_density(xs, perm, nullptr, t);
         AK(cudaGetLastError());
         return FLUID_OK;
     }
@@ -1768,13 +1879,12 @@ struct AdjImpl : AdjBase {
     int32_t substep(uint32_t k, V3<T> f, T c, Tape<T> &t, bool record) {
         const bool decide = !frozen && !record;
         // the state in cell order, then lists and densities over slots
-        int32_t rc = grid(x);
+        int32_t rc = grid();
         if (rc != FLUID_OK) return rc;
         k_m_gather<T><<<nblk(n, 256), 256, 0, stream>>>(n, perm, x, v, pp, id, t.x, t.vdiv[0], t.pp, id2, t.perm);
         std::swap(id, id2);
-        const uint32_t B = nblk(n, kAdjThreads), BL = nblk(n * kLanes, kAdjThreads);
-        k_m_density<T><<<B, kAdjThreads, 0, stream>>>(mp, n, t.x, pos4, starts, nullptr, t.nbr, gsl, t.nbr_n,
-                                                      t.rho, t.rhon, t.alpha, t.wg, over);
+        const uint32_t BL = nblk(n * kLanes, kAdjThreads);
+        launch_density(t.x, nullptr, gsl, t);
         // divergence loop
         uint32_t nd = decide ? 0u : div_it[k];
         if (decide) AK(cudaMemsetAsync(res_acc, 0, 8, stream));
@@ -1831,7 +1941,7 @@ struct AdjImpl : AdjBase {
             den_it[k] = it;
         }
         k_m_integrate<T><<<nblk(n, 256), 256, 0, stream>>>(mp, n, dt, vclamp, t.x, x, t.vden[it], v, pressure, pp,
-                                                           t.rho);
+                                                           t.rho, pos4);
         AK(cudaGetLastError());
         return FLUID_OK;
     }
@@ -2005,6 +2115,8 @@ struct AdjImpl : AdjBase {
             AK(cudaMemcpyAsync(v, ck_v[q], sizeof(V3<T>) * n, cudaMemcpyDeviceToDevice, stream));
             AK(cudaMemcpyAsync(pp, ck_pp[q], sizeof(T) * n, cudaMemcpyDeviceToDevice, stream));
             AK(cudaMemcpyAsync(id, ck_id[q], 4ull * n, cudaMemcpyDeviceToDevice, stream));
+            rc = grid_positions();
+            if (rc != FLUID_OK) return rc;
             for (uint32_t k = f0 * spf; k < f1 * spf; ++k) {
                 rc = substep(k, force_of(k), T(xsph), seg[k - f0 * spf], true);
                 if (rc != FLUID_OK) return rc;

@@ -16,6 +16,7 @@
 #include <cuda_fp16.h>
 
 #include "solve.cuh"
+#include "wide.cuh"
 
 // Neighbour batches of the list sweeps (see walk below): entries whose
 // records are loaded before any is used. Position + kappa records, position

@@ -6,72 +6,9 @@
 // walk, ~45 neighbours one after another, each a round trip to L2 and a
 // chain of square roots and divisions (37 us for the forces of 1,620
 // particles and 51 us for 16,384, on a GPU that does a million in 490 us).
-// Here the L lanes of a particle form L pairs' terms at once. Only the sums
-// must keep their order (they define the result's bits), and they are cheap:
-// the lanes leave their terms in shared memory, term-major, and lane a adds
-// term a of the L pairs in list order, so the additions of a chunk are L long
-// chains that run side by side, one per lane, instead of one per particle.
-// Empty places add +0, which changes no sum (a sum that starts at +0 never
-// becomes -0). Every result is the one-thread sweep's, bit for bit.
-
-constexpr int kWideThreads = 128;
-constexpr int kWideWarps = kWideThreads / 32;
-// A term's row of 32 lanes, padded so that the lanes of a group read their
-// rows' 16-byte pieces from different banks.
-constexpr int kRowPad = 36;
-
-// Lane `lane` of the group holding particle i. Every lane of a warp stays to
-// the end; those past n work on the last particle with nothing to walk.
-struct WideLane {
-    uint32_t i, lane, group;  // group: the particle's place in its warp
-    bool live;
-};
-template <int L>
-__device__ __forceinline__ WideLane wide_lane(uint32_t n) {
-    const uint32_t t = blockIdx.x * kWideThreads + threadIdx.x;
-    const uint32_t i = t / L;
-    return WideLane{i < n ? i : n - 1, t % L, (threadIdx.x & 31u) / L, i < n};
-}
-
-// acc plus the L values of a row's group, in order.
-template <int L>
-__device__ __forceinline__ float fold_row(float acc, const float *row) {
-#pragma unroll
-    for (int e = 0; e < L; e += 4) {
-        const float4 q = *reinterpret_cast<const float4 *>(row + e);
-        acc += q.x;
-        acc += q.y;
-        acc += q.z;
-        acc += q.w;
-    }
-    return acc;
-}
-
-// The sums of R terms over a group's pairs: lane a keeps those of terms a,
-// a + L, ...
-template <int L, int R>
-struct WideSums {
-    static constexpr int kPer = (R + L - 1) / L;
-    float acc[kPer];
-    __device__ __forceinline__ WideSums() {
-#pragma unroll
-        for (int q = 0; q < kPer; ++q) acc[q] = 0.0f;
-    }
-    // Adds one chunk: `rows` holds the warp's terms, written before a
-    // __syncwarp by every lane.
-    __device__ __forceinline__ void add(const float (*rows)[kRowPad], const WideLane &w) {
-#pragma unroll
-        for (int q = 0; q < kPer; ++q) {
-            const int a = (int)w.lane + q * L;
-            if (a < R) acc[q] = fold_row<L>(acc[q], rows[a] + w.group * L);
-        }
-    }
-    // Term a's sum, on every lane of the group.
-    template <int A>
-    __device__ __forceinline__ float get() const {
-        return __shfl_sync(0xffffffffu, acc[A / L], A % L, L);
-    }
-};
+// Here the L lanes of a particle form L pairs' terms at once and add them in
+// list order (wide.cuh), so every result is the one-thread sweep's, bit for
+// bit.
 
 // Walks the list of the group's particle, L entries at a time: each lane
 // loads one entry and its neighbour's record and calls terms(scale, record)
@@ -79,7 +16,7 @@ struct WideSums {
 // next chunk's entries are asked for before this chunk's records are used.
 template <int L, int R, class T, class Load, class Terms, class Fold>
 __device__ __forceinline__ void walk_wide(const uint2 *__restrict__ nbr, uint32_t n, const WideLane &w, uint32_t cnt,
-                                          float (*rows)[kRowPad], Load load, Terms terms, Fold fold) {
+                                          float (*rows)[kRowOf<float>], Load load, Terms terms, Fold fold) {
     const uint32_t most = __reduce_max_sync(0xffffffffu, cnt);
     const uint32_t at = threadIdx.x & 31u;
     uint2 e = w.lane < cnt ? list_ld(&nbr[(size_t)w.lane * n + w.i]) : make_uint2(w.i, 0u);
@@ -109,18 +46,12 @@ __device__ __forceinline__ void walk_wide(const uint2 *__restrict__ nbr, uint32_
 // candidates L at a time in stencil order; a ballot gives each hit its place
 // in the particle's staged list. The staged hits are then processed L at a
 // time, and the boundary's polynomials are spread over the lanes.
-constexpr uint32_t kWideStage = 64;  // hits staged before they are processed
-template <int L>
-constexpr int kWideLoads = L >= 32 ? 2 : 4;  // candidates a lane loads before testing any
-template <int L>
-constexpr int kWideCap = (int)kWideStage + L * kWideLoads<L>;  // staged hits at most
-
 __device__ __forceinline__ float axis_of(F3 v, int a) { return a == 0 ? v.x : (a == 1 ? v.y : v.z); }
 
 template <bool kB, int L>
 __global__ void __launch_bounds__(kWideThreads) k_density_wide(const __grid_constant__ Geo g, SimBufs b, int slot) {
     constexpr int G = 32 / L, U = kWideLoads<L>;
-    __shared__ __align__(16) float s_rows[kWideWarps][7][kRowPad];
+    __shared__ __align__(16) float s_rows[kWideWarps][7][kRowOf<float>];
     __shared__ uint32_t s_hit[kWideWarps][G][kWideCap<L>];
     __shared__ uint32_t s_beg[kWideWarps][G][9], s_len[kWideWarps][G][9];
     const uint32_t n = g.n, warp = threadIdx.x >> 5, at = threadIdx.x & 31u;
@@ -144,18 +75,10 @@ __global__ void __launch_bounds__(kWideThreads) k_density_wide(const __grid_cons
         }
     }
     __syncwarp();
-    // this lane's next candidate: `off` in row `row`; 9 when the rows are done
-    uint32_t row = 0, off = w.lane;
-    auto settle = [&] {
-        while (row < 9u && off >= len[row]) {
-            off -= len[row];
-            ++row;
-        }
-    };
-    settle();
-    const uint32_t mine = L == 32 ? 0xffffffffu : ((1u << (L & 31)) - 1u) << (w.group * L);
+    WideRows c(beg, len, w.lane);
+    const uint32_t mine = group_mask<L>(w);
     const uint32_t before = mine & ((1u << at) - 1u);
-    WideSums<L, 7> sums;
+    WideSums<float, L, 7> sums;
     if (w.lane == 0) sums.acc[0] = P.sigma;  // the self term W(0), sim_solve.wgsl:426
     uint32_t found = 0;
     bool more = true;
@@ -167,12 +90,9 @@ __global__ void __launch_bounds__(kWideThreads) k_density_wide(const __grid_cons
             float4 pc[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                j[u] = scan && row < 9u ? beg[row] + off : i;  // i: nothing (a particle is not its own neighbour)
+                j[u] = scan && c.any() ? c.at() : i;  // i: nothing (a particle is not its own neighbour)
                 pc[u] = __ldg(&b.wpos[j[u]]);
-                if (scan) {
-                    off += L;
-                    settle();
-                }
+                if (scan) c.next<L>();
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -183,7 +103,7 @@ __global__ void __launch_bounds__(kWideThreads) k_density_wide(const __grid_cons
                 staged += __popc(hits & mine);
             }
             // the group's first lane has the group's earliest candidate
-            const uint32_t row0 = __shfl_sync(0xffffffffu, row, 0, L);
+            const uint32_t row0 = __shfl_sync(0xffffffffu, c.row, 0, L);
             if (scan) more = row0 < 9u;
         }
         __syncwarp();
@@ -291,10 +211,10 @@ __global__ void __launch_bounds__(kWideThreads) k_density_wide(const __grid_cons
 // divergence_sum over the group's lanes.
 template <int L>
 __device__ __forceinline__ float divergence_wide(const SimBufs &b, uint32_t n, const WideLane &w, bool on,
-                                                 float (*rows)[kRowPad]) {
+                                                 float (*rows)[kRowOf<float>]) {
     const F3 pos = xyz(__ldg(&b.wpos[w.i]));
     const F3 vel = xyz(__ldg(&b.wvel[w.i]));
-    WideSums<L, 1> sums;
+    WideSums<float, L, 1> sums;
     walk_wide<L, 1, PosVel>(
         b.nbr, n, w, on ? __ldg(&b.nbr_n[w.i]) : 0u, rows,
         [&](uint32_t j) { return PosVel{__ldg(&b.wpos[j]), __ldg(&b.wvel[j])}; },
@@ -305,7 +225,7 @@ __device__ __forceinline__ float divergence_wide(const SimBufs &b, uint32_t n, c
 
 template <bool kB, int L>
 __global__ void __launch_bounds__(kWideThreads) k_div_kappa_wide(Geo g, SimBufs b, int slot, int gate) {
-    __shared__ __align__(16) float s_rows[kWideWarps][1][kRowPad];
+    __shared__ __align__(16) float s_rows[kWideWarps][1][kRowOf<float>];
     const WideLane w = wide_lane<L>(g.n);
     const uint32_t bi = box_index<kB>(g, w.i);
     const bool on = w.live && !gated_out<kB>(g, bi, gate);
@@ -317,7 +237,7 @@ __global__ void __launch_bounds__(kWideThreads) k_div_kappa_wide(Geo g, SimBufs 
 
 template <bool kB, int L>
 __global__ void __launch_bounds__(kWideThreads) k_den_kappa_wide(Geo g, SimBufs b, int slot, int gate) {
-    __shared__ __align__(16) float s_rows[kWideWarps][1][kRowPad];
+    __shared__ __align__(16) float s_rows[kWideWarps][1][kRowOf<float>];
     const WideLane w = wide_lane<L>(g.n);
     const uint32_t bi = box_index<kB>(g, w.i);
     const bool on = w.live && !gated_out<kB>(g, bi, gate);
@@ -329,14 +249,14 @@ __global__ void __launch_bounds__(kWideThreads) k_den_kappa_wide(Geo g, SimBufs 
 
 template <bool kB, int L>
 __global__ void __launch_bounds__(kWideThreads) k_apply_wide(Geo g, SimBufs b, int add_pressure, int gate) {
-    __shared__ __align__(16) float s_rows[kWideWarps][3][kRowPad];
+    __shared__ __align__(16) float s_rows[kWideWarps][3][kRowOf<float>];
     const WideLane w = wide_lane<L>(g.n);
     const uint32_t bi = box_index<kB>(g, w.i);
     const bool on = w.live && !gated_out<kB>(g, bi, gate);
     const F3 pos = xyz(__ldg(&b.wpos[w.i]));
     const float kd_i = b.kd[w.i];
-    float(*rows)[kRowPad] = s_rows[threadIdx.x >> 5];
-    WideSums<L, 3> sums;
+    float(*rows)[kRowOf<float>] = s_rows[threadIdx.x >> 5];
+    WideSums<float, L, 3> sums;
     walk_wide<L, 3, float4>(
         b.nbr, g.n, w, on ? __ldg(&b.nbr_n[w.i]) : 0u, rows, [&](uint32_t j) { return __ldg(&b.wpk[j]); },
         [&](float gs, const float4 &q, float *t) {
@@ -354,14 +274,14 @@ __global__ void __launch_bounds__(kWideThreads) k_apply_wide(Geo g, SimBufs b, i
 // divergence, then the heat's two parts, which one lane adds in turn.
 template <bool kB, bool kDiv, int L>
 __global__ void __launch_bounds__(kWideThreads) k_forces_wide(Geo g, SimBufs b, int slot, int gate) {
-    __shared__ __align__(16) float s_rows[kWideWarps][18][kRowPad];
+    __shared__ __align__(16) float s_rows[kWideWarps][18][kRowOf<float>];
     const WideLane w = wide_lane<L>(g.n);
     const uint32_t bi = box_index<kB>(g, w.i);
     const bool on = w.live && !(kDiv && gated_out<kB>(g, bi, gate));
     const DevParams &P = params_ref<kB>(g, bi);
     const ForceCtx c = force_ctx(b, P, w.i);
-    float(*rows)[kRowPad] = s_rows[threadIdx.x >> 5];
-    WideSums<L, 16> sums;
+    float(*rows)[kRowOf<float>] = s_rows[threadIdx.x >> 5];
+    WideSums<float, L, 16> sums;
     float heat = 0.0f;
     walk_wide<L, 18, Nbr3>(
         b.nbr, g.n, w, on ? __ldg(&b.nbr_n[w.i]) : 0u, rows,
