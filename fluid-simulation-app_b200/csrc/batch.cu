@@ -185,14 +185,19 @@ int32_t batch_graph_tolerance(FluidBatch *s, cudaGraphExec_t *out) {
     const bool fused = c.max_iters >= 1;
     const SimBufs bd = divergence_bufs(s->b), bf = after_forces(s->b);
     if (e == cudaSuccess) {
-        launch_density_div(st, geo, bd, 0);
-        launch_tol_finish(st, geo, 0, 1, c.div_tol, c.max_iters, hdiv);
+        // the first divergence apply before the loop (as the one-box substep)
+        launch_density_div(st, geo, bd, fused ? 1 : 0);
+        if (fused) {
+            launch_apply(st, geo, bd, false, kGateNone);
+            launch_forces_div(st, geo, s->b, 0, kGateNone);
+        }
+        launch_tol_finish(st, geo, 0, fused ? 1 : 0, c.div_tol, c.max_iters, hdiv);
         rc = host_add_while(st, g, hdiv, &bdiv);
     }
     if (e == cudaSuccess && rc == FLUID_OK) {
         if (!fused) launch_forces_eval(st, geo, s->b);
         launch_den_kappa(st, geo, bf, 0, kGateNone);
-        launch_tol_finish(st, geo, 1, 1, c.den_tol, c.max_iters, hden);
+        launch_tol_finish(st, geo, 1, 0, c.den_tol, c.max_iters, hden);
         rc = host_add_while(st, g, hden, &bden);
     }
     if (e == cudaSuccess && rc == FLUID_OK) launch_integrate(st, geo, bf, -1, -1, 0, 0);
@@ -212,12 +217,12 @@ int32_t batch_graph_tolerance(FluidBatch *s, cudaGraphExec_t *out) {
     launch_apply(s->side, geo, bd, false, kGateDiv);
     if (fused) launch_forces_div(s->side, geo, s->b, 0, kGateDiv);
     else launch_div_kappa(s->side, geo, bd, 0, kGateDiv);
-    launch_tol_finish(s->side, geo, 0, 0, c.div_tol, c.max_iters, hdiv);
+    launch_tol_finish(s->side, geo, 0, kTolNext, c.div_tol, c.max_iters, hdiv);
     BK(cudaStreamEndCapture(s->side, &bdiv));
     BK(cudaStreamBeginCaptureToGraph(s->side, bden, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     launch_apply(s->side, geo, bf, true, kGateDen);
     launch_den_kappa(s->side, geo, bf, 0, kGateDen);
-    launch_tol_finish(s->side, geo, 1, 0, c.den_tol, c.max_iters, hden);
+    launch_tol_finish(s->side, geo, 1, kTolNext, c.den_tol, c.max_iters, hden);
     BK(cudaStreamEndCapture(s->side, &bden));
     e = cudaGraphInstantiate(&s->tol_graph, g, 0);
     cudaGraphDestroy(g);

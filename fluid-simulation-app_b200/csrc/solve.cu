@@ -1142,27 +1142,28 @@ __global__ void __launch_bounds__(TPB) k_integrate(Geo g, SimBufs b, int div_slo
 }
 
 // The tolerance loops' bookkeeping, one block over the boxes: for each box
-// whose loop runs (every box on the first call), read and clear its
-// residual accumulator of `which` (0 divergence, 1 density), count the
-// iteration unless `first`, record the residual, and go on while under
-// max_iters and above tol (the divergence loop always makes its first
-// apply, as the reference). The graph's loop continues while any box does.
-__global__ void __launch_bounds__(256) k_tol_finish(Geo g, int which, int first, float tol,
+// whose loop runs (every box on a substep's first call), read and clear its
+// residual accumulator of `which` (0 divergence, 1 density), record the
+// residual and the iterations made, and go on while under max_iters and
+// above tol (the divergence loop always makes its first apply, as the
+// reference). The graph's loop continues while any box does. `done` is the
+// iterations made before a substep's first call, or kTolNext inside the loop.
+__global__ void __launch_bounds__(256) k_tol_finish(Geo g, int which, int done, float tol,
                                                     uint32_t max_iters,
                                                     cudaGraphConditionalHandle handle) {
     int any = 0;
     for (uint32_t bi = threadIdx.x; bi < g.nboxes; bi += blockDim.x) {
         DevSolve *sv = &g.solve[bi];
         uint32_t *active = which == 0 ? &sv->div_active : &sv->den_active;
-        if (!first && !*active) continue;
+        if (done == kTolNext && !*active) continue;
         unsigned long long *acc = which == 0 ? &sv->acc_div[0] : &sv->acc_den[0];
         const uint32_t cnt = g.box_of ? g.box[bi].count : g.one.count;
         const double res = (double)*acc / kFixedScale / (double)cnt;
         *acc = 0ull;
         uint32_t *iters = which == 0 ? &sv->div_iters : &sv->den_iters;
-        const uint32_t it = first ? 0u : *iters + 1u;
+        const uint32_t it = done == kTolNext ? *iters + 1u : (uint32_t)done;
         *iters = it;
-        if (!first) {
+        if (done != 0) {
             if (which == 0) sv->total_div_iters += 1ull;
             else sv->total_den_iters += 1ull;
         }
@@ -1538,12 +1539,12 @@ void launch_integrate(cudaStream_t s, const Geo &g, const SimBufs &b, int div_sl
 #undef FCU_WIDE_AT
 #undef FCU_SWEEP_WIDE
 
-void launch_tol_finish(cudaStream_t s, const Geo &g, int which, int first, float tol,
+void launch_tol_finish(cudaStream_t s, const Geo &g, int which, int done, float tol,
                        uint32_t max_iters, cudaGraphConditionalHandle handle) {
     uint32_t threads = (g.nboxes + 31u) & ~31u;
     if (threads > 256u) threads = 256u;
     if (threads < 32u) threads = 32u;
-    k_tol_finish<<<1, threads, 0, s>>>(g, which, first, tol, max_iters, handle);
+    k_tol_finish<<<1, threads, 0, s>>>(g, which, done, tol, max_iters, handle);
 }
 void launch_stats(cudaStream_t s, const Geo &g, const SimBufs &b, uint32_t chunks) {
     if (!g.nboxes || !chunks) return;

@@ -126,9 +126,11 @@ void launch_den_kappa(cudaStream_t s, const Geo &g, const SimBufs &b, int slot, 
 void launch_integrate(cudaStream_t s, const Geo &g, const SimBufs &b, int div_slot, int den_slot,
                       int div_iters, int den_iters);
 // The tolerance loop's step after a prediction sweep: records each box's
-// residual of `which` (0 divergence, 1 density), counts the iteration,
+// residual of `which` (0 divergence, 1 density) and its iterations (`done` of
+// them before the substep's first call, one more each call with kTolNext),
 // keeps each box's loop going or stops it, and sets `handle` while any goes.
-void launch_tol_finish(cudaStream_t s, const Geo &g, int which, int first, float tol,
+constexpr int kTolNext = -1;
+void launch_tol_finish(cudaStream_t s, const Geo &g, int which, int done, float tol,
                        uint32_t max_iters, cudaGraphConditionalHandle handle);
 // reduce_stats of every box (chunks: blocks per box).
 void launch_stats(cudaStream_t s, const Geo &g, const SimBufs &b, uint32_t chunks);
