@@ -19,6 +19,7 @@
 //                    inclusive max-scan of the run ends gives starts, the
 //                    exclusive scan of the cell counts, without counting
 //
+// Up to 1.2M positions the build is grid_coop.cu's single launch instead.
 // A simulation's own grid (keys of cell and x slab, few particles a key) is
 // built by counting instead: k_count_keys, the scan, k_place, k_order.
 #include <algorithm>
@@ -774,6 +775,9 @@ cudaError_t grid_build_enqueue(cudaStream_t stream, const float4 *pos, uint32_t 
                                uint32_t *starts, uint32_t *perm, GridWork &w) {
     cudaError_t e;
     const uint32_t cells = w.cells;
+    e = cudaMemsetAsync(w.err, 0, 4 * kErrWords, stream);
+    if (e != cudaSuccess) return e;
+    if (coop_build_fits(w)) return coop_build_enqueue(stream, pos, g, keys, starts, perm, w);
     const SortRegion r = sort_region(w.scan_ctl, n, cells, w.passes);
     e = cudaMemsetAsync(w.scan_ctl, 0, w.scan_ctl_bytes, stream);
     if (e != cudaSuccess) return e;

@@ -43,11 +43,14 @@ inline int radix_passes(uint32_t cells) {
 }
 
 // Scratch of one grid build, carved from one device allocation.
+// Words from the error word on that a build clears: the error word and, at
+// kErrBarrier, the cooperative build's barrier counter.
+constexpr uint32_t kErrWords = 32, kErrBarrier = 16;
 struct GridWork {
     unsigned long long *scan_ctl;  // look-back words and digit counts, zeroed per build
     size_t scan_ctl_bytes;
     uint32_t *k1, *k2, *v1, *v2;   // ping-pong keys / values
-    uint32_t *err;                 // device error word (may alias the sim's)
+    uint32_t *err;                 // device error word, and room for kErrWords from it
     int passes;
     uint32_t cells, n;
 };
@@ -64,9 +67,17 @@ int32_t read_build_status(const uint32_t *err, cudaStream_t stream, const char *
 // publishes: its bounded look-back waits give up and set w.err.
 cudaError_t enqueue_stalled_radix_pass(const GridWork &w, cudaStream_t stream);
 
+// The build in one cooperative launch (grid_coop.cu), for as many positions
+// as one block per SM holds at once (1.2M positions).
+constexpr uint32_t kCoopBlocks = 148;
+bool coop_build_fits(const GridWork &w);
+cudaError_t coop_build_enqueue(cudaStream_t stream, const float4 *pos, const GridGeom &g, uint32_t *keys,
+                               uint32_t *starts, uint32_t *perm, const GridWork &w);
+
 // Enqueues keys -> stable radix sort -> starts on `stream`. `keys` receives
 // each input's cell key, `starts` the exclusive scan of the cell counts with
-// starts[cells] = n, `perm` the stable permutation.
+// starts[cells] = n, `perm` the stable permutation. Clears the error word
+// first.
 cudaError_t grid_build_enqueue(cudaStream_t stream, const float4 *pos, uint32_t n, const GridGeom &g, uint32_t *keys,
                                uint32_t *starts, uint32_t *perm, GridWork &w);
 

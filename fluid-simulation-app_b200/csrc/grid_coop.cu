@@ -1,0 +1,325 @@
+// grid_coop.cu — the neighbour grid of a small or middling input in one
+// cooperative launch.
+//
+// The digit passes of grid.cu are a launch each, with a look-back chain over
+// the tiles in every one: up to a million positions that is latency, not
+// work (98 us at 1M positions, 43 us at 20k). Here the whole build is one
+// kernel of at most a block per SM, each block owning a contiguous piece of
+// the input: keys, then per digit the piece ranked (its counts published), a
+// grid barrier, the piece's digit offsets from everybody's counts, the piece
+// written in digit order through shared memory, a barrier; finally the
+// starts, each block searching its share of the cells in the sorted keys. A
+// digit is as narrow as the keys allow in the same number of passes. The same
+// stable order and starts as the digit passes, whatever the distribution.
+//
+// Barriers are bounded like every wait of the grid: one that gives up sets
+// the build's error word, and the writes after it stay in bounds.
+//
+// Measured, us a build against the digit passes: 20k positions 23 / 46, 65k
+// 25 / 48, 262k 38 / 70, 1M 63 / 97 (in 7,000-position clusters 76 / 98, all
+// in one cell 75 / 89). At 1M a pass takes about 13 us, a third of it the two
+// barriers; past one piece a block the passes' tiles overlap better
+// (two tiles a block, 3M: 229 / 187).
+#include <algorithm>
+
+#include "grid.cuh"
+
+namespace fcu {
+
+namespace {
+
+constexpr int kThreads = 1024;
+constexpr int kWarps = kThreads / 32;
+constexpr int kItems = 8;
+constexpr uint32_t kTile = kThreads * kItems;  // the largest piece
+constexpr int kMinBits = 4, kMaxBits = 8;
+constexpr uint32_t kMaxDigits = 1u << kMaxBits;
+
+struct Coop {
+    const float4 *pos;
+    GridGeom g;
+    uint32_t n, cells, blocks, piece;  // piece: positions a block owns
+    int passes, bits;          // digit passes of `bits` bits each
+    uint2 *a, *b;              // (key, index) ping-pong
+    uint32_t *keys;            // the caller's keys, or null
+    uint32_t *starts, *perm;
+    uint32_t *counts;          // [block][digit]
+    uint32_t *barrier, *err;
+};
+
+struct CoopShared {
+    uint32_t hist[kWarps][kMaxDigits];
+    uint2 pair[kTile];
+    uint32_t off[kMaxDigits], start[kMaxDigits];  // output and staged index of a digit's first element
+    uint32_t part[4][kMaxDigits], before[4][kMaxDigits];
+    uint32_t sum[kWarps];
+    uint32_t lo, hi;
+};
+
+// Every block's `phase`-th arrival.
+__device__ void grid_barrier(const Coop &c, uint32_t phase) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(c.barrier, 1u);
+        const uint32_t want = phase * gridDim.x;
+        uint32_t v, spins = 0;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(c.barrier) : "memory");
+        } while (v < want && ++spins < kSpinLimit);
+        if (v < want) atomicOr(c.err, ERRF_SORT_TIMEOUT);
+        __threadfence();
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ uint2 ld_pair(const uint2 *p) { return __ldcg(p); }  // other blocks wrote it
+
+// The first index of the sorted keys k[0 .. n) not below `key`, by a whole
+// warp: 33 parts a round, so four rounds for a million keys.
+__device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t *k, uint32_t n, uint32_t key) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t lo = 0, len = n;  // the answer is in lo .. lo + len
+    while (len > 0) {
+        const uint32_t step = len / 33 + 1;
+        const uint64_t at = (uint64_t)lo + (uint64_t)step * (lane + 1) - 1;
+        const bool below = at < lo + len && __ldcg(&k[at]) < key;
+        const uint32_t c = (uint32_t)__popc(__ballot_sync(0xffffffffu, below));
+        const uint32_t hi = lo + len;
+        lo += c * step;
+        len = min(step - 1, hi - lo);
+    }
+    return lo;
+}
+
+// Exclusive scan over the digits of the first kMaxDigits threads' values, in
+// two halves around a __syncthreads.
+__device__ __forceinline__ uint32_t digit_scan_warp(CoopShared &s, uint32_t v) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= (uint32_t)o) x += y;
+    }
+    if (lane == 31) s.sum[warp] = x;
+    return x - v;
+}
+__device__ __forceinline__ uint32_t digit_scan_block(const CoopShared &s) {
+    uint32_t w = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kMaxDigits / 32; ++k)
+        if (k < threadIdx.x >> 5) w += s.sum[k];
+    return w;
+}
+
+template <int kBits>
+__global__ void __launch_bounds__(kThreads, 1) k_grid_coop(Coop c) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    CoopShared &s = *reinterpret_cast<CoopShared *>(s_raw);
+    constexpr uint32_t kDigits = 1u << kBits, kMask = kDigits - 1u;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t first = min(blockIdx.x * c.piece, c.n), len = min(c.piece, c.n - first);
+    // warp w holds a contiguous run of the piece, so that ranks taken round
+    // by round keep the input order
+    const int rounds = (int)((len + kThreads - 1) / kThreads);
+    const uint32_t run = warp * 32u * rounds;
+    uint32_t phase = 0;
+
+    for (uint32_t i = first + tid; i < first + len; i += kThreads) {
+        const float4 p = __ldg(&c.pos[i]);
+        const uint32_t cx = axis_cell(p.x, c.g.min[0], c.g.cell, c.g.dims[0]);
+        const uint32_t cy = axis_cell(p.y, c.g.min[1], c.g.cell, c.g.dims[1]);
+        const uint32_t cz = axis_cell(p.z, c.g.min[2], c.g.cell, c.g.dims[2]);
+        const uint32_t key = (cz * c.g.dims[1] + cy) * c.g.dims[0] + cx;
+        c.a[i] = make_uint2(key, i);  // read back by this block alone
+        if (c.keys) c.keys[i] = key;
+    }
+    __syncthreads();
+
+    const uint2 *in = c.a;
+    uint2 *out = c.b;
+    for (int pass = 0; pass < c.passes; ++pass) {
+        const bool last = pass == c.passes - 1;
+        const int shift = pass * kBits;
+        uint2 p[kItems];
+        uint32_t rank[kItems];
+#pragma unroll
+        for (int r = 0; r < kItems; ++r) {
+            const uint32_t q = run + r * 32 + lane;
+            p[r] = r < rounds && q < len ? ld_pair(&in[first + q]) : make_uint2(0u, 0u);
+        }
+        for (uint32_t d = lane; d < kMaxDigits; d += 32) s.hist[warp][d] = 0u;
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < kItems; ++r) {
+            if (r >= rounds) break;
+            const bool live = run + r * 32 + lane < len;
+            const uint32_t d = (p[r].x >> shift) & kMask;
+            uint32_t peers = __ballot_sync(0xffffffffu, live);
+#pragma unroll
+            for (int b = 0; b < kBits; ++b) {
+                const uint32_t bit = (d >> b) & 1u, bal = __ballot_sync(0xffffffffu, bit);
+                peers &= bit ? bal : ~bal;
+            }
+            uint32_t before = 0;
+            const uint32_t leader = live ? (uint32_t)__ffs(peers) - 1u : lane;
+            if (live && lane == leader) {
+                before = s.hist[warp][d];
+                s.hist[warp][d] = before + (uint32_t)__popc(peers);
+            }
+            rank[r] = __shfl_sync(0xffffffffu, before, leader) + __popc(peers & ((1u << lane) - 1u));
+            __syncwarp();
+        }
+        __syncthreads();
+        // the warps' exclusive counts of a digit, the piece's count of it for
+        // the other blocks, and the digits' staged starts
+        uint32_t mine = 0;
+        if (tid < kMaxDigits) {
+            uint32_t total = 0;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) {
+                const uint32_t v = s.hist[w][tid];
+                s.hist[w][tid] = total;
+                total += v;
+            }
+            if (tid < kDigits) c.counts[blockIdx.x * kDigits + tid] = total;
+            mine = digit_scan_warp(s, total);
+        }
+        __syncthreads();
+        if (tid < kMaxDigits) s.start[tid] = mine + digit_scan_block(s);
+        __syncthreads();
+        // staged while the barrier waits for the other blocks
+#pragma unroll
+        for (int r = 0; r < kItems; ++r) {
+            if (r >= rounds) break;
+            if (run + r * 32 + lane < len) {
+                const uint32_t d = (p[r].x >> shift) & kMask;
+                s.pair[s.start[d] + s.hist[warp][d] + rank[r]] = p[r];
+            }
+        }
+        grid_barrier(c, ++phase);
+
+        // offsets: the digit's elements in earlier pieces, and all smaller
+        // digits' elements; four groups of threads share the pieces
+        {
+            const uint32_t d = tid % kMaxDigits, q = tid / kMaxDigits;
+            uint32_t all = 0, pre = 0;
+            if (d < kDigits) {
+#pragma unroll 8
+                for (uint32_t b = q; b < gridDim.x; b += 4) {
+                    const uint32_t v = __ldcg(&c.counts[b * kDigits + d]);
+                    all += v;
+                    if (b < blockIdx.x) pre += v;
+                }
+            }
+            s.part[q][d] = all;
+            s.before[q][d] = pre;
+        }
+        __syncthreads();
+        if (tid < kMaxDigits)
+            mine = digit_scan_warp(s, s.part[0][tid] + s.part[1][tid] + s.part[2][tid] + s.part[3][tid]);
+        __syncthreads();
+        if (tid < kMaxDigits)
+            s.off[tid] = mine + digit_scan_block(s) + s.before[0][tid] + s.before[1][tid] + s.before[2][tid] +
+                         s.before[3][tid];
+        __syncthreads();
+        for (uint32_t j = tid; j < len; j += kThreads) {
+            const uint2 v = s.pair[j];
+            const uint32_t d = (v.x >> shift) & kMask;
+            const uint32_t dst = s.off[d] + (j - s.start[d]);
+            if (dst >= c.n) continue;  // only after a barrier that gave up
+            if (last) {
+                c.perm[dst] = v.y;
+                reinterpret_cast<uint32_t *>(out)[dst] = v.x;
+            } else {
+                out[dst] = v;
+            }
+        }
+        grid_barrier(c, ++phase);
+        uint2 *const was = const_cast<uint2 *>(in);
+        in = out;
+        out = was;
+    }
+
+    // starts: this block's share of the cells in the sorted keys
+    const uint32_t *sorted = reinterpret_cast<const uint32_t *>(in);
+    const uint32_t share = (c.cells + gridDim.x - 1) / gridDim.x;
+    const uint32_t c0 = min(blockIdx.x * share, c.cells), c1 = min(c0 + share, c.cells);
+    if (warp < 2) {
+        const uint32_t at = warp_lower_bound(sorted, c.n, warp ? c1 : c0);
+        if (lane == 0) (warp ? s.hi : s.lo) = at;
+    }
+    __syncthreads();
+    const uint32_t lo = s.lo, m = s.hi > lo ? s.hi - lo : 0u;
+    uint32_t *k = reinterpret_cast<uint32_t *>(s.pair);
+    const bool staged = m <= 2 * kTile;
+    if (staged)
+        for (uint32_t j = tid; j < m; j += kThreads) k[j] = __ldcg(&sorted[lo + j]);
+    __syncthreads();
+    for (uint32_t x = c0 + tid; x < c1; x += kThreads) {
+        uint32_t at = 0, top = m;
+        while (at < top) {
+            const uint32_t mid = (at + top) >> 1;
+            const uint32_t v = staged ? k[mid] : __ldcg(&sorted[lo + mid]);
+            if (v < x) at = mid + 1;
+            else top = mid;
+        }
+        c.starts[x] = lo + at;
+    }
+    if (blockIdx.x == 0 && tid == 0) c.starts[c.cells] = c.n;
+}
+
+// Passes, digit width and pieces: a block per SM where the positions or the
+// cells (their starts) are many.
+Coop shape_of(const GridWork &w) {
+    Coop c{};
+    c.n = w.n;
+    c.cells = w.cells;
+    int bits = 0;
+    while (bits < 32 && ((uint64_t)w.cells - 1) >> bits) ++bits;
+    c.passes = std::max(1, (bits + kMaxBits - 1) / kMaxBits);
+    c.bits = std::max(kMinBits, (bits + c.passes - 1) / c.passes);
+    c.blocks = std::min(kCoopBlocks, std::max(div_up(w.n, kThreads), div_up(w.cells, 4096u)));
+    c.piece = std::max((uint32_t)kThreads, div_up(div_up(w.n, c.blocks), 32) * 32);
+    return c;
+}
+
+template <int kBits>
+cudaError_t launch(cudaStream_t stream, Coop &c) {
+    if (c.bits != kBits) {
+        if constexpr (kBits > kMinBits) return launch<kBits - 1>(stream, c);
+    }
+    const cudaError_t e = cudaFuncSetAttribute(k_grid_coop<kBits>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sizeof(CoopShared));
+    if (e != cudaSuccess) return e;
+    void *args[] = {&c};
+    return cudaLaunchCooperativeKernel((const void *)k_grid_coop<kBits>, dim3(c.blocks), dim3(kThreads), args,
+                                       sizeof(CoopShared), stream);
+}
+
+}  // namespace
+
+bool coop_build_fits(const GridWork &w) {
+    if (w.n == 0 || w.n > kCoopBlocks * kTile) return false;
+    const Coop c = shape_of(w);
+    return 4ull * ((uint64_t)c.blocks << c.bits) <= w.scan_ctl_bytes;
+}
+
+cudaError_t coop_build_enqueue(cudaStream_t stream, const float4 *pos, const GridGeom &g, uint32_t *keys,
+                               uint32_t *starts, uint32_t *perm, const GridWork &w) {
+    Coop c = shape_of(w);
+    c.pos = pos;
+    c.g = g;
+    c.a = reinterpret_cast<uint2 *>(w.k1);       // k1, k2
+    c.b = reinterpret_cast<uint2 *>(w.v1);       // v1, v2
+    c.keys = keys == w.k2 ? nullptr : keys;      // k2: no buffer of the caller's
+    c.starts = starts;
+    c.perm = perm;
+    c.counts = reinterpret_cast<uint32_t *>(w.scan_ctl);
+    c.err = w.err;
+    c.barrier = w.err + kErrBarrier;
+    return launch<kMaxBits>(stream, c);
+}
+
+}  // namespace fcu

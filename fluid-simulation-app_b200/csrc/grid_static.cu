@@ -117,7 +117,6 @@ extern "C" int32_t fluid_grid_build_static(const float *pos4, uint32_t n, const 
     cudaStream_t st = (cudaStream_t)stream;
     GridWork w = grid_work_carve(static_cast<char *>(ws) + kErrBytes, n, (uint32_t)cells,
                                  static_cast<uint32_t *>(ws));
-    e = cudaMemsetAsync(w.err, 0, 4, st);
     // Without a caller buffer the keys live in k2: pass 0 reads them and
     // writes k1, and k2 is next written by pass 1, after they are consumed.
     GridGeom g;
@@ -126,8 +125,7 @@ extern "C" int32_t fluid_grid_build_static(const float *pos4, uint32_t n, const 
         g.dims[i] = grid->dims[i];
     }
     g.cell = grid->cell;
-    if (e == cudaSuccess)
-        e = grid_build_enqueue(st, (const float4 *)pos4, n, g, keys ? keys : w.k2, starts, perm, w);
+    e = grid_build_enqueue(st, (const float4 *)pos4, n, g, keys ? keys : w.k2, starts, perm, w);
     if (e != cudaSuccess)
         return report_error(FLUID_ERR_CUDA, std::string("fluid_grid_build_static: ") + cudaGetErrorString(e));
     return FLUID_OK;

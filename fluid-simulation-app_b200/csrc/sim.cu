@@ -1164,7 +1164,6 @@ int32_t fluid_grid_build(const float *pos4, uint32_t n, const FluidGrid *grid, u
     if (((uintptr_t)pos4 & 15u)) return fail(FLUID_ERR_ARG, "positions must be 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
     GridWork w = grid_work_carve(workspace, n, (uint32_t)cells, nullptr);
-    CK(cudaMemsetAsync(w.err, 0, 4, st));
     // Without a caller buffer the keys live in k2: pass 0 reads them and
     // writes k1, and k2 is next written by pass 1, after they are consumed.
     uint32_t *k = keys ? keys : w.k2;
