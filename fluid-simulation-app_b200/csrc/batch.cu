@@ -336,6 +336,7 @@ int32_t batch_create_into(FluidBatch *s, const FluidSimConfig *boxes, uint32_t n
     BK(s->alloc(&b.wpk, n));
     BK(s->alloc(&b.kd2, n));
     BK(s->alloc(&b.wpk2, n));
+    b.posm = b.wpk;
     BK(s->alloc(&b.aux, n));
     BK(s->alloc(&b.fvel, n));
     BK(s->alloc(&b.ftemp, n));

@@ -672,6 +672,7 @@ static int32_t create_into(FluidSim *s, const FluidSimConfig *cfg) {
     CK(s->alloc(&b.wpk, n));
     CK(s->alloc(&b.kd2, n));
     CK(s->alloc(&b.wpk2, n));
+    b.posm = b.wpk;
     CK(s->alloc(&b.aux, n));
     CK(s->alloc(&b.fvel, n));
     CK(s->alloc(&b.ftemp, n));

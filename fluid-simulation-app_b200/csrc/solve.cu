@@ -67,10 +67,10 @@ constexpr int kBatchKappaThreads = 768;
 #define FCU_MINB 0
 #endif
 // The forces sweep (plain and with the divergence prediction) of one box at
-// 6 blocks of 128 threads per SM (80 registers, no spills): 488 us on the 1M
-// workload against 500 at 7 (56 bytes spilled), 596 at 8 (128) and 523 at 5.
-// A batch likewise: 2.739 ms a substep of 64 boxes at 6, 2.850 at 7, 2.750
-// at 5. Scaled for other block sizes like density_div.
+// 6 blocks of 128 threads per SM (80 registers): 536 us at 43 neighbours of
+// the 1M workload against 573 at 7 and at 5 blocks. A batch likewise: 2.739
+// ms a substep of 64 boxes at 6, 2.850 at 7, 2.750 at 5. Scaled for other
+// block sizes like density_div.
 #ifndef FCU_MINB_FORCES
 #define FCU_MINB_FORCES 6
 #endif
@@ -89,11 +89,15 @@ __device__ __forceinline__ KernelConsts kernel_consts(const DevParams &P) {
     return KernelConsts{P.sigma, P.sigma_h, P.inv_h, P.support_sq};
 }
 
+// The pair terms form both branches of the kernel and select: a warp takes
+// both anyway, and its branches' bookkeeping cost more than the unused half
+// (density_div 709 -> 684 us, the forces 494 -> 475 at 43 neighbours).
 template <class KP>
 __device__ __forceinline__ float kernel_q(const KP &P, float q) {  // :176-182
-    if (q < 1.0f) return P.sigma * (1.0f - 1.5f * q * q * (1.0f - 0.5f * q));
+    const float near = P.sigma * (1.0f - 1.5f * q * q * (1.0f - 0.5f * q));
     const float t = 2.0f - q;
-    return P.sigma * 0.25f * t * t * t;
+    const float far = P.sigma * 0.25f * t * t * t;
+    return q < 1.0f ? near : far;
 }
 
 // grad_q (sim_solve.wgsl:184-196) returns (dw / r) * x; this is its scalar
@@ -101,22 +105,16 @@ __device__ __forceinline__ float kernel_q(const KP &P, float q) {  // :176-182
 // guard's zero vector: a signed zero added to any sum leaves it unchanged).
 template <class KP>
 __device__ __forceinline__ float grad_scale(const KP &P, float r, float q) {
-    if (r < 1e-9f) return 0.0f;
-    float dw;
-    if (q < 1.0f) {
-        dw = P.sigma_h * (-3.0f * q + 2.25f * q * q);
-    } else {
-        const float t = 2.0f - q;
-        dw = P.sigma_h * (-0.75f * t * t);
-    }
-    return dw / r;
+    const float t = 2.0f - q;
+    const float in = -3.0f * q + 2.25f * q * q, out = -0.75f * t * t;
+    const float gs = P.sigma_h * (q < 1.0f ? in : out) / r;
+    return r < 1e-9f ? 0.0f : gs;
 }
 
 __device__ __forceinline__ float cohesion(float r, float c, float k, float near) {  // :201-210
-    if (r >= c || r < 1e-9f) return 0.0f;
     const float a = (c - r) * (c - r) * (c - r) * r * r * r;
-    if (2.0f * r > c) return k * a;
-    return k * (2.0f * a - near);
+    const float v = k * (2.0f * r > c ? a : 2.0f * a - near);
+    return r >= c || r < 1e-9f ? 0.0f : v;
 }
 
 __device__ __forceinline__ float wall_density(float t) {  // :213-222
@@ -338,7 +336,7 @@ struct PosVel {
     float4 p, v;
 };
 struct Nbr3 {
-    float4 p, v, a;  // position, velocity, (density, near density, temperature, warm kd)
+    float4 p, v, a;  // (position, mass / density), velocity, (density, near density, temperature, warm kd)
 };
 
 // Particle counts stay below 2^28 (the host rejects more), so masking a list
@@ -597,6 +595,7 @@ __device__ __forceinline__ unsigned long long density_finish(const Geo &g, const
     // forces_eval can form forces_den_apply's sum in its own walk
     const float half = 0.5f * __ldg(&b.wpp[i]);
     b.aux[i] = make_float4(rho, d.rho_near, __ldg(&b.wtemp[i]), half / (rho * rho));
+    b.posm[i] = make_float4(pos.x, pos.y, pos.z, P.mass / rho);
     const float a = rho / fmaxf(dot(grad_sum, grad_sum) + grad_sq, 1e-4f);
     b.alpha[i] = a;
     drho += dot(vel, wg);
@@ -872,7 +871,10 @@ __device__ __forceinline__ F3 fingers(const FluidStep &st, F3 pos, F3 v) {
 // schedule runs this after each divergence apply, so the prediction that
 // only decides whether the loop stops costs no sweep of its own.
 // Measured on the 1M workload (37 neighbours): 488 us against 443 + 107 us
-// for the two kernels apart, the substep 1.953 -> 1.892 ms.
+// for the two kernels apart, the substep 1.953 -> 1.892 ms; 412 us with the
+// shared reciprocal, mass / density stored and branches selected. What is
+// left is bound by issue: about 250 instructions a pair, four divisions and a
+// square root among them.
 
 // What a pair needs of its particle and its box.
 struct ForceCtx {
@@ -880,6 +882,7 @@ struct ForceCtx {
     float mass, inv_h, rho0, soft, coh_c, coh_k, coh_near;
     F3 pos, vel;
     float rho, near, temp, kd;
+    bool plain;  // coordinate differences to any particle are 0 or in 2^-60 .. 2^61
 };
 struct ForceSums {
     F3 visc, blend, near, tension, push;
@@ -904,6 +907,10 @@ __device__ __forceinline__ ForceCtx force_ctx(const SimBufs &b, const DevParams 
     c.coh_k = 32.0f / (3.14159265f * c3 * c3 * c3);
     c.coh_near = c3 * c3 / 64.0f;
     c.pos = xyz(__ldg(&b.wpos[i]));
+    // (two floats at or above 2^-36 differ by a multiple of 2^-60, and one far
+    // below leaves the other's size)
+    const F3 ap = f3(fabsf(c.pos.x), fabsf(c.pos.y), fabsf(c.pos.z));
+    c.plain = fminf(fminf(ap.x, ap.y), ap.z) >= 0x1p-36f && fmaxf(fmaxf(ap.x, ap.y), ap.z) < 0x1p60f;
     c.vel = xyz(__ldg(&b.wvel[i]));
     const float4 a = __ldg(&b.aux[i]);
     c.rho = a.x;
@@ -913,6 +920,25 @@ __device__ __forceinline__ ForceCtx force_ctx(const SimBufs &b, const DevParams 
     return c;
 }
 
+// a / b rounded to nearest, given y = 1 / b rounded to nearest: two
+// corrections by the exact remainder. The first leaves the quotient within
+// one ulp, and from there a quotient corrected with a correctly rounded
+// reciprocal is the correctly rounded one (P. Markstein, Computation of
+// elementary functions on the IBM RISC System/6000 processor, 1990), as long
+// as no remainder underflows: |a| of 2^-100 or more, or 0.
+__device__ __forceinline__ float quotient(float a, float b, float y) {
+    float q = __fmul_rn(a, y);
+    q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+    return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+}
+
+// The near pressure's and the tension's six quotients by the distance share
+// one reciprocal: a pair's ten divisions were 39 % of the sweep (555 us on
+// the 1M workload without m / rho_j stored, 338 with every one left out),
+// these six 534 -> 496 us. Where a numerator might be too small for the
+// corrections (a particle within 2^-36 of a coordinate plane, whose
+// coordinate differences can be arbitrarily small; a vanishing cohesion) the
+// pair divides as written.
 template <bool kDiv>
 __device__ __forceinline__ ForceTerms force_pair(const ForceCtx &c, float gs, const Nbr3 &q) {
     constexpr float visc_k = 2.0f * DYNAMIC_VISCOSITY;
@@ -929,13 +955,23 @@ __device__ __forceinline__ ForceTerms force_pair(const ForceCtx &c, float gs, co
     const F3 dv = c.vel - xyz(q.v);
     t.drho = kDiv ? dot(dv, e) : 0.0f;
     const float wn = fmaxf(1.0f - r * c.inv_h, 0.0f);
-    t.near = ((c.near + q.a.y) * wn * wn) * (x / fmaxf(r, 1e-5f));
     t.visc = (visc_k * pair) * dv;
-    t.blend = (c.mass / rho_j * kernel_q(c.K, r * c.inv_h)) * dv;
+    t.blend = (q.p.w * kernel_q(c.K, r * c.inv_h)) * dv;
     t.heat_in = heat_k * pair * (c.temp - q.a.z);
     t.heat_out = diss_k * pair * dot(dv, dv);
     const float corr = 2.0f * c.rho0 / (c.rho + rho_j);
-    t.tension = ((corr * c.mass * cohesion(r, c.coh_c, c.coh_k, c.coh_near)) * x) / fmaxf(r, 1e-9f);
+    const float k = corr * c.mass * cohesion(r, c.coh_c, c.coh_k, c.coh_near);
+    const F3 kx = k * x;
+    F3 unit;
+    if (c.plain && r >= 1e-5f && (__float_as_uint(k) << 1) - (87u << 24) < (100u << 24)) {  // |k| in 2^-40 .. 2^60
+        const float y = __frcp_rn(r);
+        unit = f3(quotient(x.x, r, y), quotient(x.y, r, y), quotient(x.z, r, y));
+        t.tension = f3(quotient(kx.x, r, y), quotient(kx.y, r, y), quotient(kx.z, r, y));
+    } else {
+        unit = x / fmaxf(r, 1e-5f);
+        t.tension = kx / fmaxf(r, 1e-9f);
+    }
+    t.near = ((c.near + q.a.y) * wn * wn) * unit;
     t.push = (c.kd + q.a.w) * e;
     return t;
 }
@@ -1004,7 +1040,7 @@ __device__ __forceinline__ void forces_eval_body(const Geo &g, const SimBufs &b,
         ForceSums s{zero, zero, zero, zero, zero, 0.0f, 0.0f};
         auto load = [&](uint32_t code) {
             const uint32_t j = list_slot(code);
-            return Nbr3{__ldg(&b.wpos[j]), __ldg(&b.wvel[j]), __ldg(&b.aux[j])};
+            return Nbr3{__ldg(&b.posm[j]), __ldg(&b.wvel[j]), __ldg(&b.aux[j])};
         };
         walk<FCU_B_N3, Nbr3>(b.nbr, n, i, cnt, load, [&](float gs, const Nbr3 &q) {
             const ForceTerms t = force_pair<kDiv>(c, gs, q);

@@ -27,9 +27,11 @@ struct SimBufs {
     // writes the warm start's kd, also forms the divergence prediction
     float *kd2;
     float4 *wpk2;
-    // forces_eval's one record per neighbour beside position and velocity:
-    // density, near density, temperature and the warm start's kd
-    float4 *aux;
+    // forces_eval's records of a neighbour beside its velocity: position with
+    // mass / density, and density, near density, temperature and the warm
+    // start's kd. posm may share wpk's memory: the density solve's kappas,
+    // which go there, come after the forces.
+    float4 *posm, *aux;
     // velocity and temperature after the forces: forces_eval writes them
     // while other particles still read wvel / wtemp, and the density solve
     // and integrate go on from them

@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kWideThreads) k_forces_wide(Geo g, SimBufs b, 
     float heat = 0.0f;
     walk_wide<L, 18, Nbr3>(
         b.nbr, g.n, w, on ? __ldg(&b.nbr_n[w.i]) : 0u, rows,
-        [&](uint32_t j) { return Nbr3{__ldg(&b.wpos[j]), __ldg(&b.wvel[j]), __ldg(&b.aux[j])}; },
+        [&](uint32_t j) { return Nbr3{__ldg(&b.posm[j]), __ldg(&b.wvel[j]), __ldg(&b.aux[j])}; },
         [&](float gs, const Nbr3 &q, float *t) {
             const ForceTerms f = force_pair<kDiv>(c, gs, q);
             const F3 v[5] = {f.visc, -f.blend, f.near, -f.tension, f.push};
