@@ -753,10 +753,8 @@ __device__ __forceinline__ bool gated_out(const Geo &g, uint32_t bi, int gate) {
 // density_div's divergence sums again over the list, with this
 // iteration's velocities.
 __device__ __forceinline__ unsigned long long div_kappa_finish(const Geo &g, const SimBufs &b, const DevParams &P,
-                                                               uint32_t bi, uint32_t i, float sum) {
-    const float dt = g.st[bi].s.dt;
-    const F3 pos = xyz(__ldg(&b.wpos[i]));
-    const F3 vel = xyz(__ldg(&b.wvel[i]));
+                                                               uint32_t bi, uint32_t i, float dt, F3 pos,
+                                                               F3 vel, float sum) {
     float drho = P.mass * sum;
     drho += dot(vel, xyz(__ldg(&b.wgrad[i])));
     const float rho = __ldg(&b.density[i]);
@@ -787,9 +785,10 @@ __global__ void __launch_bounds__(TPB, kB ? kBatchKappaThreads / TPB : FCU_MINB_
     unsigned long long term = 0;
     if (live && !gated_out<kB>(g, bi, gate)) {
         const DevParams P = params_of<kB>(g, bi);
+        const float dt = g.st[bi].s.dt;
         const F3 pos = xyz(__ldg(&b.wpos[i]));
         const F3 vel = xyz(__ldg(&b.wvel[i]));
-        term = div_kappa_finish(g, b, P, bi, i, divergence_sum(b, n, i, pos, vel));
+        term = div_kappa_finish(g, b, P, bi, i, dt, pos, vel, divergence_sum(b, n, i, pos, vel));
     }
     add_term<kB>(&g.solve[bi].acc_div[slot], term);
 }
@@ -1079,11 +1078,9 @@ __global__ void __launch_bounds__(TPB, FCU_MINB_FORCES * 128 / TPB) k_forces_fus
 
 // ---- den_kappa (sim_solve.wgsl:674-698) ------------------------------------
 __device__ __forceinline__ unsigned long long den_kappa_finish(const Geo &g, const SimBufs &b, const DevParams &P,
-                                                               uint32_t bi, uint32_t i, float sum) {
+                                                               uint32_t bi, uint32_t i, float dt, F3 pos,
+                                                               F3 vel, float sum) {
     const float mass = P.mass, rho0 = P.rho0;
-    const float dt = g.st[bi].s.dt;
-    const F3 pos = xyz(__ldg(&b.wpos[i]));
-    const F3 vel = xyz(__ldg(&b.wvel[i]));
     const float rho = __ldg(&b.density[i]);
     const float drho = mass * sum + dot(vel, xyz(__ldg(&b.wgrad[i])));
     const float rho_star = rho + dt * drho;
@@ -1105,9 +1102,10 @@ __global__ void __launch_bounds__(TPB, kB ? kBatchKappaThreads / TPB : FCU_MINB_
     unsigned long long term = 0;
     if (live && !gated_out<kB>(g, bi, gate)) {
         const DevParams P = params_of<kB>(g, bi);
+        const float dt = g.st[bi].s.dt;
         const F3 pos = xyz(__ldg(&b.wpos[i]));
         const F3 vel = xyz(__ldg(&b.wvel[i]));
-        term = den_kappa_finish(g, b, P, bi, i, divergence_sum(b, n, i, pos, vel));
+        term = den_kappa_finish(g, b, P, bi, i, dt, pos, vel, divergence_sum(b, n, i, pos, vel));
     }
     add_term<kB>(&g.solve[bi].acc_den[slot], term);
 }

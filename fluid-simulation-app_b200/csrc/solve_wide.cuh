@@ -231,7 +231,8 @@ __global__ void __launch_bounds__(kWideThreads) k_div_kappa_wide(Geo g, SimBufs 
     const bool on = w.live && !gated_out<kB>(g, bi, gate);
     const float drho = divergence_wide<L>(b, g.n, w, on, s_rows[threadIdx.x >> 5]);
     unsigned long long term = 0;
-    if (on && w.lane == 0) term = div_kappa_finish(g, b, params_ref<kB>(g, bi), bi, w.i, drho);
+    if (on && w.lane == 0)
+        term = div_kappa_finish(g, b, params_ref<kB>(g, bi), bi, w.i, g.st[bi].s.dt, xyz(__ldg(&b.wpos[w.i])), xyz(__ldg(&b.wvel[w.i])), drho);
     add_term<kB>(&g.solve[bi].acc_div[slot], term);
 }
 
@@ -243,7 +244,8 @@ __global__ void __launch_bounds__(kWideThreads) k_den_kappa_wide(Geo g, SimBufs 
     const bool on = w.live && !gated_out<kB>(g, bi, gate);
     const float drho = divergence_wide<L>(b, g.n, w, on, s_rows[threadIdx.x >> 5]);
     unsigned long long term = 0;
-    if (on && w.lane == 0) term = den_kappa_finish(g, b, params_ref<kB>(g, bi), bi, w.i, drho);
+    if (on && w.lane == 0)
+        term = den_kappa_finish(g, b, params_ref<kB>(g, bi), bi, w.i, g.st[bi].s.dt, xyz(__ldg(&b.wpos[w.i])), xyz(__ldg(&b.wvel[w.i])), drho);
     add_term<kB>(&g.solve[bi].acc_den[slot], term);
 }
 
