@@ -9,19 +9,16 @@
 //   k_cell_keys      key = cell_of(pos), and every radix pass's digit
 //                    counts over all keys
 //   k_radix_pass     one stable 8-bit digit pass: warp ranking in input
-//                    order (digit peers from eight ballots), each tile's
-//                    digit offsets by decoupled look-back over the earlier
-//                    tiles, the tile staged in shared memory in digit order
-//                    and written out coalesced; the last pass also stores
-//                    the end of every run of equal keys at starts[key + 1]
-//   k_scan_lookback  single-pass scan (sum or max), decoupled look-back with
-//                    warp shuffles and ballots; every spin is bounded. The
-//                    inclusive max-scan of the run ends gives starts, the
-//                    exclusive scan of the cell counts, without counting
+//                    order (digit peers from eight ballots), the tile staged
+//                    in shared memory in digit order, its digit offsets by
+//                    decoupled look-back over the earlier tiles, written out
+//                    coalesced; every spin is bounded
+//   k_starts         starts from the sorted keys, tile of cells by tile
 //
 // Up to 1.2M positions the build is grid_coop.cu's single launch instead.
 // A simulation's own grid (keys of cell and x slab, few particles a key) is
-// built by counting instead: k_count_keys, the scan, k_place, k_order.
+// built by counting instead: k_count_keys, k_scan_lookback (a single-pass
+// exclusive scan, decoupled look-back with bounded spins), k_place, k_order.
 #include <algorithm>
 #include <string>
 
@@ -62,27 +59,13 @@ __device__ __forceinline__ uint32_t digit_peers(uint32_t act, uint32_t d) {
     return m;
 }
 
-// Adds the run of equal digits this lane starts (in adjacent lanes) to the
-// shared histogram h; positions in cell order give long runs. Every lane of
-// the warp calls it.
-__device__ __forceinline__ void count_digit_runs(uint32_t *h, bool live, uint32_t d) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t live_mask = __ballot_sync(0xffffffffu, live);
-    const uint32_t prev = __shfl_up_sync(0xffffffffu, d, 1);
-    const bool prev_live = lane > 0 && ((live_mask >> (lane - 1)) & 1u);
-    const bool head = live && (!prev_live || prev != d);
-    const uint32_t stops = __ballot_sync(0xffffffffu, head) | ~live_mask;
-    if (head) {
-        const uint32_t after = stops & ~((2u << lane) - 1u);  // stops above this lane
-        const uint32_t end = after ? (uint32_t)(__ffs(after) - 1) : 32u;
-        atomicAdd(&h[d], end - lane);
-    }
-}
-
 // Every pass's digit counts over all keys: a block's shared histograms,
-// then one global add per nonzero bin. Every lane of the block calls both.
-__device__ __forceinline__ void count_digits(uint32_t (*h)[kRadix], int passes, bool live, uint32_t key) {
-    for (int p = 0; p < passes; ++p) count_digit_runs(h[p], live, (key >> (p * kRadixBits)) & (kRadix - 1));
+// then one global add per nonzero bin. One shared add a key and digit: the
+// unit merges the adds of equal digits in a warp, so that finding runs of
+// them first only cost (the kernel 109 -> 68 us at 16.7M positions in
+// any order).
+__device__ __forceinline__ void count_digits(uint32_t (*h)[kRadix], int passes, uint32_t key) {
+    for (int p = 0; p < passes; ++p) atomicAdd(&h[p][(key >> (p * kRadixBits)) & (kRadix - 1)], 1u);
 }
 __device__ __forceinline__ void flush_digits(uint32_t (*h)[kRadix], int passes, uint32_t *digit_counts) {
     __syncthreads();
@@ -113,41 +96,30 @@ __global__ void __launch_bounds__(kSortThreads) k_cell_keys(const float4 *__rest
 #pragma unroll
         for (int u = 0; u < kKeyItems; ++u) {
             const uint64_t i = at + (uint64_t)u * kSortThreads + threadIdx.x;
-            const bool live = i < n;
-            uint32_t key = 0;
-            if (live) {
+            if (i < n) {
                 const uint32_t cx = axis_cell(p[u].x, g.min[0], g.cell, g.dims[0]);
                 const uint32_t cy = axis_cell(p[u].y, g.min[1], g.cell, g.dims[1]);
                 const uint32_t cz = axis_cell(p[u].z, g.min[2], g.cell, g.dims[2]);
-                key = (cz * g.dims[1] + cy) * g.dims[0] + cx;
+                const uint32_t key = (cz * g.dims[1] + cy) * g.dims[0] + cx;
                 keys[i] = key;
+                count_digits(h, passes, key);
             }
-            count_digits(h, passes, live, key);
         }
     }
     flush_digits(h, passes, digit_counts);
 }
 
-// Combine of the single-pass scan: sum, or max (kMax); 0 is the identity of
-// both on unsigned values.
-template <bool kMax>
-__device__ __forceinline__ uint32_t scan_op(uint32_t a, uint32_t b) {
-    return kMax ? max(a, b) : a + b;
-}
-template <bool kMax>
-__device__ __forceinline__ uint32_t warp_reduce(uint32_t v) {
+__device__ __forceinline__ uint32_t warp_sum(uint32_t v) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = scan_op<kMax>(v, __shfl_xor_sync(0xffffffffu, v, o));
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
-// Scan of in[0..n) into out[0..n), single pass: exclusive sums, or with
-// kMax inclusive maxima. Tiles are claimed in launch order through ctl[0];
+// Exclusive sums of in[0..n) into out[0..n), single pass. Tiles are claimed in launch order through ctl[0];
 // ctl[1 + t] is tile t's status word: flag in the high half (1 aggregate,
 // 2 inclusive prefix), value in the low half. With write_total, out[n]
 // receives the grand total. With zero_in, the input is cleared after it is
 // read.
-template <bool kMax>
 __global__ void __launch_bounds__(kScanThreads) k_scan_lookback(uint32_t *in, uint32_t *out,
                                                                 uint32_t n,
                                                                 unsigned long long *ctl,
@@ -182,14 +154,14 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_lookback(uint32_t *in, ui
     }
     uint32_t sum = 0;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) sum = scan_op<kMax>(sum, v[k]);
+    for (int k = 0; k < kScanItems; ++k) sum += v[k];
 
     // block-wide scan of the thread sums
     uint32_t x = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= (uint32_t)o) x = scan_op<kMax>(x, y);
+        if (lane >= (uint32_t)o) x += y;
     }
     uint32_t x_before = __shfl_up_sync(0xffffffffu, x, 1);
     if (lane == 0) x_before = 0u;
@@ -200,13 +172,13 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_lookback(uint32_t *in, ui
 #pragma unroll
         for (int o = 1; o < kScanThreads / 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= (uint32_t)o) w = scan_op<kMax>(w, y);
+            if (lane >= (uint32_t)o) w += y;
         }
         if (lane < kScanThreads / 32) s_warp[lane] = w;
     }
     __syncthreads();
     const uint32_t block_total = s_warp[kScanThreads / 32 - 1];
-    const uint32_t thread_excl = scan_op<kMax>(warp > 0 ? s_warp[warp - 1] : 0u, x_before);
+    const uint32_t thread_excl = (warp > 0 ? s_warp[warp - 1] : 0u) + x_before;
 
     // decoupled look-back, warp 0
     if (warp == 0) {
@@ -234,30 +206,25 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_lookback(uint32_t *in, ui
                 const uint32_t val = (uint32_t)st;
                 if (pmask) {
                     const int j = __ffs(pmask) - 1;
-                    exclusive = scan_op<kMax>(exclusive, warp_reduce<kMax>((int)lane <= j ? val : 0u));
+                    exclusive += warp_sum((int)lane <= j ? val : 0u);
                     break;
                 }
-                exclusive = scan_op<kMax>(exclusive, warp_reduce<kMax>(val));
+                exclusive += warp_sum(val);
                 pred -= 32;
             }
             if (lane == 0)
-                st_relaxed(&status[tile], kFlagPrefix | (unsigned long long)scan_op<kMax>(exclusive, block_total));
+                st_relaxed(&status[tile], kFlagPrefix | (unsigned long long)(exclusive + block_total));
         }
         if (lane == 0) s_excl = exclusive;
     }
     __syncthreads();
-    uint32_t run = scan_op<kMax>(s_excl, thread_excl);
+    uint32_t run = s_excl + thread_excl;
     if (vec) {
         uint32_t o[kScanItems];
 #pragma unroll
         for (int k = 0; k < kScanItems; ++k) {
-            if (kMax) {
-                run = max(run, v[k]);
-                o[k] = run;
-            } else {
-                o[k] = run;
-                run += v[k];
-            }
+            o[k] = run;
+            run += v[k];
         }
         uint4 *dst = reinterpret_cast<uint4 *>(out + base);
 #pragma unroll
@@ -271,16 +238,15 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_lookback(uint32_t *in, ui
     } else {
 #pragma unroll
         for (int k = 0; k < kScanItems; ++k) {
-            if (kMax) run = max(run, v[k]);
             if (base + k < n) {
                 out[base + k] = run;
                 if (zero_in) in[base + k] = 0u;
             }
-            if (!kMax) run += v[k];
+            run += v[k];
         }
     }
     if (write_total && threadIdx.x == 0 && (uint64_t)(tile + 1) * kScanTile >= n)
-        out[n] = scan_op<kMax>(s_excl, block_total);
+        out[n] = s_excl + block_total;
 }
 
 // One stable digit pass. Tiles are claimed in launch order through
@@ -295,15 +261,11 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_lookback(uint32_t *in, ui
 // number of smaller digits over all keys (digit_counts) plus its count in
 // earlier tiles. The tile is laid out in shared memory in (digit, input)
 // order and written out by consecutive threads to consecutive addresses.
-// `vals_in` null means the identity (the first pass); `keys_out` may be
-// null (the last pass). With `starts` (the last pass, keys now in final
-// order) every run of equal keys also stores its end at starts[key + 1]:
-// inside a tile's digit segment the next output element is the next staged
-// one, and the last element of a segment, whose successor another tile
-// writes, stores with atomicMax (the true end of its run is larger).
+// `vals_in` null means the identity (the first pass).
 static_assert(kRadix == kSortThreads, "one thread per digit");
-// Blocks per SM the pass kernel is compiled for: 4 (64 registers) measured
-// 0.75 ms at 16.7M positions against 0.84 at 3 and 1.01 at 1.
+// Blocks per SM the pass kernel is compiled for: 522 us a build of 16.7M
+// positions at 4 (64 registers), 598 at 5 (spills); tiles of 8,192 keys by
+// 512 threads 539, of 16,384 by 1,024 604, of 3,072 by 256 558.
 #ifndef FCU_SORT_MINB
 #define FCU_SORT_MINB 4
 #endif
@@ -314,15 +276,13 @@ static_assert(kRadix == kSortThreads, "one thread per digit");
 #define FCU_SORT_MATCH 0
 #endif
 // FCU_VAL_PREFETCH > 0: a digit pass asks L1 for the values of every
-// FCU_VAL_PREFETCH-th round of its tile while it ranks the keys. Measured:
-// grid_16m 0.683 -> 0.648 ms a build at 1 (0.676 at 4); the 1M workload's
-// grid 0.1153 -> 0.1147 ms.
+// FCU_VAL_PREFETCH-th round of its tile while it ranks the keys: 554 us a
+// build of 16.7M positions without, 522 at 1.
 #ifndef FCU_VAL_PREFETCH
 #define FCU_VAL_PREFETCH 1
 #endif
-// Earlier tiles' status words a digit's look-back loads at once. Measured:
-// the 1M workload's grid 0.1215 ms at 1, 0.1158 at 4, 0.1157 at 8 (16 bytes
-// spilled), 0.1203 at 16; grid_16m 0.70 / 0.68 / 0.69 / 0.74 ms a build.
+// Earlier tiles' status words a digit's look-back loads at once: 524 us a
+// build of 16.7M positions at 2, 519 at 4, 525 at 8 (spills).
 #ifndef FCU_LOOK_WINDOW
 #define FCU_LOOK_WINDOW 4
 #endif
@@ -331,8 +291,7 @@ constexpr int kLookWindow = FCU_LOOK_WINDOW;
 __global__ void __launch_bounds__(kSortThreads, FCU_SORT_MINB) k_radix_pass(
     const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in, uint32_t n, int shift,
     const uint32_t *__restrict__ digit_counts, unsigned long long *tile_status, uint32_t *tile_ctr,
-    uint32_t *err, uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out,
-    uint32_t *__restrict__ starts, uint32_t cells) {
+    uint32_t *err, uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out) {
     __shared__ uint32_t s_hist[kSortWarps][kRadix];
     __shared__ uint32_t s_off[kRadix];    // output index of this tile's first element of digit d
     __shared__ uint32_t s_start[kRadix];  // staged index of the tile's first element of digit d
@@ -445,6 +404,27 @@ __global__ void __launch_bounds__(kSortThreads, FCU_SORT_MINB) k_radix_pass(
         s_gsum[warp] = y;
     }
 
+    __syncthreads();
+    uint32_t wx = 0, wy = 0;
+    for (uint32_t w = 0; w < warp; ++w) {
+        wx += s_wsum[w];
+        wy += s_gsum[w];
+    }
+    s_start[dig] = wx + x - total;
+    __syncthreads();
+    // staged while the earlier tiles publish their counts (behind the
+    // look-back instead: 149 us a pass at 16.7M positions, 125 so)
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r) {
+        const uint32_t i = wbase + r * 32 + lane;
+        if (full || i < n) {
+            const uint32_t d = (key[r] >> shift) & (kRadix - 1);
+            const uint32_t at = s_start[d] + s_hist[warp][d] + rank[r];
+            s_key[at] = key[r];
+            s_val[at] = vals_in ? __ldg(&vals_in[i]) : i;
+        }
+    }
+
     // look-back over the earlier tiles' counts of this digit: the status
     // words of kLookWindow earlier tiles are loaded at once, then taken in
     // order (an entry read while unpublished is re-read until it is), adding
@@ -464,42 +444,24 @@ __global__ void __launch_bounds__(kSortThreads, FCU_SORT_MINB) k_radix_pass(
 #pragma unroll
             for (int u = 0; u < kLookWindow; ++u) {
                 if (done) continue;
-                unsigned long long x = v[u];
+                unsigned long long st = v[u];
                 uint32_t spins = 0;
-                while ((x >> 32) == 0) {
+                while ((st >> 32) == 0) {
                     if (++spins > kSpinLimit) {
                         atomicOr(err, ERRF_SCAN_TIMEOUT);
-                        x = kFlagPrefix;  // give up: count it as zero and stop
+                        st = kFlagPrefix;  // give up: count it as zero and stop
                         break;
                     }
-                    x = ld_relaxed(&tile_status[(uint64_t)(pred - u) * kRadix + dig]);
+                    st = ld_relaxed(&tile_status[(uint64_t)(pred - u) * kRadix + dig]);
                 }
-                excl += (uint32_t)x;
-                if ((x >> 32) == 2ull) done = true;
+                excl += (uint32_t)st;
+                if ((st >> 32) == 2ull) done = true;
             }
             pred -= kLookWindow;
         }
         st_relaxed(&mine[dig], kFlagPrefix | (unsigned long long)(excl + total));
     }
-    __syncthreads();
-    uint32_t wx = 0, wy = 0;
-    for (uint32_t w = 0; w < warp; ++w) {
-        wx += s_wsum[w];
-        wy += s_gsum[w];
-    }
-    s_start[dig] = wx + x - total;
     s_off[dig] = wy + y - gc + excl;
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < kSortItems; ++r) {
-        const uint32_t i = wbase + r * 32 + lane;
-        if (full || i < n) {
-            const uint32_t d = (key[r] >> shift) & (kRadix - 1);
-            const uint32_t at = s_start[d] + s_hist[warp][d] + rank[r];
-            s_key[at] = key[r];
-            s_val[at] = vals_in ? __ldg(&vals_in[i]) : i;
-        }
-    }
     __syncthreads();
     const uint32_t tbase = tile * kSortTile;
     const uint32_t count = full ? kSortTile : n - tbase;
@@ -511,15 +473,96 @@ __global__ void __launch_bounds__(kSortThreads, FCU_SORT_MINB) k_radix_pass(
         // look-back that gave up (garbage offsets) from writing out of bounds.
         if (dst < n) {
             vals_out[dst] = s_val[j];
-            if (keys_out) keys_out[dst] = k;
-            if (starts && k < cells) {
-                const uint32_t kn = j + 1 < count ? s_key[j + 1] : 0u;
-                const bool seg_end = j + 1 == count || ((kn >> shift) & (kRadix - 1)) != d;
-                if (seg_end) atomicMax(&starts[k + 1], dst + 1);
-                else if (kn != k) starts[k + 1] = dst + 1;
-            }
+            keys_out[dst] = k;
         }
     }
+}
+
+// The starts from the sorted keys. A block takes kStartTile cells, finds
+// their range of keys by two searches, marks the end of every run of equal
+// keys in shared memory and carries the marks over the empty cells by a
+// block-wide max scan, so nothing waits on another block. Where the range is
+// many keys for its cells (kStartStream), each cell's start is searched
+// instead, four cells of a thread side by side: all keys in one cell then
+// cost no more than the searches. The look-back max scan this replaces, over
+// run ends that the last digit pass scattered into cleared starts, took 65 us
+// at 2^24 cells, with its memset 80; this takes 45.
+constexpr int kStartThreads = 256, kStartSearch = 4, kStartMinBlocks = 6;
+constexpr uint32_t kStartStream = 65536;
+
+template <int kStartItems>
+__global__ void __launch_bounds__(kStartThreads, kStartMinBlocks)
+    k_starts(const uint32_t *__restrict__ sorted, uint32_t n, uint32_t cells, uint32_t *__restrict__ starts) {
+    constexpr uint32_t kStartTile = kStartThreads * kStartItems;
+    __shared__ uint32_t s_end[kStartTile + kStartThreads];
+    auto start_word = [](uint32_t x) { return x + x / kStartItems; };  // no bank conflicts
+    __shared__ uint32_t s_bound[2], s_warp[kStartThreads / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t c0 = blockIdx.x * kStartTile, count = min(kStartTile, cells - c0);
+    if (warp < 2) {
+        // (a bound past the last cell is above every key)
+        const uint32_t at = warp_lower_bound(sorted, n, warp ? c0 + count : c0);
+        if (lane == 0) s_bound[warp] = at;
+    }
+    for (uint32_t x = tid; x < kStartTile + kStartThreads; x += kStartThreads) s_end[x] = 0u;
+    __syncthreads();
+    const uint32_t lo = s_bound[0], hi = max(s_bound[1], lo);
+    if (blockIdx.x == gridDim.x - 1 && tid == 0) starts[cells] = n;
+    if (hi - lo > kStartStream) {
+        for (uint32_t x0 = tid; x0 < count; x0 += kStartSearch * kStartThreads) {
+            uint32_t at[kStartSearch];
+#pragma unroll
+            for (int u = 0; u < kStartSearch; ++u) at[u] = lo;
+            // the answer is in at .. at + len; the same len for all
+            for (uint32_t len = hi - lo; len > 0;) {
+                const uint32_t half = len >> 1;
+#pragma unroll
+                for (int u = 0; u < kStartSearch; ++u) {
+                    const bool below = __ldg(&sorted[at[u] + half]) < c0 + x0 + u * kStartThreads;
+                    at[u] = below ? at[u] + len - half : at[u];
+                }
+                len = half;
+            }
+#pragma unroll
+            for (int u = 0; u < kStartSearch; ++u)
+                if (x0 + u * kStartThreads < count) starts[c0 + x0 + u * kStartThreads] = at[u];
+        }
+        return;
+    }
+#pragma unroll 4
+    for (uint32_t j = lo + tid; j < hi; j += kStartThreads) {
+        const uint32_t k = __ldg(&sorted[j]);
+        const uint32_t kn = j + 1 < hi ? __ldg(&sorted[j + 1]) : ~k;
+        const uint32_t x = k - c0;
+        if (kn != k && x < count) s_end[start_word(x)] = j + 1;  // (x is below count unless a digit pass gave up)
+    }
+    __syncthreads();
+    uint32_t v[kStartItems];
+    uint32_t top = 0;
+#pragma unroll
+    for (int u = 0; u < kStartItems; ++u) {
+        v[u] = s_end[start_word(tid * kStartItems + u)];
+        top = max(top, v[u]);
+    }
+    uint32_t x = top;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= (uint32_t)o) x = max(x, y);
+    }
+    uint32_t run = __shfl_up_sync(0xffffffffu, x, 1);
+    if (lane == 0) run = 0u;
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    run = max(run, lo);
+    for (uint32_t w = 0; w < warp; ++w) run = max(run, s_warp[w]);
+#pragma unroll
+    for (int u = 0; u < kStartItems; ++u) {
+        s_end[start_word(tid * kStartItems + u)] = run;
+        run = max(run, v[u]);
+    }
+    __syncthreads();
+    for (uint32_t y = tid; y < count; y += kStartThreads) starts[c0 + y] = s_end[start_word(y)];
 }
 
 // ---- the counting build of the simulations ------------------------------------
@@ -663,15 +706,13 @@ size_t scan_region_bytes(uint32_t len) {
     return align256(8ull * (1ull + div_up(len, kScanTile)));
 }
 
-// The zeroed part of the workspace: the starts scan's look-back region,
-// every pass's tile counter and tile status words, every pass's digit
-// counts.
 __global__ void k_fill_u32(uint32_t *p, uint32_t n, uint32_t v) {
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) p[i] = v;
 }
 
+// The zeroed part of the workspace: every pass's tile counter and tile status
+// words, every pass's digit counts.
 struct SortRegion {
-    unsigned long long *fill_ctl;
     uint32_t *tile_ctr[kMaxPasses];
     unsigned long long *tile_status[kMaxPasses];
     uint32_t *digit_counts;
@@ -683,8 +724,7 @@ SortRegion sort_region(void *base, uint32_t n, uint32_t cells, int passes) {
     const uint32_t tiles = div_up(n > 0 ? n : 1, kSortTile);
     const uintptr_t b = reinterpret_cast<uintptr_t>(base);
     size_t off = 0;
-    r.fill_ctl = reinterpret_cast<unsigned long long *>(b + off);
-    off += scan_region_bytes(cells + 1);
+    off += scan_region_bytes(cells + 1);  // room for a cooperative build's piece counts
     for (int q = 0; q < passes; ++q) {
         r.tile_ctr[q] = reinterpret_cast<uint32_t *>(b + off);
         off += 256;
@@ -758,7 +798,7 @@ cudaError_t count_grid_enqueue(cudaStream_t stream, const float4 *pos, const Gri
     const uint32_t blocks = div_up(w.n, kCountThreads * kCountItems);
     if (boxes) k_count_keys<true><<<blocks, kCountThreads, 0, stream>>>(pos, g, *boxes, w, r);
     else k_count_keys<false><<<blocks, kCountThreads, 0, stream>>>(pos, g, BoxKeys{}, w, r);
-    k_scan_lookback<false><<<div_up(w.cells, kScanTile), kScanThreads, 0, stream>>>(w.count, w.starts, w.cells, w.ctl,
+    k_scan_lookback<<<div_up(w.cells, kScanTile), kScanThreads, 0, stream>>>(w.count, w.starts, w.cells, w.ctl,
                                                                                    w.err, 1, 1);
     k_place<<<div_up(w.n, kCountThreads), kCountThreads, 0, stream>>>(w);
     return cudaGetLastError();
@@ -781,29 +821,30 @@ cudaError_t grid_build_enqueue(cudaStream_t stream, const float4 *pos, uint32_t 
     const SortRegion r = sort_region(w.scan_ctl, n, cells, w.passes);
     e = cudaMemsetAsync(w.scan_ctl, 0, w.scan_ctl_bytes, stream);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(starts, 0, 4ull * cells + 4, stream);
-    if (e != cudaSuccess) return e;
+    const uint32_t *sorted = nullptr;
     if (n > 0) {
         const uint32_t blocks = std::min(div_up(n, kSortThreads * kKeyItems), kKeyBlocks);
         k_cell_keys<<<blocks, kSortThreads, 0, stream>>>(pos, n, g, keys, w.passes, r.digit_counts);
-    }
-    if (n > 0) {
         const uint32_t tiles = div_up(n, kSortTile);
         const uint32_t *kin = keys;
         const uint32_t *vin = nullptr;
         for (int pass = 0; pass < w.passes; ++pass) {
             const bool last = pass == w.passes - 1;
-            uint32_t *kout = last ? nullptr : ((pass & 1) ? w.k2 : w.k1);
+            uint32_t *kout = (pass & 1) ? w.k2 : w.k1;
             uint32_t *vout = last ? perm : ((pass & 1) ? w.v2 : w.v1);
             k_radix_pass<<<tiles, kSortThreads, 0, stream>>>(
                 kin, vin, n, pass * kRadixBits, r.digit_counts + pass * kRadix, r.tile_status[pass],
-                r.tile_ctr[pass], w.err, kout, vout, last ? starts : nullptr, cells);
+                r.tile_ctr[pass], w.err, kout, vout);
             kin = kout;
             vin = vout;
         }
+        sorted = kin;
     }
-    k_scan_lookback<true><<<div_up(cells + 1ull, kScanTile), kScanThreads, 0, stream>>>(starts, starts, cells + 1,
-                                                                                        r.fill_ctl, w.err, 0, 0);
+    // small tiles until the large ones fill the GPU
+    if (cells < 148u * kStartMinBlocks * 16u * kStartThreads)
+        k_starts<4><<<div_up(cells, 4 * kStartThreads), kStartThreads, 0, stream>>>(sorted, n, cells, starts);
+    else
+        k_starts<16><<<div_up(cells, 16 * kStartThreads), kStartThreads, 0, stream>>>(sorted, n, cells, starts);
     return cudaGetLastError();
 }
 
@@ -840,7 +881,7 @@ cudaError_t enqueue_stalled_radix_pass(const GridWork &w, cudaStream_t st) {
     // the tile counter starts at 1, so the one block claims tile 1
     k_fill_u32<<<1, 32, 0, st>>>(r.tile_ctr[0], 1, 1u);
     k_radix_pass<<<1, kSortThreads, 0, st>>>(w.k2, nullptr, w.n, 0, r.digit_counts, r.tile_status[0],
-                                             r.tile_ctr[0], w.err, w.k1, w.v1, nullptr, 1u);
+                                             r.tile_ctr[0], w.err, w.k1, w.v1);
     return cudaGetLastError();
 }
 
@@ -930,7 +971,7 @@ extern "C" int32_t fluid_selftest_scan_wait(int32_t device, float *ms) {
         if ((e = cudaEventCreate(&ev[0])) != cudaSuccess) break;
         if ((e = cudaEventCreate(&ev[1])) != cudaSuccess) break;
         cudaEventRecord(ev[0]);
-        k_scan_lookback<false><<<1, kScanThreads>>>(in, out, n, ctl, err, 0, 0);
+        k_scan_lookback<<<1, kScanThreads>>>(in, out, n, ctl, err, 0, 0);
         cudaEventRecord(ev[1]);
         if ((e = cudaEventSynchronize(ev[1])) != cudaSuccess) break;
         if ((e = cudaGetLastError()) != cudaSuccess) break;

@@ -42,12 +42,29 @@ inline int radix_passes(uint32_t cells) {
     return p < 1 ? 1 : p;
 }
 
+// The first index of the sorted keys k[0 .. n) not below `key`, by a whole
+// warp: 33 parts a round, so four rounds for a million keys.
+__device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t *k, uint32_t n, uint32_t key) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t lo = 0, len = n;  // the answer is in lo .. lo + len
+    while (len > 0) {
+        const uint32_t step = len / 33 + 1;
+        const uint64_t at = (uint64_t)lo + (uint64_t)step * (lane + 1) - 1;
+        const bool below = at < lo + len && __ldcg(&k[at]) < key;
+        const uint32_t c = (uint32_t)__popc(__ballot_sync(0xffffffffu, below));
+        const uint32_t hi = lo + len;
+        lo += c * step;
+        len = min(step - 1, hi - lo);
+    }
+    return lo;
+}
+
 // Scratch of one grid build, carved from one device allocation.
 // Words from the error word on that a build clears: the error word and, at
 // kErrBarrier, the cooperative build's barrier counter.
 constexpr uint32_t kErrWords = 32, kErrBarrier = 16;
 struct GridWork {
-    unsigned long long *scan_ctl;  // look-back words and digit counts, zeroed per build
+    unsigned long long *scan_ctl;  // look-back words and digit counts, zeroed per build (or a cooperative build's piece counts)
     size_t scan_ctl_bytes;
     uint32_t *k1, *k2, *v1, *v2;   // ping-pong keys / values
     uint32_t *err;                 // device error word, and room for kErrWords from it

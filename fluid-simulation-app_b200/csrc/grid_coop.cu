@@ -75,23 +75,6 @@ __device__ void grid_barrier(const Coop &c, uint32_t phase) {
 
 __device__ __forceinline__ uint2 ld_pair(const uint2 *p) { return __ldcg(p); }  // other blocks wrote it
 
-// The first index of the sorted keys k[0 .. n) not below `key`, by a whole
-// warp: 33 parts a round, so four rounds for a million keys.
-__device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t *k, uint32_t n, uint32_t key) {
-    const uint32_t lane = threadIdx.x & 31;
-    uint32_t lo = 0, len = n;  // the answer is in lo .. lo + len
-    while (len > 0) {
-        const uint32_t step = len / 33 + 1;
-        const uint64_t at = (uint64_t)lo + (uint64_t)step * (lane + 1) - 1;
-        const bool below = at < lo + len && __ldcg(&k[at]) < key;
-        const uint32_t c = (uint32_t)__popc(__ballot_sync(0xffffffffu, below));
-        const uint32_t hi = lo + len;
-        lo += c * step;
-        len = min(step - 1, hi - lo);
-    }
-    return lo;
-}
-
 // Exclusive scan over the digits of the first kMaxDigits threads' values, in
 // two halves around a __syncthreads.
 __device__ __forceinline__ uint32_t digit_scan_warp(CoopShared &s, uint32_t v) {
