@@ -19,7 +19,8 @@
 // 25 / 48, 262k 38 / 70, 1M 63 / 97 (in 7,000-position clusters 76 / 98, all
 // in one cell 75 / 89). At 1M a pass takes about 13 us, a third of it the two
 // barriers; past one piece a block the passes' tiles overlap better
-// (two tiles a block, 3M: 229 / 187).
+// (two tiles a block, 3M: 229 / 187). The digit passes are as they were then;
+// since, 1.3M positions take 89 there instead of 102.
 #include <algorithm>
 
 #include "grid.cuh"
