@@ -287,6 +287,12 @@ cudaError_t launch(cudaStream_t stream, Coop &c) {
 bool coop_build_fits(const GridWork &w) {
     if (w.n == 0 || w.n > kCoopBlocks * kTile) return false;
     const Coop c = shape_of(w);
+    // every block resident at once: a device with fewer SMs to give (a slice
+    // of one) builds by digit passes
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || (uint32_t)sms < c.blocks)
+        return false;
     return 4ull * ((uint64_t)c.blocks << c.bits) <= w.scan_ctl_bytes;
 }
 
