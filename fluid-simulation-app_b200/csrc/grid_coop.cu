@@ -23,6 +23,7 @@
 // since, 1.3M positions take 89 there instead of 102.
 #include <algorithm>
 
+#include "cell_range.h"
 #include "grid.cuh"
 
 namespace fcu {
@@ -228,10 +229,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_grid_coop(Coop c) {
 
     // starts: this block's share of the cells in the sorted keys
     const uint32_t *sorted = reinterpret_cast<const uint32_t *>(in);
-    const uint32_t share = (c.cells + gridDim.x - 1) / gridDim.x;
-    const uint32_t c0 = min(blockIdx.x * share, c.cells), c1 = min(c0 + share, c.cells);
+    const CellRange r = cell_range(c.cells, gridDim.x, blockIdx.x);
     if (warp < 2) {
-        const uint32_t at = warp_lower_bound(sorted, c.n, warp ? c1 : c0);
+        const uint32_t at = warp_lower_bound(sorted, c.n, warp ? r.first + r.count : r.first);
         if (lane == 0) (warp ? s.hi : s.lo) = at;
     }
     __syncthreads();
@@ -241,15 +241,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_grid_coop(Coop c) {
     if (staged)
         for (uint32_t j = tid; j < m; j += kThreads) k[j] = __ldcg(&sorted[lo + j]);
     __syncthreads();
-    for (uint32_t x = c0 + tid; x < c1; x += kThreads) {
+    for (uint32_t x = tid; x < r.count; x += kThreads) {
+        const uint32_t cell = r.first + x;
         uint32_t at = 0, top = m;
         while (at < top) {
             const uint32_t mid = (at + top) >> 1;
             const uint32_t v = staged ? k[mid] : __ldcg(&sorted[lo + mid]);
-            if (v < x) at = mid + 1;
+            if (v < cell) at = mid + 1;
             else top = mid;
         }
-        c.starts[x] = lo + at;
+        c.starts[cell] = lo + at;
     }
     if (blockIdx.x == 0 && tid == 0) c.starts[c.cells] = c.n;
 }
