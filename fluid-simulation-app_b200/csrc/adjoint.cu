@@ -1607,6 +1607,7 @@ struct AdjBase {
     virtual int32_t forward(const double *forces, double xsph, const double target[3], double *loss) = 0;
     virtual int32_t backward(double *grad_forces, double *grad_xsph) = 0;
     virtual int32_t final_state(double *pos3, double *vel3) = 0;
+    virtual int32_t stall_grid() = 0;
     uint32_t n = 0, frames = 0, spf = 0, ce = 1;
     std::vector<uint32_t> div_it, den_it;
     bool frozen = false, have_forward = false;
@@ -1645,7 +1646,10 @@ struct AdjImpl : AdjBase {
     // grid
     CountGrid gw{};
     float4 *pos4 = nullptr;
-    uint32_t *keys = nullptr, *starts = nullptr, *perm = nullptr, *over = nullptr;
+    uint32_t *keys = nullptr, *starts = nullptr, *perm = nullptr;
+    // particles past kModelCap, and beside it the grid's error word, which
+    // stays set until a call has reported it
+    uint32_t *over = nullptr;
     // state and its checkpoints
     V3<T> *x = nullptr, *v = nullptr;
     T *pp = nullptr;
@@ -1740,10 +1744,8 @@ struct AdjImpl : AdjBase {
         arena.want(&keys, N);
         arena.want(&starts, (size_t)cells + 1);
         arena.want(&perm, N);
-        arena.want(&over, 1);
+        arena.want(&over, 2);
         char *grid_ws = nullptr;
-        uint32_t *grid_err = nullptr;
-        arena.want(&grid_err, 1);
         arena.want(&grid_ws, count_grid_bytes(n, cells));
         arena.want(&x_init, N);
         arena.want(&id_init, N);
@@ -1800,8 +1802,8 @@ struct AdjImpl : AdjBase {
         arena.want(&cbar, 1);
         AK(arena.commit());
         AK(cudaMemset(grid_ws, 0, count_grid_bytes(n, cells)));
-        AK(cudaMemset(grid_err, 0, 4));
-        gw = count_grid_carve(grid_ws, n, cells, keys, starts, perm, grid_err);
+        AK(cudaMemset(over, 0, 8));
+        gw = count_grid_carve(grid_ws, n, cells, keys, starts, perm, over + 1);
         // the initial state, which every forward starts from
         std::vector<V3<T>> xs(n);
         std::vector<uint32_t> ids(n);
@@ -1956,11 +1958,18 @@ struct AdjImpl : AdjBase {
         return V3<T>{T(forces[3 * fr]), T(forces[3 * fr + 1]), T(forces[3 * fr + 2])};
     }
 
-    int32_t check_overflow() {
-        uint32_t o = 0;
-        AK(cudaMemcpyAsync(&o, over, 4, cudaMemcpyDeviceToHost, stream));
+    // What the kernels could not do: a grid whose bounded wait gave up (its
+    // permutation, and so everything after it, is invalid), a particle past
+    // the model's cap.
+    int32_t check_flags() {
+        uint32_t f[2] = {0, 0};
+        AK(cudaMemcpyAsync(f, over, 8, cudaMemcpyDeviceToHost, stream));
         AK(cudaStreamSynchronize(stream));
-        if (o) return report_error(FLUID_ERR_STATE, "adjoint: a particle has more than 128 neighbours");
+        if (f[1]) {
+            AK(cudaMemsetAsync(gw.err, 0, 4, stream));
+            return report_error(FLUID_ERR_TIMEOUT, "adjoint: a bounded wait of the neighbour grid gave up");
+        }
+        if (f[0]) return report_error(FLUID_ERR_STATE, "adjoint: a particle has more than 128 neighbours");
         return FLUID_OK;
     }
 
@@ -2004,7 +2013,7 @@ struct AdjImpl : AdjBase {
         AK(cudaEventElapsedTime(&last_forward_ms, e0, e1));
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        rc = check_overflow();
+        rc = check_flags();
         if (rc != FLUID_OK) return rc;
         double l = 0.0;
         for (int a = 0; a < 3; ++a) {
@@ -2133,8 +2142,9 @@ struct AdjImpl : AdjBase {
         AK(cudaEventElapsedTime(&last_backward_ms, e0, e1));
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        // the state is back at the last segment's end: restore the final state
-        // by re-running nothing; the final positions are still in the loss pass
+        have_forward = false;  // the state was overwritten by the recomputation
+        rc = check_flags();
+        if (rc != FLUID_OK) return rc;
         if (grad_forces) {
             for (uint32_t fr = 0; fr < frames; ++fr)
                 for (int a = 0; a < 3; ++a) {
@@ -2144,7 +2154,12 @@ struct AdjImpl : AdjBase {
                 }
         }
         if (grad_xsph) *grad_xsph = cb;
-        have_forward = false;  // the state was overwritten by the recomputation
+        return FLUID_OK;
+    }
+
+    int32_t stall_grid() override {
+        AK(cudaSetDevice(device));
+        AK(enqueue_stalled_scan(gw, stream));
         return FLUID_OK;
     }
 
@@ -2260,6 +2275,11 @@ int32_t fluid_adjoint_set_schedule(FluidAdjoint *a, const uint32_t *div_iters, c
 int32_t fluid_adjoint_final_state(FluidAdjoint *a, double *pos3, double *vel3) {
     if (!a) return report_error(FLUID_ERR_ARG, "adjoint: null handle");
     return a->impl->final_state(pos3, vel3);
+}
+
+int32_t fluid_selftest_adjoint_wait(FluidAdjoint *a) {
+    if (!a) return report_error(FLUID_ERR_ARG, "adjoint: null handle");
+    return a->impl->stall_grid();
 }
 
 int32_t fluid_adjoint_timing(const FluidAdjoint *a, float *forward_ms, float *backward_ms) {

@@ -804,6 +804,15 @@ cudaError_t count_grid_enqueue(cudaStream_t stream, const float4 *pos, const Gri
     return cudaGetLastError();
 }
 
+cudaError_t enqueue_stalled_scan(const CountGrid &w, cudaStream_t st) {
+    // the tile counter starts at 1, so the one block claims tile 1 (of no
+    // cells where there is one tile; the look-back words have room for it)
+    k_fill_u32<<<1, 32, 0, st>>>(reinterpret_cast<uint32_t *>(w.ctl), 1, 1u);
+    k_scan_lookback<<<1, kScanThreads, 0, st>>>(w.count, w.starts, w.cells, w.ctl, w.err, 0, 1);
+    const cudaError_t e = cudaMemsetAsync(w.ctl, 0, 8 * 3, st);
+    return e == cudaSuccess ? cudaGetLastError() : e;
+}
+
 cudaError_t count_grid_order(cudaStream_t stream, const CountGrid &w, const GridGather *gather) {
     const uint32_t blocks = div_up(w.n, kCountThreads);
     if (gather) k_order<true><<<blocks, kCountThreads, 0, stream>>>(w, *gather);

@@ -150,6 +150,11 @@ struct GridGather {
 // run; with `boxes` the keys are the batch's (`g` unused). n > 0.
 cudaError_t count_grid_enqueue(cudaStream_t stream, const float4 *pos, const GridGeom &g, const BoxKeys *boxes,
                                const CountGrid &w, const StepRing &r);
+// Enqueues one block of the scan that claims tile 1 while tile 0 never
+// publishes: its bounded look-back gives up and sets w.err. The starts are
+// invalid afterwards; counts and look-back words are left zero, as a build
+// leaves them.
+cudaError_t enqueue_stalled_scan(const CountGrid &w, cudaStream_t stream);
 // Then the stable permutation and, with `gather`, the records in its order.
 cudaError_t count_grid_order(cudaStream_t stream, const CountGrid &w, const GridGather *gather);
 

@@ -413,7 +413,9 @@ FluidAdjoint *fluid_adjoint_create(const FluidSimConfig *cfg, uint32_t frames,
 void fluid_adjoint_destroy(FluidAdjoint *adj);
 uint32_t fluid_adjoint_count(const FluidAdjoint *adj);
 /* forces[frames][3], the XSPH coefficient, target[3]; writes the loss.
- * Synchronises. */
+ * Synchronises. FLUID_ERR_STATE when a particle has more than 128
+ * neighbours; FLUID_ERR_TIMEOUT, here and from the backward, when a bounded
+ * wait of the neighbour grid gave up. */
 int32_t fluid_adjoint_forward(FluidAdjoint *adj, const double *forces, double xsph,
                               const double target[3], double *loss);
 /* Gradients of the last forward's loss: grad_forces[frames][3], grad_xsph
@@ -511,6 +513,11 @@ int32_t fluid_selftest_radix_wait(int32_t device, float *ms);
  * fluid_grid_build_static_status: FLUID_ERR_TIMEOUT, as it should.
  * Allocates nothing. */
 int32_t fluid_selftest_static_radix_wait(int32_t device, float *ms);
+
+/* The stalled scan on an adjoint handle's own grid buffers, enqueued on its
+ * stream: the handle's next forward or backward returns FLUID_ERR_TIMEOUT,
+ * and the one after that works again. FLUID_OK when enqueued. */
+int32_t fluid_selftest_adjoint_wait(FluidAdjoint *adjoint);
 
 #ifdef __cplusplus
 }
