@@ -528,7 +528,9 @@ __global__ void __launch_bounds__(kWideThreads) k_m_density(MP<T> p, uint32_t n,
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const V3<T> xij = xi - xj[u];
-                const bool is = j[u] != i && dot(xij, xij) < p.sup2;
+                // (not `<`: a distance that is no number counts, so that a
+                // state that is none goes past kModelCap and is reported)
+                const bool is = j[u] != i && !(dot(xij, xij) >= p.sup2);
                 const uint32_t hits = __ballot_sync(0xffffffffu, is);
                 if (is) hit[staged + __popc(hits & before)] = j[u];
                 staged += __popc(hits & mine);

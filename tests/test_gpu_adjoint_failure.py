@@ -34,3 +34,16 @@ def test_a_grid_wait_that_gives_up_is_reported(fcu, wl, precision):
         assert a.forward(*CONTROLS) == loss
     g2, gx2 = a.backward()
     assert np.array_equal(g2.view(np.uint64), grad.view(np.uint64)) and gx2 == gx
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("precision", [32, 64])
+def test_a_state_that_is_no_number_is_refused(fcu, wl, precision, bad):
+    # positions that are NaN all stand in one cell, each a neighbour of every
+    # other: past the model's cap of 128
+    a = small(fcu, wl, precision)
+    forces, xsph, target = CONTROLS
+    with pytest.raises(fcu.FluidError) as e:
+        a.forward([forces[0], [0.0, bad, 0.0]], xsph, target)
+    assert e.value.code == fcu.ERR_STATE and "128 neighbours" in str(e.value)
+    assert np.isfinite(a.forward(*CONTROLS))
