@@ -826,7 +826,10 @@ cudaError_t grid_build_enqueue(cudaStream_t stream, const float4 *pos, uint32_t 
     const uint32_t cells = w.cells;
     e = cudaMemsetAsync(w.err, 0, 4 * kErrWords, stream);
     if (e != cudaSuccess) return e;
-    if (coop_build_fits(w)) return coop_build_enqueue(stream, pos, g, keys, starts, perm, w);
+    if (coop_build_fits(w, stream)) {
+        e = coop_build_enqueue(stream, pos, g, keys, starts, perm, w);
+        if (e != cudaErrorCooperativeLaunchTooLarge) return e;
+    }
     const SortRegion r = sort_region(w.scan_ctl, n, cells, w.passes);
     e = cudaMemsetAsync(w.scan_ctl, 0, w.scan_ctl_bytes, stream);
     if (e != cudaSuccess) return e;

@@ -85,9 +85,12 @@ int32_t read_build_status(const uint32_t *err, cudaStream_t stream, const char *
 cudaError_t enqueue_stalled_radix_pass(const GridWork &w, cudaStream_t stream);
 
 // The build in one cooperative launch (grid_coop.cu), for as many positions
-// as one block per SM holds at once (1.2M positions).
+// as one block per SM holds at once (1.2M positions) on the SMs that the
+// stream may use.
 constexpr uint32_t kCoopBlocks = 148;
-bool coop_build_fits(const GridWork &w);
+bool coop_build_fits(const GridWork &w, cudaStream_t stream);
+// cudaErrorCooperativeLaunchTooLarge, with nothing enqueued and no error left
+// behind, where the driver would not hold every block at once after all.
 cudaError_t coop_build_enqueue(cudaStream_t stream, const float4 *pos, const GridGeom &g, uint32_t *keys,
                                uint32_t *starts, uint32_t *perm, const GridWork &w);
 

@@ -21,6 +21,9 @@
 // barriers; past one piece a block the passes' tiles overlap better
 // (two tiles a block, 3M: 229 / 187). The digit passes are as they were then;
 // since, 1.3M positions take 89 there instead of 102.
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
 #include <algorithm>
 
 #include "cell_range.h"
@@ -279,21 +282,58 @@ cudaError_t launch(cudaStream_t stream, Coop &c) {
                                                (int)sizeof(CoopShared));
     if (e != cudaSuccess) return e;
     void *args[] = {&c};
-    return cudaLaunchCooperativeKernel((const void *)k_grid_coop<kBits>, dim3(c.blocks), dim3(kThreads), args,
-                                       sizeof(CoopShared), stream);
+    const cudaError_t l = cudaLaunchCooperativeKernel((const void *)k_grid_coop<kBits>, dim3(c.blocks), dim3(kThreads),
+                                                      args, sizeof(CoopShared), stream);
+    if (l == cudaErrorCooperativeLaunchTooLarge) (void)cudaGetLastError();  // the caller goes another way
+    return l;
+}
+
+// Driver entry points, null where the driver has none.
+struct GreenCalls {
+    PFN_cuStreamGetGreenCtx ctx_of = nullptr;
+    PFN_cuGreenCtxGetDevResource resource = nullptr;
+};
+const GreenCalls &green_calls() {
+    static const GreenCalls calls = [] {
+        GreenCalls c;
+        void *p[2] = {nullptr, nullptr};
+        const char *const name[2] = {"cuStreamGetGreenCtx", "cuGreenCtxGetDevResource"};
+        for (int k = 0; k < 2; ++k) {
+            cudaDriverEntryPointQueryResult found;
+            if (cudaGetDriverEntryPointByVersion(name[k], &p[k], 12040, cudaEnableDefault, &found) != cudaSuccess ||
+                found != cudaDriverEntryPointSuccess)
+                return c;
+        }
+        c.ctx_of = reinterpret_cast<PFN_cuStreamGetGreenCtx>(p[0]);
+        c.resource = reinterpret_cast<PFN_cuGreenCtxGetDevResource>(p[1]);
+        return c;
+    }();
+    return calls;
+}
+
+// SMs the stream's kernels may run on: its green context's, or the device's.
+uint32_t sms_of(cudaStream_t stream) {
+    const GreenCalls &calls = green_calls();
+    CUgreenCtx green = nullptr;
+    if (calls.ctx_of && calls.ctx_of(stream, &green) == CUDA_SUCCESS && green) {
+        CUdevResource r{};
+        return calls.resource(green, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS ? r.sm.smCount : 0u;
+    }
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0u;
+    return (uint32_t)sms;
 }
 
 }  // namespace
 
-bool coop_build_fits(const GridWork &w) {
+bool coop_build_fits(const GridWork &w, cudaStream_t stream) {
     if (w.n == 0 || w.n > kCoopBlocks * kTile) return false;
     const Coop c = shape_of(w);
-    // every block resident at once: a device with fewer SMs to give (a slice
-    // of one) builds by digit passes
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || (uint32_t)sms < c.blocks)
-        return false;
+    // every block resident at once: a stream with fewer SMs to give (a slice
+    // of the device, a green context) builds by digit passes
+    if (sms_of(stream) < c.blocks) return false;
     return 4ull * ((uint64_t)c.blocks << c.bits) <= w.scan_ctl_bytes;
 }
 
