@@ -15,14 +15,20 @@ namespace fcu {
 struct CellRange {
     uint32_t first, count;
 };
-// Block b's part of 0 .. cells - 1 in `blocks` even pieces. In 64 bits, since
-// cells + blocks passes 2^32 at the largest cell counts; first + count never
-// does, nor does an offset below count that has one stride of a block added.
-FCU_HD inline CellRange cell_range(uint32_t cells, uint32_t blocks, uint32_t b) {
-    const uint64_t share = ((uint64_t)cells + blocks - 1) / blocks;
-    const uint64_t at = share * b, first = at < cells ? at : cells;
-    const uint64_t left = cells - first;
-    return CellRange{(uint32_t)first, (uint32_t)(share < left ? share : left)};
+// Cells of one of `blocks` even pieces, in 64 bits, since cells + blocks
+// passes 2^32 at the largest cell counts. (Once a build, on the host: the
+// division in the kernel cost a build of 65,536 positions 0.8 of 23 us.)
+FCU_HD inline uint32_t cell_share(uint32_t cells, uint32_t blocks) {
+    return (uint32_t)(((uint64_t)cells + blocks - 1) / blocks);
+}
+// Block b's part of 0 .. cells - 1 in pieces of `share`. first + count never
+// passes 2^32, nor does an offset below count that has one stride of a block
+// added.
+FCU_HD inline CellRange cell_range(uint32_t cells, uint32_t share, uint32_t b) {
+    const uint64_t at = (uint64_t)share * b;
+    const uint32_t first = at < cells ? (uint32_t)at : cells;
+    const uint32_t left = cells - first;
+    return CellRange{first, share < left ? share : left};
 }
 
 }  // namespace fcu

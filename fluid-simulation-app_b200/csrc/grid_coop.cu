@@ -43,7 +43,7 @@ constexpr uint32_t kMaxDigits = 1u << kMaxBits;
 struct Coop {
     const float4 *pos;
     GridGeom g;
-    uint32_t n, cells, blocks, piece;  // piece: positions a block owns
+    uint32_t n, cells, blocks, piece, share;  // piece, share: positions and cells a block owns
     int passes, bits;          // digit passes of `bits` bits each
     uint2 *a, *b;              // (key, index) ping-pong
     uint32_t *keys;            // the caller's keys, or null
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_grid_coop(Coop c) {
 
     // starts: this block's share of the cells in the sorted keys
     const uint32_t *sorted = reinterpret_cast<const uint32_t *>(in);
-    const CellRange r = cell_range(c.cells, gridDim.x, blockIdx.x);
+    const CellRange r = cell_range(c.cells, c.share, blockIdx.x);
     if (warp < 2) {
         const uint32_t at = warp_lower_bound(sorted, c.n, warp ? r.first + r.count : r.first);
         if (lane == 0) (warp ? s.hi : s.lo) = at;
@@ -270,6 +270,7 @@ Coop shape_of(const GridWork &w) {
     c.bits = std::max(kMinBits, (bits + c.passes - 1) / c.passes);
     c.blocks = std::min(kCoopBlocks, std::max(div_up(w.n, kThreads), div_up(w.cells, 4096u)));
     c.piece = std::max((uint32_t)kThreads, div_up(div_up(w.n, c.blocks), 32) * 32);
+    c.share = cell_share(w.cells, c.blocks);
     return c;
 }
 

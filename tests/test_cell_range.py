@@ -16,8 +16,9 @@ MAIN = """
 #include "cell_range.h"
 int main(int, char **v) {
     const uint32_t cells = strtoul(v[1], 0, 10), blocks = strtoul(v[2], 0, 10);
+    const uint32_t share = fcu::cell_share(cells, blocks);
     for (uint32_t b = 0; b < blocks; ++b) {
-        const fcu::CellRange r = fcu::cell_range(cells, blocks, b);
+        const fcu::CellRange r = fcu::cell_range(cells, share, b);
         printf("%u %u\\n", r.first, r.count);
     }
 }
