@@ -1663,6 +1663,8 @@ struct AdjImpl : AdjBase {
     std::vector<uint32_t *> ck_id;
     // forward scratch (one substep) and the backward's segment tapes
     Tape<T> work;
+    V3<T> *work_v[2] = {nullptr, nullptr};
+    T *work_kd = nullptr;
     std::vector<Tape<T>> seg;
     uint32_t seg_div_cap = 0, seg_den_cap = 0;
     Tape<T> fin;  // the final density pass of the loss
@@ -1767,8 +1769,12 @@ struct AdjImpl : AdjBase {
             arena.want(&ck_pp[k], N);
             arena.want(&ck_id[k], N);
         }
-        // the forward's scratch substep holds the longest schedule any substep may take
-        want_tape(work, kMaxIters + 1, kMaxIters + 1, true);
+        // The forward's scratch substep may take any schedule, and no sweep
+        // looks further back than the iteration before its own: two
+        // velocities a loop in turn, and one kappa.
+        want_tape(work, 0, 0, true);
+        for (auto &p : work_v) arena.want(&p, N);
+        arena.want(&work_kd, N);
         want_tape(fin, 0, 0, false);
         arena.want(&kd, N);
         arena.want(&gsl, N * kModelCap);
@@ -1803,6 +1809,12 @@ struct AdjImpl : AdjBase {
         arena.want(&fbar, (size_t)frames * spf * 3);
         arena.want(&cbar, 1);
         AK(arena.commit());
+        for (uint32_t q = 1; q < kMaxIters + 2; ++q) {
+            work.vdiv.push_back(q & 1 ? work_v[0] : work.vdiv[0]);
+            work.vden.push_back(q & 1 ? work_v[1] : work.vden[0]);
+        }
+        work.kddiv.assign(kMaxIters + 1, work_kd);
+        work.kdden.assign(kMaxIters + 1, work_kd);
         AK(cudaMemset(grid_ws, 0, count_grid_bytes(n, cells)));
         AK(cudaMemset(over, 0, 8));
         gw = count_grid_carve(grid_ws, n, cells, keys, starts, perm, over + 1);
