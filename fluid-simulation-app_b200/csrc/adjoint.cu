@@ -79,6 +79,12 @@ constexpr uint32_t kAdjSlabs = kSimSlabs;
 // 4: two block waves. Forward of 8,192 particles in 64 bits 1.007 ms at 8,
 // 1.091 at 4, 1.030 at 16; of 65,536 in 32 bits 4.316, 4.251 and 4.514.
 constexpr uint32_t kDensityMost = 148u * 2048u;
+// Particles from which it takes one thread each, four lanes then only adding
+// work (us of one thread / of 4 lanes; 32 bits: 98k 101 / 99, 131k 143 / 128,
+// 197k 172 / 186, 262k 228 / 242, 524k 405 / 473, 1M 798 / 934; 64 bits: 131k
+// 189 / 166, 262k 331 / 321, 393k 454 / 476, 524k 586 / 630, 1M 1154 / 1243).
+template <class T>
+constexpr uint32_t kDensityOne = 148u * (sizeof(T) == 4 ? 1200u : 2200u);
 
 // ---- small vector and dual types --------------------------------------------
 // Padded to four values, so that a record is one 16-byte load (two for
@@ -430,6 +436,75 @@ __global__ void __launch_bounds__(256) k_m_pos4(const V3<T> *__restrict__ x, flo
     if (i < n) pos4[i] = make_float4((float)x[i].x, (float)x[i].y, (float)x[i].z, 0.0f);
 }
 
+// The stencil rows of a model particle. Stencil cells and x slabs beyond the
+// support are skipped, as in the simulation's density sweep: on the float
+// position the grid was built from, the distances to the own cell's faces
+// shrunk by a margin far above both its rounding and the float / T difference
+// of positions.
+struct ModelStencil {
+    int bx, by, bz;
+    float px, sup2, margin, xl, xh, yl, yh, zl, zh;
+};
+template <class T>
+DEV ModelStencil model_stencil(const MP<T> &p, V3<T> xi) {
+    ModelStencil t;
+    const float px = (float)xi.x, py = (float)xi.y, pz = (float)xi.z;
+    t.px = px;
+    t.bx = (int)axis_cell(px, p.box_min[0], p.cell, p.dims[0]);
+    t.by = (int)axis_cell(py, p.box_min[1], p.cell, p.dims[1]);
+    t.bz = (int)axis_cell(pz, p.box_min[2], p.cell, p.dims[2]);
+    const float cellf = p.cell;
+    t.sup2 = (float)p.sup2;
+    t.margin = 1e-3f * cellf + 1e-6f * (fabsf(px) + fabsf(py) + fabsf(pz));
+    const float fx = px - (p.box_min[0] + (float)t.bx * cellf);
+    const float fy = py - (p.box_min[1] + (float)t.by * cellf);
+    const float fz = pz - (p.box_min[2] + (float)t.bz * cellf);
+    t.xl = fmaxf(fx - t.margin, 0.0f), t.xh = fmaxf(cellf - fx - t.margin, 0.0f);
+    t.yl = fmaxf(fy - t.margin, 0.0f), t.yh = fmaxf(cellf - fy - t.margin, 0.0f);
+    t.zl = fmaxf(fz - t.margin, 0.0f), t.zh = fmaxf(cellf - fz - t.margin, 0.0f);
+    return t;
+}
+// Slots s .. e - 1 of row (oz, oy), none where s >= e.
+template <class T>
+DEV void model_row(const MP<T> &p, const ModelStencil &t, const uint32_t *__restrict__ starts, uint32_t n, int oz,
+                   int oy, uint32_t &s, uint32_t &e) {
+    s = e = 0u;
+    const int cz = t.bz + oz, cy = t.by + oy;
+    const float dperp = (oz < 0 ? t.zl * t.zl : (oz > 0 ? t.zh * t.zh : 0.0f)) +
+                        (oy < 0 ? t.yl * t.yl : (oy > 0 ? t.yh * t.yh : 0.0f));
+    if (!(cz >= 0 && cz < (int)p.dims[2] && cy >= 0 && cy < (int)p.dims[1] && dperp < t.sup2)) return;
+    const float cellf = p.cell;
+    const uint32_t row = ((uint32_t)cz * p.dims[1] + (uint32_t)cy) * p.dims[0];
+    const int cx0 = (t.bx > 0 && dperp + t.xl * t.xl < t.sup2) ? t.bx - 1 : t.bx;
+    const int cx1 = (t.bx + 1 < (int)p.dims[0] && dperp + t.xh * t.xh < t.sup2) ? t.bx + 1 : t.bx;
+    const float half = sqrtf(t.sup2 - dperp) * 1.001f + t.margin;
+    const float xa = t.px - half, xb = t.px + half;
+    const uint32_t ca = axis_cell(xa, p.box_min[0], cellf, p.dims[0]);
+    const uint32_t cb = axis_cell(xb, p.box_min[0], cellf, p.dims[0]);
+    const uint32_t klo = max(ca * kAdjSlabs + axis_slab(xa, p.box_min[0], cellf, ca, kAdjSlabs),
+                             (uint32_t)cx0 * kAdjSlabs);
+    const uint32_t khi = min(cb * kAdjSlabs + axis_slab(xb, p.box_min[0], cellf, cb, kAdjSlabs),
+                             (uint32_t)cx1 * kAdjSlabs + (kAdjSlabs - 1));
+    s = starts[row * kAdjSlabs + klo];
+    e = min(starts[row * kAdjSlabs + khi + 1], n);
+}
+
+// The particle's outputs from its finished sums, the walls' fill and gradient.
+template <class T>
+DEV void model_density(const MP<T> &p, uint32_t i, uint32_t cnt, T w_sum, T near, V3<T> gsum, T gsq, T fill, V3<T> g,
+                       uint32_t *nbr_n, T *rho, T *rhon, T *alpha, V3<T> *wg, uint32_t *over) {
+    nbr_n[i] = cnt < kModelCap ? cnt : kModelCap;
+    if (cnt > kModelCap) atomicAdd(over, 1u);
+    const T r = p.m * w_sum + p.rho0 * fill;
+    wg[i] = g;
+    const V3<T> G = p.m * gsum + g;
+    T den = dot(G, G) + p.m * p.m * gsq;
+    if (den < T(1e-4f)) den = T(1e-4f);
+    rho[i] = r;
+    rhon[i] = near;
+    alpha[i] = r / den;
+}
+
 // Neighbour list of every particle (stencil order, grid order inside a
 // cell) with each pair's gradient scale gs (into gsl when given), density,
 // near density, alpha and the wall gradient. With `perm`
@@ -459,43 +534,10 @@ __global__ void __launch_bounds__(kWideThreads) k_m_density(MP<T> p, uint32_t n,
     const V3<T> xi = x[i];
     uint32_t *beg = s_beg[warp][w.group], *len = s_len[warp][w.group], *hit = s_hit[warp][w.group];
     {
-        // Stencil cells and x slabs beyond the support are skipped, as in the
-        // simulation's density sweep: on the float position the grid was built
-        // from, the distances to the own cell's faces shrunk by a margin far
-        // above both its rounding and the float / T difference of positions.
-        const float px = (float)xi.x, py = (float)xi.y, pz = (float)xi.z;
-        const int bx = (int)axis_cell(px, p.box_min[0], p.cell, p.dims[0]);
-        const int by = (int)axis_cell(py, p.box_min[1], p.cell, p.dims[1]);
-        const int bz = (int)axis_cell(pz, p.box_min[2], p.cell, p.dims[2]);
-        const float cellf = p.cell, sup2f = (float)p.sup2;
-        const float margin = 1e-3f * cellf + 1e-6f * (fabsf(px) + fabsf(py) + fabsf(pz));
-        const float fx = px - (p.box_min[0] + (float)bx * cellf);
-        const float fy = py - (p.box_min[1] + (float)by * cellf);
-        const float fz = pz - (p.box_min[2] + (float)bz * cellf);
-        const float xl = fmaxf(fx - margin, 0.0f), xh = fmaxf(cellf - fx - margin, 0.0f);
-        const float yl = fmaxf(fy - margin, 0.0f), yh = fmaxf(cellf - fy - margin, 0.0f);
-        const float zl = fmaxf(fz - margin, 0.0f), zh = fmaxf(cellf - fz - margin, 0.0f);
+        const ModelStencil st = model_stencil(p, xi);
         for (uint32_t r = w.lane; r < 9u; r += L) {
-            const int oz = (int)(r / 3u) - 1, oy = (int)(r % 3u) - 1;
-            const int cz = bz + oz, cy = by + oy;
             uint32_t s = 0, e = 0;
-            const float dperp = (oz < 0 ? zl * zl : (oz > 0 ? zh * zh : 0.0f)) +
-                                (oy < 0 ? yl * yl : (oy > 0 ? yh * yh : 0.0f));
-            if (w.live && cz >= 0 && cz < (int)p.dims[2] && cy >= 0 && cy < (int)p.dims[1] && dperp < sup2f) {
-                const uint32_t row = ((uint32_t)cz * p.dims[1] + (uint32_t)cy) * p.dims[0];
-                const int cx0 = (bx > 0 && dperp + xl * xl < sup2f) ? bx - 1 : bx;
-                const int cx1 = (bx + 1 < (int)p.dims[0] && dperp + xh * xh < sup2f) ? bx + 1 : bx;
-                const float half = sqrtf(sup2f - dperp) * 1.001f + margin;
-                const float xa = px - half, xb = px + half;
-                const uint32_t ca = axis_cell(xa, p.box_min[0], cellf, p.dims[0]);
-                const uint32_t cb = axis_cell(xb, p.box_min[0], cellf, p.dims[0]);
-                const uint32_t klo = max(ca * kAdjSlabs + axis_slab(xa, p.box_min[0], cellf, ca, kAdjSlabs),
-                                         (uint32_t)cx0 * kAdjSlabs);
-                const uint32_t khi = min(cb * kAdjSlabs + axis_slab(xb, p.box_min[0], cellf, cb, kAdjSlabs),
-                                         (uint32_t)cx1 * kAdjSlabs + (kAdjSlabs - 1));
-                s = starts[row * kAdjSlabs + klo];
-                e = min(starts[row * kAdjSlabs + khi + 1], n);
-            }
+            if (w.live) model_row(p, st, starts, n, (int)(r / 3u) - 1, (int)(r % 3u) - 1, s, e);
             beg[r] = s;
             len[r] = s < e ? e - s : 0u;
         }
@@ -626,16 +668,80 @@ __global__ void __launch_bounds__(kWideThreads) k_m_density(MP<T> p, uint32_t n,
     g.x = g.x + scale * S[3];
     g.y = g.y + scale * S[4];
     g.z = g.z + scale * S[5];
-    nbr_n[i] = cnt < kModelCap ? cnt : kModelCap;
-    if (cnt > kModelCap) atomicAdd(over, 1u);
-    const T r = p.m * w_sum + p.rho0 * (f - ws);
-    wg[i] = g;
-    const V3<T> G = p.m * gsum + g;
-    T den = dot(G, G) + p.m * p.m * gsq;
-    if (den < T(1e-4f)) den = T(1e-4f);
-    rho[i] = r;
-    rhon[i] = near;
-    alpha[i] = r / den;
+    model_density(p, i, cnt, w_sum, near, gsum, gsq, f - ws, g, nbr_n, rho, rhon, alpha, wg, over);
+}
+
+// The same with one thread a particle, for counts that fill the GPU so: the
+// same sums in the same order, so the same bits.
+template <class T>
+__global__ void __launch_bounds__(kAdjThreads) k_m_density_one(MP<T> p, uint32_t n, const V3<T> *__restrict__ x,
+                                                               const uint32_t *__restrict__ starts,
+                                                               const uint32_t *__restrict__ perm, uint32_t *nbr,
+                                                               T *gsl, uint32_t *nbr_n, T *rho, T *rhon, T *alpha,
+                                                               V3<T> *wg, uint32_t *over) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const V3<T> xi = x[i];
+    const ModelStencil st = model_stencil(p, xi);
+    T w_sum = p.sigma, near = T(0), gsq = T(0);
+    V3<T> gsum = zero3<T>();
+    uint32_t cnt = 0;
+    for (int oz = -1; oz <= 1; ++oz)
+        for (int oy = -1; oy <= 1; ++oy) {
+            uint32_t s, e;
+            model_row(p, st, starts, n, oz, oy, s, e);
+            // candidates four at a time: their positions load together
+            for (uint32_t k0 = s; k0 < e; k0 += 4) {
+                uint32_t jj[4];
+                V3<T> xj[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    uint32_t k = k0 + u < e ? (perm ? perm[k0 + u] : k0 + u) : i;
+                    if (k >= n) k = i;  // only after a grid build that gave up
+                    jj[u] = k;
+                    xj[u] = x[k];
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const V3<T> xij = xi - xj[u];
+                    const T r2 = dot(xij, xij);
+                    if (jj[u] == i || r2 >= p.sup2) continue;
+                    const Radial<T> R = radial(p, r2);
+                    w_sum += R.W;
+                    const T wn = R.q < T(1) ? T(1) - R.q : T(0);
+                    near += wn * wn * wn;
+                    const V3<T> gw = R.gs * xij;
+                    gsum = gsum + gw;
+                    gsq += dot(gw, gw);
+                    if (cnt < kModelCap) {
+                        nbr[(size_t)cnt * n + i] = jj[u];
+                        if (gsl) gsl[(size_t)cnt * n + i] = R.gs;
+                    }
+                    cnt++;
+                }
+            }
+        }
+    V3<T> g = zero3<T>();
+    w_grad<T, T>(p, xi.x, xi.y, xi.z, g.x, g.y, g.z);
+    model_density(p, i, cnt, w_sum, near, gsum, gsq, w_fill<T, T>(p, xi.x, xi.y, xi.z), g, nbr_n, rho, rhon, alpha, wg,
+                  over);
+}
+
+// Adds to *out the 32-bit words in which a and b differ: `words` a particle,
+// or with `cnt` in each of its first cnt[i] list entries.
+__global__ void __launch_bounds__(256) k_differ(const uint32_t *__restrict__ a, const uint32_t *__restrict__ b,
+                                                uint32_t words, uint32_t n, const uint32_t *__restrict__ cnt,
+                                                unsigned long long *out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t entries = cnt ? cnt[i] : 1u;
+    unsigned long long d = 0;
+    for (uint32_t k = 0; k < entries; ++k)
+        for (uint32_t w = 0; w < words; ++w) {
+            const size_t at = ((size_t)k * n + i) * words + w;
+            d += a[at] != b[at] ? 1u : 0u;
+        }
+    if (d) atomicAdd(out, d);
 }
 
 // The substep's state in the grid's cell order: slot k takes particle
@@ -1610,6 +1716,7 @@ struct AdjBase {
     virtual int32_t backward(double *grad_forces, double *grad_xsph) = 0;
     virtual int32_t final_state(double *pos3, double *vel3) = 0;
     virtual int32_t stall_grid() = 0;
+    virtual int32_t compare_densities(uint64_t *differ) = 0;
     uint32_t n = 0, frames = 0, spf = 0, ce = 1;
     std::vector<uint32_t> div_it, den_it;
     bool frozen = false, have_forward = false;
@@ -1860,14 +1967,52 @@ struct AdjImpl : AdjBase {
         return FLUID_OK;
     }
 
-    // k_m_density at 8 or 4 lanes a particle (kDensityMost).
-    void launch_density(const V3<T> *xs, const uint32_t *pm, T *scales, Tape<T> &t) {
-        auto at = [&](auto kernel, uint32_t lanes) {
-            kernel<<<nblk(n, kWideThreads / lanes), kWideThreads, 0, stream>>>(
-                mp, n, xs, starts, pm, t.nbr, scales, t.nbr_n, t.rho, t.rhon, t.alpha, t.wg, over);
+    // The density sweep at `lanes` a particle (8, 4, or 1).
+    void launch_density_at(uint32_t lanes, const V3<T> *xs, const uint32_t *pm, T *scales, Tape<T> &t) {
+        auto at = [&](auto kernel, uint32_t threads) {
+            kernel<<<nblk(n, threads / lanes), threads, 0, stream>>>(mp, n, xs, starts, pm, t.nbr, scales, t.nbr_n,
+                                                                     t.rho, t.rhon, t.alpha, t.wg, over);
         };
-        if ((uint64_t)n * 8 <= kDensityMost) at(k_m_density<T, 8>, 8);
-        else at(k_m_density<T, 4>, 4);
+        if (lanes == 8) at(k_m_density<T, 8>, kWideThreads);
+        else if (lanes == 4) at(k_m_density<T, 4>, kWideThreads);
+        else at(k_m_density_one<T>, kAdjThreads);
+    }
+    void launch_density(const V3<T> *xs, const uint32_t *pm, T *scales, Tape<T> &t) {
+        launch_density_at((uint64_t)n * 8 <= kDensityMost ? 8u : n < kDensityOne<T> ? 4u : 1u, xs, pm, scales, t);
+    }
+
+    // The density sweep of the current state at 4 and at 1 lanes against 8.
+    int32_t compare_densities(uint64_t *differ) override {
+        if (!have_forward) return report_error(FLUID_ERR_STATE, "adjoint: no forward state to sweep");
+        AK(cudaSetDevice(device));
+        have_forward = false;  // the loss's density pass is overwritten
+        int32_t rc = grid_positions();
+        if (rc == FLUID_OK) rc = grid();
+        if (rc != FLUID_OK) return rc;
+        T *const scales = reinterpret_cast<T *>(pair);
+        constexpr uint32_t kT = sizeof(T) / 4;
+        AK(cudaMemsetAsync(res_acc, 0, 8, stream));
+        launch_density_at(8, x, perm, gsl, work);
+        for (uint32_t lanes : {4u, 1u}) {
+            launch_density_at(lanes, x, perm, scales, fin);
+            auto cmp = [&](const void *a, const void *b, uint32_t words, const uint32_t *cnt) {
+                k_differ<<<nblk(n, 256), 256, 0, stream>>>((const uint32_t *)a, (const uint32_t *)b, words, n, cnt,
+                                                           res_acc);
+            };
+            cmp(work.nbr_n, fin.nbr_n, 1, nullptr);
+            cmp(work.nbr, fin.nbr, 1, work.nbr_n);
+            cmp(gsl, scales, kT, work.nbr_n);
+            cmp(work.rho, fin.rho, kT, nullptr);
+            cmp(work.rhon, fin.rhon, kT, nullptr);
+            cmp(work.alpha, fin.alpha, kT, nullptr);
+            cmp(work.wg, fin.wg, 4 * kT, nullptr);
+        }
+        AK(cudaGetLastError());
+        unsigned long long d = 0;
+        AK(cudaMemcpyAsync(&d, res_acc, 8, cudaMemcpyDeviceToHost, stream));
+        AK(cudaStreamSynchronize(stream));
+        *differ = d;
+        return check_flags();
     }
 
     // Neighbour grid of the state's positions xs, then lists and densities into t (the
@@ -2294,6 +2439,11 @@ int32_t fluid_adjoint_final_state(FluidAdjoint *a, double *pos3, double *vel3) {
 int32_t fluid_selftest_adjoint_wait(FluidAdjoint *a) {
     if (!a) return report_error(FLUID_ERR_ARG, "adjoint: null handle");
     return a->impl->stall_grid();
+}
+
+int32_t fluid_selftest_adjoint_density(FluidAdjoint *a, uint64_t *differ) {
+    if (!a || !differ) return report_error(FLUID_ERR_ARG, "adjoint: null argument");
+    return a->impl->compare_densities(differ);
 }
 
 int32_t fluid_adjoint_timing(const FluidAdjoint *a, float *forward_ms, float *backward_ms) {

@@ -163,6 +163,7 @@ def lib():
         "fluid_selftest_scan_wait": (i32, [i32, C.POINTER(C.c_float)]),
         "fluid_selftest_radix_wait": (i32, [i32, C.POINTER(C.c_float)]),
         "fluid_selftest_adjoint_wait": (i32, [P]),
+        "fluid_selftest_adjoint_density": (i32, [P, C.POINTER(u64)]),
         "fluid_batch_create": (P, [C.POINTER(FluidSimConfig), u32]),
         "fluid_batch_destroy": (None, [P]),
         "fluid_batch_boxes": (u32, [P]),

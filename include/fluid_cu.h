@@ -519,6 +519,13 @@ int32_t fluid_selftest_static_radix_wait(int32_t device, float *ms);
  * and the one after that works again. FLUID_OK when enqueued. */
 int32_t fluid_selftest_adjoint_wait(FluidAdjoint *adjoint);
 
+/* The adjoint's density sweep comes in three widths, chosen by the particle
+ * count, that must agree to the bit: runs all three on the state the last
+ * forward left and writes the number of 32-bit words (lists, scales,
+ * densities, alphas, wall gradients) in which they differ, 0 as it should.
+ * The handle needs a forward before its next backward. */
+int32_t fluid_selftest_adjoint_density(FluidAdjoint *adjoint, uint64_t *differ);
+
 #ifdef __cplusplus
 }
 #endif
