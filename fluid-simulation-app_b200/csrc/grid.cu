@@ -878,7 +878,7 @@ int32_t read_build_status(const uint32_t *err, cudaStream_t st, const char *who)
     if (e != cudaSuccess) return report_error(FLUID_ERR_CUDA, std::string(who) + ": " + cudaGetErrorString(e));
     if (flags & (ERRF_SCAN_TIMEOUT | ERRF_SORT_TIMEOUT))
         return report_error(FLUID_ERR_TIMEOUT,
-                            std::string(who) + ": a look-back wait of the build gave up; its starts and "
+                            std::string(who) + ": a bounded wait of the build gave up; its starts and "
                                                "permutation are invalid");
     return FLUID_OK;
 }

@@ -77,7 +77,8 @@ size_t grid_work_bytes(uint32_t n, uint32_t cells);
 GridWork grid_work_carve(void *ws, uint32_t n, uint32_t cells, uint32_t *err);
 
 // Reads a build's error word on `stream` (waiting for it): FLUID_OK, or
-// FLUID_ERR_TIMEOUT with a reason when a bounded look-back wait gave up.
+// FLUID_ERR_TIMEOUT with a reason when a bounded wait gave up (a look-back's,
+// or the one-launch build's barrier).
 int32_t read_build_status(const uint32_t *err, cudaStream_t stream, const char *who);
 // Enqueues one block of a radix digit pass on the scratch of `w` (carved for
 // at least two tiles of keys) that claims tile 1 while tile 0 never
@@ -93,6 +94,10 @@ bool coop_build_fits(const GridWork &w, cudaStream_t stream);
 // behind, where the driver would not hold every block at once after all.
 cudaError_t coop_build_enqueue(cudaStream_t stream, const float4 *pos, const GridGeom &g, uint32_t *keys,
                                uint32_t *starts, uint32_t *perm, const GridWork &w);
+// Enqueues the same build with a barrier that expects an arrival more than
+// come: every wait gives up and sets w.err.
+cudaError_t enqueue_stalled_coop_build(cudaStream_t stream, const float4 *pos, const GridGeom &g, uint32_t *starts,
+                                       uint32_t *perm, const GridWork &w);
 
 // Enqueues keys -> stable radix sort -> starts on `stream`. `keys` receives
 // each input's cell key, `starts` the exclusive scan of the cell counts with

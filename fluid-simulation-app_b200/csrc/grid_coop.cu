@@ -25,11 +25,15 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <string>
+#include <vector>
 
 #include "cell_range.h"
 #include "grid.cuh"
 
 namespace fcu {
+
+int32_t report_error(int32_t code, const std::string &msg);
 
 namespace {
 
@@ -354,4 +358,80 @@ cudaError_t coop_build_enqueue(cudaStream_t stream, const float4 *pos, const Gri
     return launch<kMaxBits>(stream, c);
 }
 
+cudaError_t enqueue_stalled_coop_build(cudaStream_t stream, const float4 *pos, const GridGeom &g, uint32_t *starts,
+                                       uint32_t *perm, const GridWork &w) {
+    if (!coop_build_fits(w, stream)) return cudaErrorInvalidValue;
+    cudaError_t e = cudaMemsetAsync(w.err, 0, 4 * kErrWords, stream);
+    // one arrival short from the first barrier on: its count starts at -1
+    if (e == cudaSuccess) e = cudaMemsetAsync(w.err + kErrBarrier, 0xff, 4, stream);
+    if (e == cudaSuccess) e = coop_build_enqueue(stream, pos, g, w.k2, starts, perm, w);
+    return e;
+}
+
 }  // namespace fcu
+
+// The build's barrier, run out on purpose on a real workspace and reported
+// through fluid_grid_build_status: every barrier expects an arrival more than
+// come, so every block gives up at every one and the kernel ends by itself.
+// What it then writes from counts that nobody published stays inside the
+// outputs: the words on either side of them are checked.
+extern "C" int32_t fluid_selftest_coop_wait(int32_t device, float *ms) {
+    using namespace fcu;
+    auto fail = [](cudaError_t e) {
+        return report_error(FLUID_ERR_CUDA, std::string("fluid_selftest_coop_wait: ") + cudaGetErrorString(e));
+    };
+    cudaError_t e = cudaSetDevice(device);
+    if (e != cudaSuccess) return fail(e);
+    constexpr uint32_t n = 5003, side = 16, cells = side * side * side, guard = 64, mark = 0xa5a5a5a5u;
+    FluidGrid grid{};
+    grid.cell = 1.0f;
+    for (int a = 0; a < 3; ++a) grid.dims[a] = side;
+    GridGeom g{};
+    g.cell = 1.0f;
+    for (int a = 0; a < 3; ++a) g.dims[a] = side;
+    const size_t words = 3 * guard + cells + 1 + n;  // guard, starts, guard, perm, guard
+    std::vector<uint32_t> out(words, 0u);
+    std::vector<float> at(4 * n);
+    for (size_t k = 0; k < at.size(); ++k) at[k] = (float)((k * 7919u) % 1600u) * 0.01f;
+    char *ws = nullptr;
+    uint32_t *dst = nullptr;
+    float4 *pos = nullptr;
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    float t = 0.0f;
+    int32_t rc = FLUID_OK;
+    do {
+        const size_t bytes = grid_work_bytes(n, cells);
+        if ((e = cudaMalloc(&ws, bytes)) != cudaSuccess) break;
+        if ((e = cudaMalloc(&dst, 4 * words)) != cudaSuccess) break;
+        if ((e = cudaMalloc(&pos, 16 * n)) != cudaSuccess) break;
+        if ((e = cudaMemset(ws, 0x5a, bytes)) != cudaSuccess) break;
+        if ((e = cudaMemset(dst, 0xa5, 4 * words)) != cudaSuccess) break;
+        if ((e = cudaMemcpy(pos, at.data(), 16 * n, cudaMemcpyHostToDevice)) != cudaSuccess) break;
+        if ((e = cudaEventCreate(&ev[0])) != cudaSuccess) break;
+        if ((e = cudaEventCreate(&ev[1])) != cudaSuccess) break;
+        const GridWork w = grid_work_carve(ws, n, cells, nullptr);
+        cudaEventRecord(ev[0]);
+        e = enqueue_stalled_coop_build(nullptr, pos, g, dst + guard, dst + 2 * guard + cells + 1, w);
+        if (e != cudaSuccess) break;
+        cudaEventRecord(ev[1]);
+        if ((e = cudaEventSynchronize(ev[1])) != cudaSuccess) break;
+        cudaEventElapsedTime(&t, ev[0], ev[1]);
+        rc = fluid_grid_build_status(ws, n, &grid, nullptr);
+        if ((e = cudaMemcpy(out.data(), dst, 4 * words, cudaMemcpyDeviceToHost)) != cudaSuccess) break;
+    } while (false);
+    for (cudaEvent_t x : ev)
+        if (x) cudaEventDestroy(x);
+    cudaFree(ws);
+    cudaFree(dst);
+    cudaFree(pos);
+    if (e != cudaSuccess) return fail(e);
+    if (ms) *ms = t;
+    for (size_t k = 0; k < guard; ++k)
+        if (out[k] != mark || out[guard + cells + 1 + k] != mark || out[words - 1 - k] != mark)
+            return report_error(FLUID_ERR_STATE, "fluid_selftest_coop_wait: a write outside the outputs");
+    if (rc == FLUID_ERR_TIMEOUT)
+        return report_error(FLUID_ERR_TIMEOUT,
+                            "fluid_selftest_coop_wait: the grid barrier gave up, as it should, and "
+                            "fluid_grid_build_status reported it");
+    return rc;
+}

@@ -162,6 +162,7 @@ def lib():
         "fluid_selftest_static_radix_wait": (i32, [i32, C.POINTER(C.c_float)]),
         "fluid_selftest_scan_wait": (i32, [i32, C.POINTER(C.c_float)]),
         "fluid_selftest_radix_wait": (i32, [i32, C.POINTER(C.c_float)]),
+        "fluid_selftest_coop_wait": (i32, [i32, C.POINTER(C.c_float)]),
         "fluid_selftest_adjoint_wait": (i32, [P]),
         "fluid_selftest_adjoint_density": (i32, [P, C.POINTER(u64)]),
         "fluid_batch_create": (P, [C.POINTER(FluidSimConfig), u32]),
@@ -250,6 +251,15 @@ def selftest_static_radix_wait(device=0):
     scratch, read back through fluid_grid_build_static_status."""
     ms = C.c_float(0.0)
     rc = lib().fluid_selftest_static_radix_wait(device, C.byref(ms))
+    return rc, ms.value
+
+
+def selftest_coop_wait(device=0):
+    """Runs the one-launch grid build's barriers out
+    (fluid_selftest_coop_wait): returns (status, kernel ms); ERR_TIMEOUT is
+    the expected status."""
+    ms = C.c_float(0.0)
+    rc = lib().fluid_selftest_coop_wait(device, C.byref(ms))
     return rc, ms.value
 
 

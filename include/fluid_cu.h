@@ -455,9 +455,9 @@ int32_t fluid_grid_build(const float *pos4, uint32_t n, const FluidGrid *grid, u
 
 /* Whether the fluid_grid_build last run on `workspace` (with the same n and
  * grid) completed: FLUID_OK, or FLUID_ERR_TIMEOUT (reason in
- * fluid_last_error()) when one of its bounded look-back waits gave up, in
- * which case its starts and permutation are invalid (a missing prefix was
- * counted as zero, so slots may repeat). Reads the build's error word on
+ * fluid_last_error()) when one of its bounded waits gave up (a look-back's, or
+ * a barrier of the one-launch build), in which case its starts and permutation
+ * are invalid (a missing count was taken as it stood, so slots may repeat). Reads the build's error word on
  * `stream` after the work queued there and waits for it; allocates nothing.
  * Follows the reference's convention that a failure carries its reason
  * (crates/fluid-ffi/src/lib.rs:86-108). */
@@ -486,7 +486,7 @@ int32_t fluid_grid_build_static(const float *pos4, uint32_t n, const FluidGrid *
                                 uint32_t *keys, uint32_t *starts, uint32_t *perm, void *stream);
 
 /* Whether the last fluid_grid_build_static on the current device completed:
- * FLUID_OK, or FLUID_ERR_TIMEOUT when a bounded look-back wait gave up and
+ * FLUID_OK, or FLUID_ERR_TIMEOUT when a bounded wait gave up and
  * its starts and permutation are invalid. The error word lives in the fixed
  * scratch, so read it after that build and before the next call on the
  * device, which clears it. Reads on `stream` and waits; allocates nothing. */
@@ -513,6 +513,13 @@ int32_t fluid_selftest_radix_wait(int32_t device, float *ms);
  * fluid_grid_build_static_status: FLUID_ERR_TIMEOUT, as it should.
  * Allocates nothing. */
 int32_t fluid_selftest_static_radix_wait(int32_t device, float *ms);
+
+/* The one-launch build of up to 148 x 8,192 positions with a barrier that
+ * expects an arrival more than come, so that every bounded wait (2^20 polls)
+ * gives up: FLUID_ERR_TIMEOUT, read back through fluid_grid_build_status, as
+ * it should; FLUID_ERR_STATE if anything was written outside the outputs.
+ * *ms (if not null) the kernel's time. */
+int32_t fluid_selftest_coop_wait(int32_t device, float *ms);
 
 /* The stalled scan on an adjoint handle's own grid buffers, enqueued on its
  * stream: the handle's next forward or backward returns FLUID_ERR_TIMEOUT,
