@@ -15,6 +15,8 @@
 // Compiled with -fmad=false: no product-sum is fused unless written so.
 #include <cuda_fp16.h>
 
+#include <string>
+
 #include "solve.cuh"
 #include "wide.cuh"
 
@@ -931,6 +933,46 @@ __device__ __forceinline__ float quotient(float a, float b, float y) {
     return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
 
+// A splitmix64 stream for k_quotients.
+__device__ __forceinline__ uint32_t next_random(unsigned long long &s) {
+    s += 0x9e3779b97f4a7c15ull;
+    unsigned long long z = s;
+    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+    return (uint32_t)((z ^ (z >> 31)) >> 32);
+}
+// A float of exponent lo .. hi with a random significand, one in eight times
+// all zeros or all ones.
+__device__ __forceinline__ float random_float(unsigned long long &s, int lo, int hi) {
+    const uint32_t r = next_random(s), m = next_random(s);
+    const uint32_t e = (uint32_t)(lo + (int)(r % (uint32_t)(hi - lo + 1)) + 127);
+    const uint32_t pick = m >> 28;
+    const uint32_t f = pick == 0u ? 0u : (pick == 1u ? 0x7fffffu : m & 0x7fffffu);
+    return __uint_as_float((next_random(s) & 0x80000000u) | (e << 23) | f);
+}
+// quotient() against the division on the pairs' operands: a distance of 2^-17
+// (1e-5 lies in that binade) to 2^62, a coordinate difference of 2^-60 or more
+// up to the distance's binade, and that times a tension factor of 2^-40 to
+// 2^60 (up to 2^40 from distances of 2^14 on, where no cohesion comes near it).
+// Adds the quotients that differ to *differ.
+__global__ void __launch_bounds__(256) k_quotients(unsigned long long seed, uint32_t rounds,
+                                                   unsigned long long *differ) {
+    unsigned long long s = seed + ((unsigned long long)(blockIdx.x * blockDim.x + threadIdx.x) << 32);
+    unsigned long long d = 0;
+    for (uint32_t k = 0; k < rounds; ++k) {
+        const float r = fabsf(random_float(s, -17, 62));
+        const int er = (int)(__float_as_uint(r) >> 23) - 127;
+        const float x = random_float(s, -60, er);
+        const float kx = random_float(s, -40, er < 14 ? 59 : 39) * x;
+        const float y = __frcp_rn(r);
+        // compared as values: a zero's sign is free
+        d += quotient(x, r, y) != x / r ? 1u : 0u;
+        d += fabsf(kx / r) >= 0x1p-126f && quotient(kx, r, y) != kx / r ? 1u : 0u;
+        d += quotient(copysignf(0.0f, x), r, y) != 0.0f ? 1u : 0u;
+    }
+    if (d) atomicAdd(differ, d);
+}
+
 // The near pressure's and the tension's six quotients by the distance share
 // one reciprocal: a pair's ten divisions were 39 % of the sweep (555 us on
 // the 1M workload without m / rho_j stored, 338 with every one left out),
@@ -1606,4 +1648,28 @@ void launch_advect(cudaStream_t s, const DevParams &P, const SimBufs &b, const D
     if (ntr) k_advect<<<blocks_for(ntr, 256), 256, 0, s>>>(P, b, st, ntr);
 }
 
+int32_t report_error(int32_t code, const std::string &msg);
+
 }  // namespace fcu
+
+extern "C" int32_t fluid_selftest_quotient(int32_t device, uint64_t seed, uint64_t pairs, uint64_t *differ) {
+    using namespace fcu;
+    if (!differ) return report_error(FLUID_ERR_ARG, "fluid_selftest_quotient: null argument");
+    constexpr uint32_t kBlocks = 148 * 8, kThreads = 256;
+    const uint64_t rounds = (pairs + kBlocks * kThreads - 1) / (kBlocks * kThreads);
+    if (rounds == 0 || rounds > 1u << 20) return report_error(FLUID_ERR_ARG, "fluid_selftest_quotient: 1..2^38 pairs");
+    unsigned long long *d = nullptr, out = 0;
+    cudaError_t e = cudaSetDevice(device);
+    if (e == cudaSuccess) e = cudaMalloc(&d, 8);
+    if (e == cudaSuccess) e = cudaMemset(d, 0, 8);
+    if (e == cudaSuccess) {
+        k_quotients<<<kBlocks, kThreads>>>(seed, (uint32_t)rounds, d);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(&out, d, 8, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e != cudaSuccess)
+        return report_error(FLUID_ERR_CUDA, std::string("fluid_selftest_quotient: ") + cudaGetErrorString(e));
+    *differ = out;
+    return FLUID_OK;
+}

@@ -162,6 +162,7 @@ def lib():
         "fluid_selftest_static_radix_wait": (i32, [i32, C.POINTER(C.c_float)]),
         "fluid_selftest_scan_wait": (i32, [i32, C.POINTER(C.c_float)]),
         "fluid_selftest_radix_wait": (i32, [i32, C.POINTER(C.c_float)]),
+        "fluid_selftest_quotient": (i32, [i32, u64, u64, C.POINTER(u64)]),
         "fluid_selftest_coop_wait": (i32, [i32, C.POINTER(C.c_float)]),
         "fluid_selftest_adjoint_wait": (i32, [P]),
         "fluid_selftest_adjoint_density": (i32, [P, C.POINTER(u64)]),

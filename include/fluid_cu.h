@@ -526,6 +526,12 @@ int32_t fluid_selftest_coop_wait(int32_t device, float *ms);
  * and the one after that works again. FLUID_OK when enqueued. */
 int32_t fluid_selftest_adjoint_wait(FluidAdjoint *adjoint);
 
+/* The forces' quotients by one shared reciprocal against the division they
+ * stand for, on `pairs` (at most 2^38) random operands of the ranges they are
+ * used on, their significands all zeros or all ones among them: writes how
+ * many differ in value, 0 as it should. */
+int32_t fluid_selftest_quotient(int32_t device, uint64_t seed, uint64_t pairs, uint64_t *differ);
+
 /* The adjoint's density sweep comes in three widths, chosen by the particle
  * count, that must agree to the bit: runs all three on the state the last
  * forward left and writes the number of 32-bit words (lists, scales,
