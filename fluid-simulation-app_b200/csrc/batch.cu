@@ -679,9 +679,12 @@ int32_t fluid_batch_autotune(FluidBatch *s, const FluidStep *steps, uint32_t *ch
     if (rc != FLUID_OK) return rc;
     BK(cudaGetLastError());
     drop_graphs(s);
+    // a sweep that shares particles among lanes ran the same kernel three
+    // times: it keeps the default
+    const bool sized = sweeps_take_block_sizes(s->n);
     for (int k = 0; k < kTuneCount; ++k) {
         int best = 1;
-        for (int c = 0; c < 3; ++c)
+        for (int c = 0; c < 3 && (sized || k == kTuneIntegrate); ++c)
             if (ms[c][k] < ms[best][k]) best = c;
         s->tpb[k] = (uint16_t)cand[best];
         if (chosen) chosen[k] = (uint32_t)cand[best];

@@ -1562,6 +1562,7 @@ inline int lanes_for(uint32_t n) {
         if ((uint64_t)n * lanes <= kWideMost) return lanes;
     return 1;
 }
+bool sweeps_take_block_sizes(uint32_t n) { return lanes_for(n) == 1; }
 #define FCU_WIDE_AT(L, one, batch, ...)                                                                     \
     do {                                                                                                    \
         const uint32_t blocks_ = blocks_for(g.n, kWideThreads / L);                                         \

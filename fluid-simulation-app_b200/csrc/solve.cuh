@@ -91,6 +91,9 @@ constexpr int kStatsThreads = 256;
 // A tolerance loop's gate: the kernel skips boxes whose loop has stopped.
 enum Gate : int { kGateNone = 0, kGateDiv = 1, kGateDen = 2 };
 
+// Whether the solve's sweeps over n particles launch at the tuned block sizes:
+// the one-thread sweeps do, the lane-shared ones of smaller counts do not.
+bool sweeps_take_block_sizes(uint32_t n);
 // Enqueue helpers: each launches one kernel on `s`.
 void launch_density_div(cudaStream_t s, const Geo &g, const SimBufs &b, int slot);
 void launch_div_kappa(cudaStream_t s, const Geo &g, const SimBufs &b, int slot, int gate);
