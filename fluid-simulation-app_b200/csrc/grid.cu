@@ -820,6 +820,15 @@ cudaError_t count_grid_order(cudaStream_t stream, const CountGrid &w, const Grid
     return cudaGetLastError();
 }
 
+cudaError_t starts_enqueue(cudaStream_t stream, const uint32_t *sorted, uint32_t n, uint32_t cells, uint32_t *starts) {
+    // small tiles until the large ones fill the GPU
+    if (cells < 148u * kStartMinBlocks * 16u * kStartThreads)
+        k_starts<4><<<div_up(cells, 4 * kStartThreads), kStartThreads, 0, stream>>>(sorted, n, cells, starts);
+    else
+        k_starts<16><<<div_up(cells, 16 * kStartThreads), kStartThreads, 0, stream>>>(sorted, n, cells, starts);
+    return cudaGetLastError();
+}
+
 cudaError_t grid_build_enqueue(cudaStream_t stream, const float4 *pos, uint32_t n, const GridGeom &g, uint32_t *keys,
                                uint32_t *starts, uint32_t *perm, GridWork &w) {
     cudaError_t e;
@@ -852,12 +861,7 @@ cudaError_t grid_build_enqueue(cudaStream_t stream, const float4 *pos, uint32_t 
         }
         sorted = kin;
     }
-    // small tiles until the large ones fill the GPU
-    if (cells < 148u * kStartMinBlocks * 16u * kStartThreads)
-        k_starts<4><<<div_up(cells, 4 * kStartThreads), kStartThreads, 0, stream>>>(sorted, n, cells, starts);
-    else
-        k_starts<16><<<div_up(cells, 16 * kStartThreads), kStartThreads, 0, stream>>>(sorted, n, cells, starts);
-    return cudaGetLastError();
+    return starts_enqueue(stream, sorted, n, cells, starts);
 }
 
 int32_t report_error(int32_t code, const std::string &msg);

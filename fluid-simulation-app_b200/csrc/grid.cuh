@@ -94,6 +94,8 @@ bool coop_build_fits(const GridWork &w, cudaStream_t stream);
 // behind, where the driver would not hold every block at once after all.
 cudaError_t coop_build_enqueue(cudaStream_t stream, const float4 *pos, const GridGeom &g, uint32_t *keys,
                                uint32_t *starts, uint32_t *perm, const GridWork &w);
+// Enqueues the starts (starts[cells] = n) of the n sorted keys.
+cudaError_t starts_enqueue(cudaStream_t stream, const uint32_t *sorted, uint32_t n, uint32_t cells, uint32_t *starts);
 // Enqueues the same build with a barrier that expects an arrival more than
 // come: every wait gives up and sets w.err.
 cudaError_t enqueue_stalled_coop_build(cudaStream_t stream, const float4 *pos, const GridGeom &g, uint32_t *starts,

@@ -8,7 +8,8 @@
 // the input: keys, then per digit the piece ranked (its counts published), a
 // grid barrier, the piece's digit offsets from everybody's counts, the piece
 // written in digit order through shared memory, a barrier; finally the
-// starts, each block searching its share of the cells in the sorted keys. A
+// starts, each block searching its share of the cells in the sorted keys, or
+// where the cells are many (kStartsApart) k_starts in a launch of its own. A
 // digit is as narrow as the keys allow in the same number of passes. The same
 // stable order and starts as the digit passes, whatever the distribution.
 //
@@ -51,7 +52,7 @@ struct Coop {
     int passes, bits;          // digit passes of `bits` bits each
     uint2 *a, *b;              // (key, index) ping-pong
     uint32_t *keys;            // the caller's keys, or null
-    uint32_t *starts, *perm;
+    uint32_t *starts, *perm;   // starts null: not written here
     uint32_t *counts;          // [block][digit]
     uint32_t *barrier, *err;
 };
@@ -228,6 +229,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_grid_coop(Coop c) {
                 out[dst] = v;
             }
         }
+        if (last && !c.starts) return;  // the starts have a launch of their own
         grid_barrier(c, ++phase);
         uint2 *const was = const_cast<uint2 *>(in);
         in = out;
@@ -293,6 +295,17 @@ cudaError_t launch(cudaStream_t stream, Coop &c) {
     return l;
 }
 
+// Cells from which the starts are k_starts' launch after this one: a thread
+// here searches a cell's start among its block's keys, which past some
+// thousand cells a block costs more than a launch that reads the keys once. us
+// a build with the starts here / apart / by digit passes, 1M positions, in any
+// order and all in one cell: 262k cells 53 / 54 / 78 and 54 / 52 / 68, 512k 58
+// / 56 / 79 and 64 / 54 / 69, 1M 62 / 58 / 82 and 75 / 56 / 70, 4.1M 94 / 63 /
+// 84 and 154 / 64 / 74, 16.8M 211 / 81 / 101 and 463 / 77 / 88; 150k positions
+// over 262k cells 35 / 35 / 56, over 2.1M 50 / 42 / 62.
+constexpr uint32_t kStartsApart = 400000;
+bool starts_apart(const GridWork &w) { return w.cells > kStartsApart; }
+
 // Driver entry points, null where the driver has none.
 struct GreenCalls {
     PFN_cuStreamGetGreenCtx ctx_of = nullptr;
@@ -350,12 +363,16 @@ cudaError_t coop_build_enqueue(cudaStream_t stream, const float4 *pos, const Gri
     c.a = reinterpret_cast<uint2 *>(w.k1);       // k1, k2
     c.b = reinterpret_cast<uint2 *>(w.v1);       // v1, v2
     c.keys = keys == w.k2 ? nullptr : keys;      // k2: no buffer of the caller's
-    c.starts = starts;
+    const bool apart = starts_apart(w);
+    c.starts = apart ? nullptr : starts;
     c.perm = perm;
     c.counts = reinterpret_cast<uint32_t *>(w.scan_ctl);
     c.err = w.err;
     c.barrier = w.err + kErrBarrier;
-    return launch<kMaxBits>(stream, c);
+    const cudaError_t e = launch<kMaxBits>(stream, c);
+    if (e != cudaSuccess || !apart) return e;
+    // the last pass left the sorted keys in its output
+    return starts_enqueue(stream, c.passes & 1 ? w.v1 : w.k1, w.n, w.cells, starts);
 }
 
 cudaError_t enqueue_stalled_coop_build(cudaStream_t stream, const float4 *pos, const GridGeom &g, uint32_t *starts,
