@@ -40,23 +40,24 @@ __device__ __forceinline__ unsigned long long fixed_w(float w) {
     return (unsigned long long)__float2uint_rn(w * (float)kFieldScale);
 }
 
-// 2^`shift` adjacent lanes per particle: its quad, radius 1.5 h around (x, y)
+// kLanes adjacent lanes per particle: its quad, radius 1.5 h around (x, y)
 // projected orthographically, over the texels whose centres it covers, a lane
-// taking every 2^shift-th column; weight (1 - |corner|^2)^2 / 2
+// taking every kLanes-th column; weight (1 - |corner|^2)^2 / 2
 // (sim_sprites.wgsl `weight`). The sums are integers, so the order of the
-// adds is free. One thread a particle walked its 100-odd texels alone, in two
-// blocks per SM at 72,072 particles: a splat of them into 295 x 639 texels,
-// waited for, 165 us by one lane, 132 by 4, 108 by 8 and 16; of 1,620 into
-// 32 x 64 41, 35, 39 and 35. What is left is the 64-bit adds.
+// adds is free. What is left is the 64-bit adds, and for many particles of
+// small quads each lane's set-up of the quad. The stride is a constant of the
+// instance, so that the columns' loop unrolls (one lane of 1,048,576
+// particles into 128 x 128 texels 129 us, with the lanes a parameter 192).
+template <int kLanes>
 __global__ void __launch_bounds__(256) k_body_splat(FieldGeom g, const float4 *__restrict__ pos,
                                                     const float4 *__restrict__ vel,
                                                     const float4 *__restrict__ pvel,
                                                     const float *__restrict__ density, uint32_t n,
-                                                    uint32_t shift, unsigned long long *acc) {
+                                                    unsigned long long *acc) {
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (uint64_t)n << shift) return;
-    const uint32_t i = (uint32_t)(t >> shift);
-    const int lanes = 1 << shift, lane = (int)t & (lanes - 1);
+    if (t >= (uint64_t)n * kLanes) return;
+    const uint32_t i = (uint32_t)(t / kLanes);
+    const int lane = (int)(t % kLanes);
     const float4 p = __ldg(&pos[i]);
     const float px = (p.x - g.cx) / g.ex, py = (p.y - g.cy) / g.ey;
     const float rx = g.radius / g.ex, ry = g.radius / g.ey;
@@ -74,7 +75,7 @@ __global__ void __launch_bounds__(256) k_body_splat(FieldGeom g, const float4 *_
     for (int ty = ty0; ty <= ty1; ++ty) {
         const float yt = 1.0f - ((float)ty + 0.5f) / H * 2.0f;
         const float cy = (yt - py) / ry;
-        for (int tx = tx0 + lane; tx <= tx1; tx += lanes) {
+        for (int tx = tx0 + lane; tx <= tx1; tx += kLanes) {
             const float xt = ((float)tx + 0.5f) / W * 2.0f - 1.0f;
             const float cx = (xt - px) / rx;
             const float falloff = fmaxf(1.0f - (cx * cx + cy * cy), 0.0f);
@@ -151,12 +152,30 @@ __global__ void __launch_bounds__(256) k_field_filter(FieldGeom g, const float2 
 void launch_field_splat(cudaStream_t s, const FieldGeom &g, const float4 *pos, const float4 *vel,
                         const float4 *pvel, const float *density, uint32_t n, float keep, float splat,
                         float2 *field, unsigned long long *acc) {
-    // as many lanes as the quad's columns (a margin of two among them) keep busy
+    // The more columns a quad has (a margin of two among them) the more lanes
+    // it keeps busy; where the particles alone fill the GPU, one lane has the
+    // least set-up for its few texels. us a splat by 1 / 2 / 4 / 8 / 16 lanes:
+    //   1,048,576 particles, 3.9 columns 66 / 60 / 99 / 173 / 334, 6.6 130 / 217
+    //   / 186 / 293 / 562, 11 1593 / 1213 / 1285 / 1198 / 1770, 32 10887 / 5827
+    //   / 5104 / 5005 / 4846;
+    //   307,200, 6.6 86 / 97 / 100 / 121 / 224, 9.6 297 / 237 / 226 / 234 / 382;
+    //   73,728, 5.4 31 / 31 / 24 / 30 / 48, 9.0 81 / 66 / 57 / 56 / 82, 14 240 /
+    //   235 / 189 / 142 / 152, 41 1162 / 845 / 639 / 551 / 482;
+    //   800, 5.9 18 / 19 / 13 / 13 / 13, 26 130 / 74 / 43 / 42 / 25.
     const float columns = g.radius / g.ex * (float)g.w + 3.0f;
-    const uint32_t shift = columns > 8.0f ? 4u : columns > 4.0f ? 3u : 2u;
-    if (n)
-        k_body_splat<<<(uint32_t)((((uint64_t)n << shift) + 255) / 256), 256, 0, s>>>(g, pos, vel, pvel, density, n,
-                                                                                      shift, acc);
+    const bool many = n >= 100000u;
+    const int lanes = columns < 5.0f ? 2 : columns < 7.3f ? (many ? 1 : 4) : columns < 10.0f && many ? 4
+                      : columns < 24.0f ? 8 : 16;
+    auto at = [&](auto kernel) {
+        kernel<<<(uint32_t)(((uint64_t)n * (uint32_t)lanes + 255) / 256), 256, 0, s>>>(g, pos, vel, pvel, density, n, acc);
+    };
+    if (n) {
+        if (lanes == 16) at(k_body_splat<16>);
+        else if (lanes == 8) at(k_body_splat<8>);
+        else if (lanes == 4) at(k_body_splat<4>);
+        else if (lanes == 2) at(k_body_splat<2>);
+        else at(k_body_splat<1>);
+    }
     const uint32_t texels = g.w * g.h;
     k_field_resolve<<<(texels + 255) / 256, 256, 0, s>>>(field, acc, texels, keep, splat);
 }
