@@ -60,10 +60,11 @@ SUBSTEP_CAP = 16
 
 # Algorithmic bytes per particle of each substep kernel: the particle's own
 # records it must read and write once (neighbour reads are cache hits in
-# cell order and not counted). keys+count 20, reorder 116, density 44,
-# divergence kappa 28 / apply 36, forces (with their apply, one sweep) 148,
-# density kappa 36 / apply 36, integrate 120.
-ALGO_BYTES = {"grid": 20.0, "gather": 116.0, "density_div": 44.0, "div_kappa": 28.0,
+# cell order and not counted). keys+count 20, reorder 116, density 84 (with
+# the forces' two records, which it forms, and the last pressure and the
+# temperature they need), divergence kappa 28 / apply 36, forces (with their
+# apply, one sweep) 148, density kappa 36 / apply 36, integrate 120.
+ALGO_BYTES = {"grid": 20.0, "gather": 116.0, "density_div": 84.0, "div_kappa": 28.0,
               "div_apply": 36.0, "forces_eval": 148.0,
               "den_kappa": 36.0, "den_apply": 36.0, "integrate": 120.0}
 # DRAM bytes (read + write) per particle per launch: a constant taken from
@@ -71,19 +72,19 @@ ALGO_BYTES = {"grid": 20.0, "gather": 116.0, "density_div": 44.0, "div_kappa": 2
 # particles, on the state after the benchmark's 25 frames
 # (dram__bytes_read.sum + dram__bytes_write.sum), not measured by this
 # script; a kernel change calls for a new capture.
-NCU_TRAFFIC_PER_PARTICLE = {"density_div": (106.80e6 + 318.62e6) / 1048576,
-                            "forces_eval": (410.57e6 + 38.01e6) / 1048576,
-                            "den_kappa": (406.19e6 + 15.34e6) / 1048576}
+NCU_TRAFFIC_PER_PARTICLE = {"density_div": (113.19e6 + 342.34e6) / 1048576,
+                            "forces_eval": (450.02e6 + 45.34e6) / 1048576,
+                            "den_kappa": (406.19e6 + 15.75e6) / 1048576}
 
 
 # What holds each leading kernel back, from the same ncu capture: none of
 # them is DRAM-bound, so their fraction of the HBM roofline stays low.
 NCU_LIMITER = {
-    "density_div": "SM issue and L1 (ncu: 65 % SM throughput, 68 % issue active, 65 % L1 "
-                   "wavefronts, 43 % warps active; ~194 candidate tests and ~33 hits a particle)",
-    "forces_eval": "SM issue (ncu: 72 % SM throughput, 76 % issue active; ten IEEE divisions "
-                   "and a square root per pair)",
-    "den_kappa": "L1 data pipe (ncu: 80 % L1 wavefronts; neighbour records gathered through L1)",
+    "density_div": "SM issue and L1 (ncu: 65 % SM throughput, 68 % issue active, 67 % L1 "
+                   "wavefronts, 44 % warps active; ~194 candidate tests and ~33 hits a particle)",
+    "forces_eval": "SM issue (ncu: 71 % SM throughput, 75 % issue active; four IEEE divisions, a "
+                   "reciprocal and a square root per pair)",
+    "den_kappa": "L1 data pipe (ncu: 81 % L1 wavefronts; neighbour records gathered through L1)",
 }
 
 
@@ -267,15 +268,12 @@ def cuda_arm(args):
         ms_max, all_substeps = ms, float(substeps)
     value = n * all_substeps / (ms_max / 1000.0)
 
-    # kernel launches inside the timed region: per substep the grid build
-    # (keys, one per digit pass, starts scan), gather, density_div and its residual
-    # step, forces pair, first density prediction and its residual step,
-    # integrate; 3 per loop iteration; per frame stats (2) and tracers (3).
-    passes = 1
-    cells = sim.keyspace
-    while (cells - 1) >> (8 * passes):
-        passes += 1
-    fixed = 2 + passes + 1 + 2 + 4 + 1
+    # kernel launches inside the timed region: per substep the grid (keys,
+    # scan, place, order with the records), density_div, the first density
+    # prediction and its residual step, integrate; 3 per loop iteration (apply,
+    # the prediction after it, its residual step); per frame stats (2) and
+    # tracers (3).
+    fixed = 4 + 1 + 2 + 1
     launches = fixed * substeps + 3 * (div_it + den_it) + 5 * args.steps
 
     # e2e: a fresh replica, frames through the C ABI with a stats read back
