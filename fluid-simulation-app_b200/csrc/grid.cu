@@ -46,8 +46,9 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 }
 
 // The lanes of `act` whose 8-bit digit equals this lane's: what
-// __match_any_sync(act, d) returns, from one ballot per digit bit (cheaper
-// than the general match on sm_100). Every lane of the warp calls it.
+// __match_any_sync(act, d) returns, from one ballot per digit bit (a build of
+// 16.7M positions 498 us, by the general match 644). Every lane of the warp
+// calls it.
 __device__ __forceinline__ uint32_t digit_peers(uint32_t act, uint32_t d) {
     uint32_t m = act;
 #pragma unroll
@@ -263,26 +264,21 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_lookback(uint32_t *in, ui
 // order and written out by consecutive threads to consecutive addresses.
 // `vals_in` null means the identity (the first pass).
 static_assert(kRadix == kSortThreads, "one thread per digit");
-// Blocks per SM the pass kernel is compiled for: 522 us a build of 16.7M
-// positions at 4 (64 registers), 598 at 5 (spills); tiles of 8,192 keys by
-// 512 threads 539, of 16,384 by 1,024 604, of 3,072 by 256 558.
+// Blocks per SM the pass kernel is compiled for: 498 us a build of 16.7M
+// positions at 4 (64 registers), 538 at 3, 577 at 5 (spills). Of a form of the
+// build that took 522: tiles of 8,192 keys by 512 threads 539, of 16,384 by
+// 1,024 604, of 3,072 by 256 558.
 #ifndef FCU_SORT_MINB
 #define FCU_SORT_MINB 4
 #endif
-// FCU_SORT_MATCH: digit peers by __match_any_sync instead of eight ballots.
-// Measured at 16.7M positions: 15 % slower on uniform keys, 4 % faster on
-// clustered ones; the simulation's grid 6 % faster.
-#ifndef FCU_SORT_MATCH
-#define FCU_SORT_MATCH 0
-#endif
 // FCU_VAL_PREFETCH > 0: a digit pass asks L1 for the values of every
-// FCU_VAL_PREFETCH-th round of its tile while it ranks the keys: 554 us a
-// build of 16.7M positions without, 522 at 1.
+// FCU_VAL_PREFETCH-th round of its tile while it ranks the keys: 539 us a
+// build of 16.7M positions without, 498 at 1.
 #ifndef FCU_VAL_PREFETCH
 #define FCU_VAL_PREFETCH 1
 #endif
-// Earlier tiles' status words a digit's look-back loads at once: 524 us a
-// build of 16.7M positions at 2, 519 at 4, 525 at 8 (spills).
+// Earlier tiles' status words a digit's look-back loads at once: 503 us a
+// build of 16.7M positions at 2, 498 at 4, 512 at 8 (spills).
 #ifndef FCU_LOOK_WINDOW
 #define FCU_LOOK_WINDOW 4
 #endif
@@ -342,11 +338,7 @@ __global__ void __launch_bounds__(kSortThreads, FCU_SORT_MINB) k_radix_pass(
 #pragma unroll
         for (int r = 0; r < kSortItems; ++r) {
             const uint32_t d = (key[r] >> shift) & (kRadix - 1);
-#if FCU_SORT_MATCH
-            rank[r] = __match_any_sync(0xffffffffu, d);
-#else
             rank[r] = digit_peers(0xffffffffu, d);
-#endif
         }
     } else {
 #pragma unroll
@@ -354,11 +346,7 @@ __global__ void __launch_bounds__(kSortThreads, FCU_SORT_MINB) k_radix_pass(
             const bool live = wbase + r * 32 + lane < n;
             const uint32_t act = __ballot_sync(0xffffffffu, live);
             const uint32_t d = (key[r] >> shift) & (kRadix - 1);
-#if FCU_SORT_MATCH
-            const uint32_t pe = live ? __match_any_sync(act, d) : 0u;
-#else
             const uint32_t pe = digit_peers(act, d);
-#endif
             rank[r] = live ? pe : 0u;  // a live lane is its own peer, so nonzero
         }
     }

@@ -26,7 +26,7 @@ constexpr uint32_t kKeyBlocks = 148 * 8;                    // grid cap of the k
 #ifndef FCU_KEY_ITEMS
 #define FCU_KEY_ITEMS 4
 #endif
-constexpr int kKeyItems = FCU_KEY_ITEMS;                    // positions per thread and round (cell keys)
+constexpr int kKeyItems = FCU_KEY_ITEMS;                    // positions per thread and round (cell keys; 498 us a 16.7M build at 4, 509 at 2, 516 at 8)
 
 inline uint32_t div_up(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 

@@ -3,7 +3,7 @@
 //
 // The digit passes of grid.cu are a launch each, with a look-back chain over
 // the tiles in every one: up to a million positions that is latency, not
-// work (98 us at 1M positions, 43 us at 20k). Here the whole build is one
+// work (82 us at 1M positions, 39 us at 20k). Here the whole build is one
 // kernel of at most a block per SM, each block owning a contiguous piece of
 // the input: keys, then per digit the piece ranked (its counts published), a
 // grid barrier, the piece's digit offsets from everybody's counts, the piece
@@ -16,12 +16,12 @@
 // Barriers are bounded like every wait of the grid: one that gives up sets
 // the build's error word, and the writes after it stay in bounds.
 //
-// Measured, us a build against the digit passes: 20k positions 23 / 46, 65k
-// 25 / 48, 262k 38 / 70, 1M 63 / 97 (in 7,000-position clusters 76 / 98, all
-// in one cell 75 / 89). At 1M a pass takes about 13 us, a third of it the two
-// barriers; past one piece a block the passes' tiles overlap better
-// (two tiles a block, 3M: 229 / 187). The digit passes are as they were then;
-// since, 1.3M positions take 89 there instead of 102.
+// Measured, us a build against the digit passes: 20k positions over 14k cells
+// 23 / 39, 65k over 33k 23 / 39, 150k over 125k 35 / 56, 400k over 262k 41 /
+// 60, 1M over 1M 58 / 82 (in 8 clusters 68 / 91, all in one cell 56 / 70). At
+// 1M a pass takes about 13 us, a third of it the two barriers; past one piece a
+// block the passes' tiles overlap better (an earlier form at two tiles a block,
+// 3M positions: 229, the digit passes of the time 187).
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
