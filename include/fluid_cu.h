@@ -451,7 +451,11 @@ uint64_t fluid_grid_workspace_bytes(uint32_t n, const FluidGrid *grid);
  * the scan of sim_scan.wgsl:97-120, stable: starts[C+1] (starts[C] = n) and
  * the permutation perm[n] (slot -> input index, ascending index inside a
  * cell). All pointers are device memory; keys may be null. `stream` is a
- * cudaStream_t (null: the legacy default stream). Asynchronous. */
+ * cudaStream_t (null: the legacy default stream). Asynchronous. Up to 148 x
+ * 8,192 positions the sort is one cooperative launch of at most a block per
+ * SM, which starts when all of its blocks have a place on the SMs the stream
+ * may use; where they never would (a green context of fewer SMs) it is one
+ * launch a digit, as for more positions. */
 int32_t fluid_grid_build(const float *pos4, uint32_t n, const FluidGrid *grid, uint32_t *keys,
                          uint32_t *starts, uint32_t *perm, void *workspace, uint64_t ws_bytes,
                          void *stream);
