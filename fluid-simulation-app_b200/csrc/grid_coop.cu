@@ -307,35 +307,48 @@ constexpr uint32_t kStartsApart = 400000;
 bool starts_apart(const GridWork &w) { return w.cells > kStartsApart; }
 
 // Driver entry points, null where the driver has none.
-struct GreenCalls {
+struct SmCalls {
     PFN_cuStreamGetGreenCtx ctx_of = nullptr;
-    PFN_cuGreenCtxGetDevResource resource = nullptr;
+    PFN_cuGreenCtxGetDevResource of_green = nullptr;
+    PFN_cuCtxGetCurrent current = nullptr;
+    PFN_cuCtxGetDevResource of_ctx = nullptr;
 };
-const GreenCalls &green_calls() {
-    static const GreenCalls calls = [] {
-        GreenCalls c;
-        void *p[2] = {nullptr, nullptr};
-        const char *const name[2] = {"cuStreamGetGreenCtx", "cuGreenCtxGetDevResource"};
-        for (int k = 0; k < 2; ++k) {
+const SmCalls &sm_calls() {
+    static const SmCalls calls = [] {
+        SmCalls c;
+        void *p[4] = {nullptr, nullptr, nullptr, nullptr};
+        const char *const name[4] = {"cuStreamGetGreenCtx", "cuGreenCtxGetDevResource", "cuCtxGetCurrent",
+                                     "cuCtxGetDevResource"};
+        for (int k = 0; k < 4; ++k) {
             cudaDriverEntryPointQueryResult found;
             if (cudaGetDriverEntryPointByVersion(name[k], &p[k], 12040, cudaEnableDefault, &found) != cudaSuccess ||
                 found != cudaDriverEntryPointSuccess)
                 return c;
         }
         c.ctx_of = reinterpret_cast<PFN_cuStreamGetGreenCtx>(p[0]);
-        c.resource = reinterpret_cast<PFN_cuGreenCtxGetDevResource>(p[1]);
+        c.of_green = reinterpret_cast<PFN_cuGreenCtxGetDevResource>(p[1]);
+        c.current = reinterpret_cast<PFN_cuCtxGetCurrent>(p[2]);
+        c.of_ctx = reinterpret_cast<PFN_cuCtxGetDevResource>(p[3]);
         return c;
     }();
     return calls;
 }
 
-// SMs the stream's kernels may run on: its green context's, or the device's.
+// SMs the stream's kernels may run on: its green context's, for a default
+// stream the current context's (which may be a green one's), else the device's.
 uint32_t sms_of(cudaStream_t stream) {
-    const GreenCalls &calls = green_calls();
-    CUgreenCtx green = nullptr;
-    if (calls.ctx_of && calls.ctx_of(stream, &green) == CUDA_SUCCESS && green) {
-        CUdevResource r{};
-        return calls.resource(green, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS ? r.sm.smCount : 0u;
+    const SmCalls &calls = sm_calls();
+    CUdevResource r{};
+    if (calls.ctx_of) {
+        CUgreenCtx green = nullptr;
+        if (stream == nullptr || stream == cudaStreamLegacy || stream == cudaStreamPerThread) {
+            CUcontext ctx = nullptr;
+            if (calls.current(&ctx) == CUDA_SUCCESS && ctx &&
+                calls.of_ctx(ctx, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS)
+                return r.sm.smCount;
+        } else if (calls.ctx_of(stream, &green) == CUDA_SUCCESS && green) {
+            return calls.of_green(green, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS ? r.sm.smCount : 0u;
+        }
     }
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
